@@ -811,13 +811,21 @@ rgf_status smatrix_run(rgf_handle h, const Problem& p, const rgf_request* req, c
   // (partial pivoting as in LAPACK zgetrf), the block is inverted and the
   // rank-32 update applied; at the end the column exchanges are undone.
   if ((st = ensure(h, h->gepp, gepp_scratch_bytes(N)))) return st;
-  auto sweep = [&](int64_t Ract, int64_t Cact, bool timed) -> rgf_status {
+  // With corner_only the caller needs nothing but rows and columns >= N of
+  // the swept matrix.
+  auto sweep = [&](int64_t Ract, int64_t Cact, bool timed, bool corner_only) -> rgf_status {
+    const bool in_cluster = gj_step_fits(Ract);
     for (int64_t j0 = 0; j0 < N; j0 += kSwW) {
       int jn = (int)std::min<int64_t>(kSwW, N - j0);
-      launch_gepp_step(M, ldm, N, Cact, j0, jn, h->gepp.p, status, h->stream);
-      h->launches += 2;
-      launch_sweep_panel(M, ldm, Ract, Cact, j0, jn, as<double2>(h->pc), as<double2>(h->u), ldm, status,
-                         h->stream);
+      if (in_cluster) {
+        RGF_CUDA_TRY(launch_gj_panel(M, ldm, Ract, N, j0, jn, corner_only, as<double2>(h->pc), h->gepp.p, status,
+                                     h->stream));
+      } else {
+        launch_gepp_step(M, ldm, N, Cact, j0, jn, h->gepp.p, status, h->stream);
+        launch_sweep_panel(M, ldm, Ract, Cact, j0, jn, as<double2>(h->pc), as<double2>(h->u), ldm, status,
+                           h->stream);
+        h->launches += 2;
+      }
       if (timed) {
         while (h->ev.size() < ev_used + 2) {
           cudaEvent_t ev;
@@ -826,7 +834,13 @@ rgf_status smatrix_run(rgf_handle h, const Problem& p, const rgf_request* req, c
         }
         RGF_CUDA_TRY(cudaEventRecord(h->ev[ev_used], h->stream));
       }
-      launch_sweep_update(M, ldm, Ract, Cact, j0, jn, as<double2>(h->pc), as<double2>(h->u), ldm, h->stream);
+      if (in_cluster) {
+        launch_gj_update(M, ldm, Ract, N, Cact, j0, jn, corner_only, as<double2>(h->pc), as<double2>(h->u),
+                         h->gepp.p, h->stream);
+        h->launches++;
+      } else {
+        launch_sweep_update(M, ldm, Ract, Cact, j0, jn, as<double2>(h->pc), as<double2>(h->u), ldm, h->stream);
+      }
       if (timed) {
         RGF_CUDA_TRY(cudaEventRecord(h->ev[ev_used + 1], h->stream));
         ev_used += 2;
@@ -834,6 +848,7 @@ rgf_status smatrix_run(rgf_handle h, const Problem& p, const rgf_request* req, c
       }
       h->launches += 2;
     }
+    if (corner_only && in_cluster) return RGF_OK;  // the exchanged columns lie outside the corner
     RGF_CUDA_TRY(launch_gepp_unpermute(M, ldm, Ract, N, h->gepp.p, h->stream));
     h->launches += 2;
     return RGF_OK;
@@ -857,7 +872,7 @@ rgf_status smatrix_run(rgf_handle h, const Problem& p, const rgf_request* req, c
   bool ran_persist = false;
   // per-slice probe residual (both engines)
   unsigned long long* probe_d = nullptr;
-  h->prof_kernel = sweep_update_kernel_name();
+  h->prof_kernel = sweep_update_kernel_name(gj_step_fits(Rp));
   if (L > 0) {
     if ((st = ensure(h, h->xprobe, sizeof(unsigned long long)))) return st;
     probe_d = as<unsigned long long>(h->xprobe);
@@ -986,7 +1001,7 @@ rgf_status smatrix_run(rgf_handle h, const Problem& p, const rgf_request* req, c
     launch_probe_init(M, ldm, N, Rp, pc1, h->stream);
     h->launches++;
     for (int64_t k = k_lo; k < k_hi; k++) {
-      if ((st = sweep(N + no_s, Cp, prof_every && (k % prof_every) == 0))) return st;
+      if ((st = sweep(N + no_s, Cp, prof_every && (k % prof_every) == 0, false))) return st;
       launch_probe_check(M, ldm, N, pc1, probe_d, h->stream);
       h->launches++;
       if (snap && (k - k_lo) % snap_mod == snap_mod - 1)
@@ -1028,7 +1043,8 @@ rgf_status smatrix_run(rgf_handle h, const Problem& p, const rgf_request* req, c
                                    sizeof(double2) * Cs, Rp, S_dev ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost,
                                    h->stream));
   } else {
-    if ((st = sweep(R, C, false))) return st;
+    // the gradient and the fields also start from the carriers of this sweep
+    if ((st = sweep(R, C, false, gr == nullptr))) return st;
 
     // (8) Fisher-Lee (cal_smatrix_RGF.m:279-289)
     double2* Sd = S_dev ? reinterpret_cast<double2*>(S) : as<double2>(h->sdev);
@@ -1314,14 +1330,22 @@ rgf_status segment_merge(rgf_handle h, const Problem& p, const rgf_request* req,
     launch_zgemm(noR, niL, N, one, ZOp{ZR, CR, 0}, ZOp{XL, CL, 0}, zero, M + (N + noL) * ldm + N, ldm, h->stream);
   launch_block_copy(M + (N + noL) * ldm + N + niL, ldm, YR, CR, noR, niR, 1.0, h->stream);
   h->launches += 9;
+  // only the corner of the swept matrix is read
+  const bool in_cluster = gj_step_fits(R);
   for (int64_t j0 = 0; j0 < N; j0 += kSwW) {
     const int jn = (int)std::min<int64_t>(kSwW, N - j0);
+    if (in_cluster) {
+      RGF_CUDA_TRY(launch_gj_panel(M, ldm, R, N, j0, jn, true, as<double2>(h->pc), h->gepp.p, status, h->stream));
+      launch_gj_update(M, ldm, R, N, C, j0, jn, true, as<double2>(h->pc), as<double2>(h->u), h->gepp.p, h->stream);
+      h->launches += 3;
+      continue;
+    }
     launch_gepp_step(M, ldm, N, C, j0, jn, h->gepp.p, status, h->stream);
     launch_sweep_panel(M, ldm, R, C, j0, jn, as<double2>(h->pc), as<double2>(h->u), ldm, status, h->stream);
     launch_sweep_update(M, ldm, R, C, j0, jn, as<double2>(h->pc), as<double2>(h->u), ldm, h->stream);
     h->launches += 4;
   }
-  RGF_CUDA_TRY(launch_gepp_unpermute(M, ldm, R, N, h->gepp.p, h->stream));
+  if (!in_cluster) RGF_CUDA_TRY(launch_gepp_unpermute(M, ldm, R, N, h->gepp.p, h->stream));
   double2* Sd = S_dev ? reinterpret_cast<double2*>(S) : as<double2>(h->sdev);
   const int64_t ldSd = S_dev ? ldS : n_out;
   launch_extract(M, ldm, N, idx_d, n_out, idx_d + n_out, n_in, Sd, ldSd, idx_d + o_pairs, (int)pairs.size() / 2,
@@ -1334,6 +1358,10 @@ rgf_status segment_merge(rgf_handle h, const Problem& p, const rgf_request* req,
   int hstatus = 0;
   RGF_CUDA_TRY(cudaMemcpyAsync(&hstatus, status, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
   RGF_CUDA_TRY(cudaStreamSynchronize(h->stream));
+  if (hstatus & kStatusTimeout) {
+    set_error("a device-side wait timed out");
+    return RGF_ERR_TIMEOUT;
+  }
   if (hstatus & kStatusSingular) {
     set_error("segment merge: the interface matrix I - g_R g_L is singular");
     return RGF_ERR_SINGULAR;

@@ -19,6 +19,10 @@
 // channels, in one pass.  The lead on the far side is attached the same way
 // (cal_smatrix_RGF.m:272-275) with G0_R^{-1} = A_lead - G0_R, and the last
 // sweep's corner block is the Fisher-Lee S/(-2i) (cal_smatrix_RGF.m:279).
+#include <algorithm>
+#include <atomic>
+
+#include "recip.cuh"
 #include "sweep.cuh"
 
 namespace rgf {
@@ -284,7 +288,9 @@ void launch_sweep_update(double2* M, int64_t ldm, int64_t R, int64_t Cc, int64_t
                                              ZAdd{nullptr, 0, 0, 0});
 }
 
-const char* sweep_update_kernel_name() { return "k_zgemm<true> (sweep rank-32 update, FP64 DMMA)"; }
+const char* sweep_update_kernel_name(bool in_cluster) {
+  return in_cluster ? "k_gj_update (sweep rank-32 update, FP64 DMMA)" : "k_zgemm<true> (sweep rank-32 update, FP64 DMMA)";
+}
 
 int sweep_block_width() { return kSw; }
 
@@ -445,7 +451,441 @@ __global__ void k_colperm(double2* M, int64_t ldm, int64_t R, int64_t N, const i
   }
 }
 
+// ---------------------------------------------------------------------------
+// The same step with the whole panel in registers, for matrices whose active
+// rows fit one cluster (R - row0 <= 16 x 256): three launches per pivot block.
+//
+//  k_gj_panel   the block column W(:, J) of every active row, swept: partial
+//               pivoting over the rows j0..N-1 (izamax's choice, as above) and
+//               Gauss-Jordan elimination of all 32 pivots, which leaves
+//               P = [-W(i,J) T (i not in J); T (i in J)], T = W(J,J)^{-1}
+//               after the exchanges: the swept matrix's columns J.
+//  k_pivot_rows the pivot rows W(J, :) -> Wr (unit columns in J), and the rows
+//               they displaced to where the exchanges put them.
+//  k_gj_update  W <- W_mod + P Wr (W with rows and columns J read as zero),
+//               64 x 64 tiles on the FP64 tensor cores.
+//
+// k_gj_panel is one cluster of up to 16 CTAs.  Four threads hold a row (column
+// 4 k + c in register k of thread c), a CTA up to 256 rows.  It is bound by the
+// chain of its 32 pivots: per pivot every warp posts its best row in shared
+// memory, one barrier, then each CTA sends its best row, and the owner of the
+// pivot position the row displaced from there, to every CTA of the cluster with
+// st.async on the receiver's mbarrier: no pivot costs a trip through global
+// memory, nor the round trip of a release after remote stores (1100 cycles of a
+// step's 2900 when it was done that way).  Lane = column with a row per register
+// needs no rotation but three times the instructions per pivot: 84 us against
+// 72 us for 1700 rows.  The one-CTA panel above (its rows in L2) takes 770 us
+// there; a whole step went from 787 to 104 us at N = 1500.
+// ---------------------------------------------------------------------------
+constexpr int kGjRows = 256;     // most rows of a CTA
+constexpr int kGjCluster = 16;   // most CTAs of a cluster
+// a row in shared memory: its 32 columns in the order the threads hold them,
+// {magnitude, row}, the reciprocal of its pivot candidate, {row before this step, -}
+constexpr int kGjMag = 32, kGjRecip = 33, kGjOrg = 34, kGjMsg = 35;
+
+struct GjShared {
+  double2 slot[2][kGjCluster + 1][kGjMsg];  // per step parity: a candidate of every CTA, the displaced row
+  double2 crow[2][32][kGjMsg];              // a candidate row of every warp
+  double2 drow[2][kGjMsg];                  // the row at the pivot position
+  alignas(8) unsigned long long mbar[2];
+};
+
+__device__ __forceinline__ uint32_t gj_smem(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+
+// best row of the lanes: the largest magnitude (compared as FP64, non-negative),
+// ties to the smaller row; row < 0: this lane has none.  Returns the winner's
+// lane; lanes that tie with it in the high word are told apart only when there
+// are several.
+__device__ __forceinline__ int gj_best(double mag, int row) {
+  const unsigned full = 0xffffffffu;
+  const unsigned hi = row < 0 ? 0u : (unsigned)__double2hiint(mag) + 1u;
+  const unsigned whi = __reduce_max_sync(full, hi);
+  unsigned who = __ballot_sync(full, hi == whi);
+  if (who & (who - 1)) {
+    const unsigned lo = hi == whi ? (unsigned)__double2loint(mag) : 0u;
+    const unsigned wlo = __reduce_max_sync(full, lo);
+    const unsigned key = (hi == whi && lo == wlo) ? (unsigned)row : 0xffffffffu;
+    who = __ballot_sync(full, key == __reduce_min_sync(full, key));
+  }
+  return __ffs(who) - 1;
+}
+
+// 1 / z for any finite nonzero z: crecip_nr on z scaled by a power of two, so
+// that |z|^2 lies in [1, 8) whatever the pivot's size
+__device__ __forceinline__ double2 gj_recip(double2 z) {
+  const int e = max((__double2hiint(z.x) >> 20) & 0x7ff, (__double2hiint(z.y) >> 20) & 0x7ff);
+  const double sc = __hiloint2double(min(max(2046 - e, 1), 2045) << 20, 0);  // 2^(1023 - e), kept normal
+  const double2 r = crecip_nr(cscale(z, sc));
+  return cscale(r, sc);
+}
+
+__device__ __forceinline__ void gj_send(uint32_t dst, uint32_t bar, double2 v) {
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.b64 [%0], {%1, %2}, [%3];" ::"r"(dst),
+               "l"(__double_as_longlong(v.x)), "l"(__double_as_longlong(v.y)), "r"(bar)
+               : "memory");
+}
+
+// bounded wait on a phase of a CTA-local mbarrier
+__device__ __forceinline__ bool gj_wait(uint32_t bar, uint32_t parity) {
+  const long long t0 = clock64();
+  for (;;) {
+    uint32_t done;
+    asm volatile("{ .reg .pred P; mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 P, [%1], %2; selp.u32 %0, 1, 0, P; "
+                 "}"
+                 : "=r"(done)
+                 : "r"(bar), "r"(parity)
+                 : "memory");
+    if (done) return true;
+    if (clock64() - t0 > 8000000000LL) return false;  // ~4 s
+  }
+}
+
+// Rows row0 .. R-1 of the panel; swaps[j0+q] as k_panel_gepp; src[q] = row
+// (before this step) now at j0+q, dst[q] = position the row j0+q went to.
+template <int kThreads>
+__global__ void __launch_bounds__(kThreads, 1)
+    k_gj_panel(const double2* __restrict__ W, int64_t ldm, int R, int N, int row0, int j0, int jn, int rows,
+               double2* __restrict__ P, int* __restrict__ swaps, int* __restrict__ src, int* __restrict__ dst,
+               int* status) {
+  extern __shared__ __align__(16) unsigned char gj_raw[];
+  GjShared& sh = *reinterpret_cast<GjShared*>(gj_raw);
+  const unsigned full = 0xffffffffu;
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5, nwarps = (int)blockDim.x >> 5;
+  const int K = (int)gridDim.x, rank = (int)blockIdx.x;
+  const int c4 = t & 3, lrow = t >> 2;
+  const int base = row0 + rank * rows;
+  const int i = base + lrow;
+  const bool valid = lrow < rows && i < R;
+  int org = i;
+  // the registers rotate by one every four pivots, so that the pivot column is
+  // always in a[0] and one loop body serves all of them
+  double2 a[8];
+#pragma unroll
+  for (int k = 0; k < 8; k++) {
+    const int col = 4 * k + c4;
+    a[k] = (valid && col < jn) ? __ldcg(W + (int64_t)i * ldm + j0 + col) : cmk(0.0, 0.0);
+  }
+  if (K > 1) {
+    if (t < 2)
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(gj_smem(&sh.mbar[t])), "r"(1) : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  }
+  bool lost = false, sing = false;
+#pragma unroll 1
+  for (int q = 0; q < kSw; q++) {
+    if (q < jn) {
+      const int par = q & 1, p = j0 + q, qc = q & 3;
+      const bool owner = c4 == qc;
+      if (K > 1 && t == 0)  // this step's messages: K candidates and one displaced row
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(gj_smem(&sh.mbar[par])),
+                     "r"((unsigned)(16 * kGjMsg * (K + 1)))
+                     : "memory");
+      // ---- candidate of this warp, and the row at the pivot position ----
+      double mag = fabs(a[0].x) + fabs(a[0].y);  // izamax's magnitude
+      if (mag != mag) mag = INFINITY;            // a NaN wins, so that it is flagged below
+      const bool elig = owner && valid && i >= p && i < N;
+      const double2 dq = gj_recip(a[0]);  // speculative, beside the search
+      const int wl = gj_best(mag, elig ? i : -1);
+      if ((lane >> 2) == (wl >> 2)) {  // the four threads of the best row
+        double2* cr = sh.crow[par][warp];
+#pragma unroll
+        for (int k = 0; k < 8; k++) cr[4 * k + c4] = a[k];
+        if (owner) {
+          cr[kGjMag] = cmk(mag, elig ? (double)i : -1.0);
+          cr[kGjRecip] = dq;
+          cr[kGjOrg] = cmk((double)org, 0.0);
+        }
+      }
+      if (valid && i == p) {
+#pragma unroll
+        for (int k = 0; k < 8; k++) sh.drow[par][4 * k + c4] = a[k];
+        if (c4 == 0) sh.drow[par][kGjOrg] = cmk((double)org, 0.0);
+      }
+      __syncthreads();
+      // ---- the CTA's candidate, the cluster's ----
+      double2 cd = lane < nwarps ? sh.crow[par][lane][kGjMag] : cmk(0.0, -1.0);
+      const double2* prow = sh.crow[par][gj_best(cd.x, (int)cd.y)];
+      const double2* drow = sh.drow[par];
+      if (K > 1) {
+        // warp k sends the candidate (and the displaced row) to CTA k
+        const uint32_t bar_l = gj_smem(&sh.mbar[par]);
+        for (int k = warp; k < K; k += nwarps) {
+          uint32_t bar, to;
+          asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(bar) : "r"(bar_l), "r"(k));
+          asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(to) : "r"(gj_smem(&sh.slot[par][rank][0])), "r"(k));
+          gj_send(to + 16 * lane, bar, prow[lane]);
+          if (lane < kGjMsg - 32) gj_send(to + 16 * (32 + lane), bar, prow[32 + lane]);
+          if (p >= base && p < base + rows) {
+            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
+                         : "=r"(to)
+                         : "r"(gj_smem(&sh.slot[par][kGjCluster][0])), "r"(k));
+            gj_send(to + 16 * lane, bar, drow[lane]);
+            if (lane < kGjMsg - 32) gj_send(to + 16 * (32 + lane), bar, drow[kGjOrg]);
+          }
+        }
+        if (!lost && !gj_wait(bar_l, (uint32_t)((q >> 1) & 1))) {
+          atomicOr(status, kStatusTimeout);
+          lost = true;
+        }
+        cd = lane < K ? sh.slot[par][lane][kGjMag] : cmk(0.0, -1.0);
+        prow = sh.slot[par][gj_best(cd.x, (int)cd.y)];
+        drow = sh.slot[par][kGjCluster];
+      }
+      // ---- exchange the pivot row with row p, eliminate column q ----
+      const double2 best = prow[kGjMag], d = prow[kGjRecip];
+      const int brow = (int)best.y;
+      sing = sing || !(best.x > 0.0) || !isfinite(best.x);
+      const bool at_p = i == p;
+      if (at_p) {
+        org = (int)prow[kGjOrg].x;
+      } else if (valid && i == brow) {
+#pragma unroll
+        for (int k = 0; k < 8; k++) a[k] = drow[4 * k + c4];
+        org = (int)drow[kGjOrg].x;
+      }
+      if (rank == 0 && t == 0) swaps[p] = brow;
+      const double mx = __shfl_sync(full, a[0].x, (lane & ~3) | qc), my = __shfl_sync(full, a[0].y, (lane & ~3) | qc);
+      const double2 m = at_p ? cneg(d) : cmul(cmk(mx, my), d);
+#pragma unroll
+      for (int k = 0; k < 8; k++) {
+        const double2 pr = prow[4 * k + c4];
+        const double2 o = at_p ? cmk(0.0, 0.0) : a[k];
+        a[k] = cmk(fma(-m.x, pr.x, fma(m.y, pr.y, o.x)), fma(-m.x, pr.y, fma(-m.y, pr.x, o.y)));
+      }
+      if (owner) a[0] = cneg(m);
+    }
+    if ((q & 3) == 3) {
+      const double2 first = a[0];
+#pragma unroll
+      for (int k = 0; k < 7; k++) a[k] = a[k + 1];
+      a[7] = first;
+    }
+  }
+  if (sing && t == 0) atomicOr(status, kStatusSingular);
+#pragma unroll
+  for (int k = 0; k < 8; k++)
+    if (valid) __stcg(P + (int64_t)i * kSw + 4 * k + c4, a[k]);
+  if (valid && c4 == 0) {
+    if (i >= j0 && i < j0 + jn) src[i - j0] = org;
+    if (org >= j0 && org < j0 + jn) dst[org - j0] = i;
+  }
+  if (K > 1) {  // no CTA leaves while another may still write to it
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  }
+}
+
 constexpr int kColpermCtas = 64;
+
+// Wr(q, c) = W(src[q], c) on columns [c0, Cc) (unit columns in J, zero rows
+// from jn on), and the displaced rows of J to their places outside it.  32
+// columns a CTA; every thread reads its rows before the CTA writes any.
+__global__ void __launch_bounds__(256) k_pivot_rows(double2* W, int64_t ldm, int64_t c0, int64_t Cc, int64_t j0, int jn,
+                                                    const int* __restrict__ src, const int* __restrict__ dst,
+                                                    double2* __restrict__ Wr) {
+  const int64_t c = c0 + blockIdx.x * (int64_t)32 + (threadIdx.x & 31);
+  const int g = threadIdx.x >> 5;
+  double2 v[4], u[4];
+  int to[4];
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    const int q = g * 4 + k;
+    to[k] = -1;
+    v[k] = u[k] = cmk(0.0, 0.0);
+    if (q < jn && c < Cc) {
+      if (c >= j0 && c < j0 + jn) {
+        v[k] = cmk(c - j0 == q ? 1.0 : 0.0, 0.0);
+      } else {
+        v[k] = W[(int64_t)src[q] * ldm + c];
+        const int d = dst[q];
+        if (d < j0 || d >= j0 + jn) {
+          u[k] = W[(j0 + q) * ldm + c];
+          to[k] = d;
+        }
+      }
+    }
+  }
+  __syncthreads();
+  if (c >= Cc) return;
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    Wr[(int64_t)(g * 4 + k) * ldm + c] = v[k];
+    if (to[k] >= 0) W[(int64_t)to[k] * ldm + c] = u[k];
+  }
+}
+
+// W <- W_mod + P Wr on rows [r0, R) and columns [c0, Cc).  The old W goes
+// straight into the accumulators while the operands come by cp.async, and
+// three CTAs share an SM, so that one's loads run under another's products.
+__global__ void __launch_bounds__(128, 3) k_gj_update(double2* W, int64_t ldm, int64_t r0, int64_t R, int64_t c0,
+                                                      int64_t Cc, int64_t j0, int jn, const double2* __restrict__ P,
+                                                      const double2* __restrict__ Wr) {
+  extern __shared__ double2 gj_sm[];
+  double2* As = gj_sm;               // [kBM][kAS]
+  double2* Bs = gj_sm + kBM * kAS;   // [kBK][kBS]
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5, wr = warp >> 1, wc = warp & 1;
+  const int64_t m0 = r0 + (int64_t)blockIdx.y * kBM, n0 = c0 + (int64_t)blockIdx.x * kBN;
+  auto copy16 = [](double2* d, const double2* g, bool in) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(gj_smem(d)), "l"(g), "r"(in ? 16 : 0)
+                 : "memory");
+  };
+#pragma unroll 4
+  for (int e = t; e < kBM * kBK; e += 128) {
+    const int r = e >> 5, k = e & 31;
+    const bool in = m0 + r < R;
+    copy16(As + r * kAS + k, in ? P + (m0 + r) * kSw + k : P, in);
+  }
+#pragma unroll 4
+  for (int e = t; e < kBK * kBN; e += 128) {
+    const int k = e >> 6, c = e & 63;
+    const bool in = n0 + c < Cc;
+    copy16(Bs + k * kBS + c, in ? Wr + (int64_t)k * ldm + n0 + c : Wr, in);
+  }
+  asm volatile("cp.async.commit_group;" ::: "memory");
+  double acc[4][4][4];
+#pragma unroll
+  for (int mi = 0; mi < 4; mi++) {
+    const int64_t r = m0 + wr * 32 + mi * 8 + (lane >> 2);
+    const bool rin = r < R && !(r >= j0 && r < j0 + jn);
+#pragma unroll
+    for (int ni = 0; ni < 4; ni++)
+#pragma unroll
+      for (int h = 0; h < 2; h++) {
+        const int64_t c = n0 + wc * 32 + ni * 8 + (lane & 3) * 2 + h;
+        const double2 v = (rin && c < Cc && !(c >= j0 && c < j0 + jn)) ? __ldcg(W + r * ldm + c) : cmk(0.0, 0.0);
+        acc[mi][ni][h] = v.x;
+        acc[mi][ni][2 + h] = v.y;
+      }
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  __syncthreads();
+#pragma unroll
+  for (int kk = 0; kk < kBK / 4; kk++) {
+    double2 b[4];
+#pragma unroll
+    for (int ni = 0; ni < 4; ni++) b[ni] = Bs[(kk * 4 + (lane & 3)) * kBS + wc * 32 + ni * 8 + (lane >> 2)];
+#pragma unroll
+    for (int mi = 0; mi < 4; mi++) {
+      const double2 a = As[(wr * 32 + mi * 8 + (lane >> 2)) * kAS + kk * 4 + (lane & 3)];
+#pragma unroll
+      for (int ni = 0; ni < 4; ni++) {
+        dmma884(acc[mi][ni][0], acc[mi][ni][1], a.x, b[ni].x);
+        dmma884(acc[mi][ni][2], acc[mi][ni][3], a.x, b[ni].y);
+      }
+#pragma unroll
+      for (int ni = 0; ni < 4; ni++) {
+        dmma884(acc[mi][ni][0], acc[mi][ni][1], -a.y, b[ni].y);
+        dmma884(acc[mi][ni][2], acc[mi][ni][3], a.y, b[ni].x);
+      }
+    }
+  }
+#pragma unroll
+  for (int mi = 0; mi < 4; mi++) {
+    const int64_t r = m0 + wr * 32 + mi * 8 + (lane >> 2);
+    if (r >= R) continue;
+#pragma unroll
+    for (int ni = 0; ni < 4; ni++)
+#pragma unroll
+      for (int h = 0; h < 2; h++) {
+        const int64_t c = n0 + wc * 32 + ni * 8 + (lane & 3) * 2 + h;
+        if (c < Cc) __stcg(W + r * ldm + c, cmk(acc[mi][ni][h], acc[mi][ni][2 + h]));
+      }
+  }
+}
+
+// largest cluster k_gj_panel can run with on the current device (16 where the
+// GPU grants the non-portable size, else 8); prepares the kernel on first use
+constexpr int kMaxDevices = 64;
+template <int kThreads>
+static int gj_max_cluster() {
+  static std::atomic<int> cached[kMaxDevices];
+  int dev = 0;
+  cudaGetDevice(&dev);
+  std::atomic<int>& mine = cached[dev & (kMaxDevices - 1)];
+  int c = mine.load();
+  if (c) return c;
+  const void* fn = (const void*)k_gj_panel<kThreads>;
+  cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(GjShared));
+  c = 8;
+  if (cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) {
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = kGjCluster;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.gridDim = dim3(kGjCluster);
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = sizeof(GjShared);
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, fn, &cfg) == cudaSuccess && n > 0) c = kGjCluster;
+  }
+  cudaGetLastError();
+  mine.store(c);
+  return c;
+}
+
+template <int kThreads>
+static cudaError_t gj_panel(const double2* W, int64_t ldm, int R, int N, int row0, int j0, int jn, int K, int rows,
+                            double2* P, int* swaps, int* src, int* dst, int* status, cudaStream_t s) {
+  cudaLaunchConfig_t cfg{};
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = K;
+  at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  cfg.gridDim = dim3(K);
+  cfg.blockDim = dim3(4 * rows);
+  cfg.dynamicSmemBytes = sizeof(GjShared);
+  cfg.stream = s;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, k_gj_panel<kThreads>, W, ldm, R, N, row0, j0, jn, rows, P, swaps, src, dst, status);
+}
+
+// 64 rows a CTA while the cluster can grow: the work of a pivot shrinks with
+// the rows, its exchange hardly grows with the cluster (panel of 1500 x 32 and
+// 32, 64 or 128 rows wanted: 35.0, 34.9, 35.0 ms for six slices; one CTA of 256
+// threads is as fast as two for up to 64 rows)
+constexpr int kGjRowsWanted = 64;
+
+bool gj_step_fits(int64_t active_rows) {
+  return active_rows <= (int64_t)kGjRows * gj_max_cluster<4 * kGjRows>();
+}
+
+cudaError_t launch_gj_panel(const double2* W, int64_t ldm, int64_t R, int64_t N, int64_t j0, int jn, bool trailing,
+                            double2* P, void* scratch, int* status, cudaStream_t s) {
+  int* swaps = reinterpret_cast<int*>(reinterpret_cast<double2*>(scratch) + (size_t)N * (kSw + kColpermCtas));
+  int* src = reinterpret_cast<int*>(scratch);
+  const int64_t row0 = trailing ? j0 : 0, n = R - row0;
+  const int most = std::min(gj_max_cluster<512>(), gj_max_cluster<4 * kGjRows>());
+  int K = 1;
+  while (K < most && n > (int64_t)K * kGjRowsWanted) K *= 2;
+  const int rows = (int)(((n + K - 1) / K + 7) & ~(int64_t)7);
+  if (rows <= 128)
+    return gj_panel<512>(W, ldm, (int)R, (int)N, (int)row0, (int)j0, jn, K, rows, P, swaps, src, src + kSw, status, s);
+  return gj_panel<4 * kGjRows>(W, ldm, (int)R, (int)N, (int)row0, (int)j0, jn, K, rows, P, swaps, src, src + kSw, status,
+                               s);
+}
+
+void launch_gj_update(double2* W, int64_t ldm, int64_t R, int64_t N, int64_t Cc, int64_t j0, int jn, bool trailing,
+                      const double2* P, double2* Wr, void* scratch, cudaStream_t s) {
+  const int* src = reinterpret_cast<const int*>(scratch);
+  const int64_t lo = trailing ? j0 + jn : 0;
+  if (lo >= Cc || lo >= R) return;
+  k_pivot_rows<<<(unsigned)((Cc - lo + 31) / 32), 256, 0, s>>>(W, ldm, lo, Cc, j0, jn, src, src + kSw, Wr);
+  static std::atomic<bool> attr[kMaxDevices];
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (!attr[dev & (kMaxDevices - 1)].load()) {
+    cudaFuncSetAttribute(k_gj_update, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGemmSmem);
+    attr[dev & (kMaxDevices - 1)].store(true);
+  }
+  const dim3 grid((unsigned)((Cc - lo + kBN - 1) / kBN), (unsigned)((R - lo + kBM - 1) / kBM));
+  k_gj_update<<<grid, 128, kGemmSmem, s>>>(W, ldm, lo, R, lo, Cc, j0, jn, P, Wr);
+}
 
 size_t gepp_scratch_bytes(int64_t N) {
   // panel N x kSw, rowtmp kColpermCtas x N (complex); swaps and src (N ints each)

@@ -27,7 +27,7 @@ void launch_sweep_panel(const double2* M, int64_t ldm, int64_t R, int64_t Cc, in
                         double2* U, int64_t ldu, int* status, cudaStream_t s);
 void launch_sweep_update(double2* M, int64_t ldm, int64_t R, int64_t Cc, int64_t j0, int jn, const double2* Pc,
                          const double2* U, int64_t ldu, cudaStream_t s);
-const char* sweep_update_kernel_name();
+const char* sweep_update_kernel_name(bool in_cluster);
 // partial pivoting over the whole remaining column (see sweep.cu): scratch of
 // gepp_scratch_bytes(N); launch_gepp_step before each sweep step (rows of W
 // exchanged over columns [0, Cc)), launch_gepp_unpermute after the last one
@@ -35,6 +35,15 @@ size_t gepp_scratch_bytes(int64_t N);
 void launch_gepp_step(double2* M, int64_t ldm, int64_t N, int64_t Cc, int64_t j0, int jn, void* scratch,
                       int* status, cudaStream_t s);
 cudaError_t launch_gepp_unpermute(double2* M, int64_t ldm, int64_t R, int64_t N, void* scratch, cudaStream_t s);
+// the same step in three launches with the panel in the registers of one
+// cluster (gj_step_fits: active rows R - j0 (trailing) or R); P: R x 32, Wr:
+// 32 x ldm.  trailing: only the rows and columns beyond the step are kept up
+// to date (enough for the corner block of the swept matrix).
+bool gj_step_fits(int64_t active_rows);
+cudaError_t launch_gj_panel(const double2* W, int64_t ldm, int64_t R, int64_t N, int64_t j0, int jn, bool trailing,
+                            double2* P, void* scratch, int* status, cudaStream_t s);
+void launch_gj_update(double2* W, int64_t ldm, int64_t R, int64_t N, int64_t Cc, int64_t j0, int jn, bool trailing,
+                      const double2* P, double2* Wr, void* scratch, cudaStream_t s);
 void launch_probe_check(const double2* M, int64_t ldm, int64_t N, int64_t pc1, unsigned long long* probe_max,
                         cudaStream_t s);
 void launch_assemble(double2* M, int64_t ldm, int64_t N, int64_t Rz, const double2* Gsrc, int64_t ldg,
