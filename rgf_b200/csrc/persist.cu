@@ -336,27 +336,54 @@ __device__ void math_role(const PersistParams& p, Shared& sh, const Sync& sy, in
   // works on its own accumulators only.  The probe pair is the column pair
   // (pc1, pc1 + 1), pc1 even, so one thread holds both as h = 0, 1.
   // Returns the largest probe residual this thread saw.
+  // No step of the sweep runs meanwhile, so what counts is the latency of the
+  // slowest warp: v and A0 v come from tables, the slice's eps is read by the
+  // warps on the diagonal or the probe pair only, all rows at once, and the
+  // stencil by the warps that hold one of its entries (a slice of N = 1000 went
+  // from 575 to 553 us, of N = 64 on 32 x 32 tiles from 42.1 to 40.4 us).
+  const bool on_diag = t.r_base < t.c_base + Tile::WC && t.c_base < t.r_base + Tile::WR;
+  const bool on_probe = p.pc1 >= t.c_base && p.pc1 < t.c_base + Tile::WC;
+  bool on_stencil = false;
+  for (int e = t.lane; e < Tile::WR * kMaxStencil; e += 32) {
+    const int i = t.r_base + e / kMaxStencil;
+    const int c = i < p.N ? __ldg(p.st_col + (int64_t)i * kMaxStencil + e % kMaxStencil) : -1;
+    on_stencil = on_stencil || (c >= t.c_base && c < t.c_base + Tile::WC);
+  }
+  on_stencil = __any_sync(kFull, on_stencil);
   auto boundary_regs = [&](const double2* eps_next, double2* snap) {
     double pmax = 0.0;
-    // the probe pair of each row goes through a small local array, so that
-    // its (long) arithmetic is instantiated once, not once per accumulator
-    double2 pr[MI][2];
-    unsigned has = 0;
+    double2 ke[MI];
+#pragma unroll
+    for (int mi = 0; mi < MI; mi++) {
+      const int i = t.row(mi);
+      ke[mi] = (eps_next && (on_diag || on_probe) && i < p.N) ? __ldg(eps_next + i) : cmk(0.0, 0.0);
+    }
+#pragma unroll
+    for (int mi = 0; mi < MI; mi++) ke[mi] = cmul(p.k2, ke[mi]);
 #pragma unroll
     for (int mi = 0; mi < MI; mi++) {
       const int i = t.row(mi);
       if (i >= p.R) continue;
-      const bool top = i < p.N;
-      const double2 ke = (eps_next && top) ? cmul(p.k2, __ldg(eps_next + i)) : cmk(0.0, 0.0);
 #pragma unroll
       for (int ni = 0; ni < NI; ni++) {
         const int j0c = t.col(ni, 0);  // even; j0c + 1 is the h = 1 column
         if (j0c >= p.C) continue;
         double* a = t.acc[mi][ni];
         if (j0c == p.pc1) {
-          pr[mi][0] = cmk(a[0], a[2]);
-          pr[mi][1] = cmk(a[1], a[3]);
-          has |= 1u << mi;
+          if (i < p.N) {
+            const double2 v = __ldg(p.probe + i);
+            const double rr = sqrt(cabs2(csub(cmk(a[1], a[3]), v)));
+            pmax = (rr == rr) ? fmax(pmax, rr) : INFINITY;  // fmax would drop a NaN
+            if (eps_next) {
+              const double2 av = csub(__ldg(p.probe + p.N + i), cmul(ke[mi], v));
+              a[1] = av.x - a[0];
+              a[3] = av.y - a[2];
+              a[0] = v.x;
+              a[2] = v.y;
+            }
+          } else if (eps_next) {
+            a[0] = a[1] = a[2] = a[3] = 0.0;
+          }
           continue;
         }
 #pragma unroll
@@ -368,61 +395,28 @@ __device__ void math_role(const PersistParams& p, Shared& sh, const Sync& sy, in
           a[h] = -a[h];  // -G_n, or the -Z rows
           a[2 + h] = -a[2 + h];
           if (i == j) {
-            a[h] -= ke.x;
-            a[2 + h] -= ke.y;
+            a[h] -= ke[mi].x;
+            a[2 + h] -= ke[mi].y;
           }
         }
       }
       // + A0 (stencil entries of row i), one entry at a time
-      if (!eps_next || !top) continue;
+      if (!eps_next || !on_stencil || i >= p.N) continue;
 #pragma unroll 1
       for (int q = 0; q < kMaxStencil; q++) {
         const int cq = __ldg(p.st_col + (int64_t)i * kMaxStencil + q);
-        if (cq < 0) continue;
+        if (cq < t.c_base || cq >= t.c_base + Tile::WC) continue;
         const double2 v = __ldg(p.st_val + (int64_t)i * kMaxStencil + q);
 #pragma unroll
         for (int ni = 0; ni < NI; ni++)
 #pragma unroll
           for (int h = 0; h < 2; h++)
-            if (cq == t.col(ni, h) && cq != p.pc1 && cq != p.pc1 + 1) {
+            if (cq == t.col(ni, h)) {  // cq < N: never a probe column
               t.acc[mi][ni][h] += v.x;
               t.acc[mi][ni][2 + h] += v.y;
             }
       }
     }
-    if (has == 0u) return pmax;
-#pragma unroll 1
-    for (int mi = 0; mi < MI; mi++) {
-      if (!((has >> mi) & 1u)) continue;
-      const int i = t.row(mi);
-      if (i < p.N) {
-        const double2 v = probe_v(i);
-        const double2 d = csub(pr[mi][1], v);
-        const double rr = sqrt(cabs2(d));
-        pmax = (rr == rr) ? fmax(pmax, rr) : INFINITY;  // fmax would drop a NaN
-        if (eps_next) {
-          double2 Av = csub(cmk(0.0, 0.0), cmul(cmul(p.k2, __ldg(eps_next + i)), v));
-          for (int q = 0; q < kMaxStencil; q++) {
-            const int cq = __ldg(p.st_col + (int64_t)i * kMaxStencil + q);
-            if (cq >= 0) Av = cadd(Av, cmul(__ldg(p.st_val + (int64_t)i * kMaxStencil + q), probe_v(cq)));
-          }
-          pr[mi][1] = csub(Av, pr[mi][0]);
-          pr[mi][0] = v;
-        }
-      } else if (eps_next) {
-        pr[mi][0] = pr[mi][1] = cmk(0.0, 0.0);
-      }
-    }
-#pragma unroll
-    for (int mi = 0; mi < MI; mi++)
-#pragma unroll
-      for (int ni = 0; ni < NI; ni++)
-        if (((has >> mi) & 1u) && t.col(ni, 0) == p.pc1) {
-          t.acc[mi][ni][0] = pr[mi][0].x;
-          t.acc[mi][ni][2] = pr[mi][0].y;
-          t.acc[mi][ni][1] = pr[mi][1].x;
-          t.acc[mi][ni][3] = pr[mi][1].y;
-        }
     return pmax;
   };
   // rank-32 update of the whole warp tile: first halves of every complex

@@ -17,6 +17,7 @@ struct PersistParams {
   const int* st_col;     // A0 stencil, kMaxStencil entries per row
   const double2* st_val;
   int pc1;               // probe columns pc1, pc1 + 1 (pc1 even), -1 = none
+  const double2* probe;  // [2][N]: the probe vector v, and A0 v
   double2* pcbuf;        // [2][TR][BM][32]
   double2* rowbuf;       // [2][TC][32][BN] pivot rows of a step (written by the panels)
   double2* prebuf;       // [2][TC][32][BN] the same rows one step earlier (written by the math warps)

@@ -897,7 +897,8 @@ rgf_status smatrix_run(rgf_handle h, const Problem& p, const rgf_request* req, c
       RGF_CUDA_TRY(cudaMemsetAsync(flags, 0xFF, sizeof(int) * nflags, h->stream));
       RGF_CUDA_TRY(cudaMemsetAsync(flags + nflags, 0, sizeof(int) * (ncons + 4), h->stream));
       launch_probe_init(M, ldm, N, Rp, pc1, h->stream);
-      h->launches++;
+      launch_probe_tables(st_col, st_val, N, h->gepp.p, h->stream);
+      h->launches += 2;
       PersistParams pp;
       pp.N = (int)N;
       pp.R = (int)Rp;
@@ -915,6 +916,7 @@ rgf_status smatrix_run(rgf_handle h, const Problem& p, const rgf_request* req, c
       pp.st_col = st_col;
       pp.st_val = st_val;
       pp.pc1 = (int)pc1;
+      pp.probe = probe_tables(h->gepp.p);
       pp.pcbuf = as<double2>(h->xpc);
       pp.rowbuf = as<double2>(h->xrow);
       pp.prebuf = as<double2>(h->xrow) + (size_t)2 * TC * 32 * BNp;

@@ -1120,6 +1120,28 @@ void launch_probe_init(double2* M, int64_t ldm, int64_t N, int64_t R, int64_t pc
   k_probe_init<<<(unsigned)((R + 7) / 8), 256, 0, s>>>(M, ldm, N, R, pc1);
 }
 
+// tables of the persistent sweep's slice boundary: v(i) and (A0 v)(i)
+__global__ void k_probe_tables(const int* __restrict__ st_col, const double2* __restrict__ st_val, int64_t N,
+                               double2* __restrict__ tab) {
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (i >= N) return;
+  double2 s = cmk(0.0, 0.0);
+#pragma unroll
+  for (int q = 0; q < kMaxStencil; q++) {
+    const int c = st_col[i * kMaxStencil + q];
+    if (c >= 0) s = cadd(s, cmul(st_val[i * kMaxStencil + q], probe_v(c)));
+  }
+  tab[i] = probe_v(i);
+  tab[N + i] = s;
+}
+
+// the tables' place in the pivoting scratch, beyond the row lists of a step
+double2* probe_tables(void* scratch) { return reinterpret_cast<double2*>(scratch) + 16; }
+
+void launch_probe_tables(const int* st_col, const double2* st_val, int64_t N, void* scratch, cudaStream_t s) {
+  k_probe_tables<<<(unsigned)((N + 127) / 128), 128, 0, s>>>(st_col, st_val, N, probe_tables(scratch));
+}
+
 // ---------------------------------------------------------------------------
 // misc
 // ---------------------------------------------------------------------------
