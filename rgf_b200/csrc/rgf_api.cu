@@ -124,6 +124,20 @@ namespace {
     }                                                                              \
   } while (0)
 
+// SM clock of a device in kHz, asked for once: the query goes to the kernel
+// driver and takes 1.1 ms, half of a small call
+int clock_khz(int device) {
+  static std::atomic<int> known[64];
+  std::atomic<int>& k = known[device & 63];
+  int v = k.load();
+  if (v == 0) {
+    v = 2000000;
+    cudaDeviceGetAttribute(&v, cudaDevAttrClockRate, device);
+    k.store(v);
+  }
+  return v;
+}
+
 rgf_status ensure(rgf_handle h, DevBuf& b, size_t bytes) {
   if (bytes == 0) bytes = 16;
   if (b.bytes >= bytes) return RGF_OK;
@@ -466,8 +480,7 @@ void gang_launch(GangBatch* g) {
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(d_ctas, ctas.data(), sizeof(int) * ctas.size(), cudaMemcpyHostToDevice, g->stream);
   if (e == cudaSuccess) e = cudaMemsetAsync(d_state, 0, sizeof(GangState), g->stream);
-  int clk_khz = 2000000;
-  cudaDeviceGetAttribute(&clk_khz, cudaDevAttrClockRate, g->device);
+  const int clk_khz = clock_khz(g->device);
   // a free CTA may wait for a whole structure to finish: bound the scheduler's
   // waits by three times the batch's sequential estimate, at least 30 s
   const double sched_s = std::max(30.0, 3.0 * est_s);
@@ -933,8 +946,7 @@ rgf_status smatrix_run(rgf_handle h, const Problem& p, const rgf_request* req, c
       pp.snap_ld = Rp * ldm;
       pp.status = status;
       pp.probe_max = probe_d;
-      int clk_khz = 2000000;
-      cudaDeviceGetAttribute(&clk_khz, cudaDevAttrClockRate, h->device);
+      const int clk_khz = clock_khz(h->device);
       // bound of every device-side wait: ~4 s, or RGF_WAIT_TIMEOUT_MS
       const char* tmo_env = getenv("RGF_WAIT_TIMEOUT_MS");
       const double tmo_ms = (tmo_env && atof(tmo_env) > 0) ? atof(tmo_env) : 4000.0;
