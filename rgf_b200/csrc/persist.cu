@@ -1267,11 +1267,24 @@ __device__ void stage_role(const PersistParams& p, Shared& sh, const Sync& sy) {
   }
 }
 
+// Independent sweeps side by side: the parts of a structure cut along its
+// length, whose chains of pivot blocks overlap.  Part q has the CTAs
+// [first[q], first[q + 1]).
+struct PersistSet {
+  int count;
+  int first[kPersistMaxParts + 1];
+  PersistParams p[kPersistMaxParts];
+};
+
 template <int BM, int BN>
-__global__ void __launch_bounds__(Cfg<BM, BN>::Threads, 1) k_persist(PersistParams p) {
+__global__ void __launch_bounds__(Cfg<BM, BN>::Threads, 1) k_persist(const __grid_constant__ PersistSet set) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   Shared& sh = *reinterpret_cast<Shared*>(smem_raw);
-  const int I = blockIdx.x / p.TC, Cq = blockIdx.x % p.TC;
+  int part = 0;
+  while (part + 1 < set.count && (int)blockIdx.x >= set.first[part + 1]) part++;
+  const PersistParams& p = set.p[part];
+  const int local = (int)blockIdx.x - set.first[part];
+  const int I = local / p.TC, Cq = local % p.TC;
   Sync sy(p);
   if (threadIdx.x == 0) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&sh.mbar)) : "memory");
@@ -1282,8 +1295,8 @@ __global__ void __launch_bounds__(Cfg<BM, BN>::Threads, 1) k_persist(PersistPara
     sh.ycons = -1;
   }
   __syncthreads();
-  const bool server = blockIdx.x == (unsigned)(p.TR * p.TC);
-  const bool yprep = blockIdx.x == (unsigned)(p.TR * p.TC + 1);
+  const bool server = local == p.TR * p.TC;
+  const bool yprep = local == p.TR * p.TC + 1;
   static_assert(Cfg<BM, BN>::MathThreads == kServerThreads, "the server uses the math warpgroups");
   if (threadIdx.x < Cfg<BM, BN>::MathThreads) {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(Cfg<BM, BN>::MathRegs));
@@ -1513,9 +1526,16 @@ bool persist_choose_tile(int64_t R, int64_t C, int sms, int* BM, int* BN, bool p
   return false;
 }
 
-cudaError_t launch_persist(const PersistParams& p, int BM, int BN, cudaStream_t s) {
-  PersistParams pp = p;
-  void* args[] = {(void*)&pp};
+cudaError_t launch_persist(const PersistParams* p, int count, int BM, int BN, cudaStream_t s) {
+  if (count < 1 || count > kPersistMaxParts) return cudaErrorInvalidValue;
+  PersistSet set;
+  set.count = count;
+  set.first[0] = 0;
+  for (int q = 0; q < count; q++) {
+    set.p[q] = p[q];
+    set.first[q + 1] = set.first[q] + p[q].TR * p[q].TC + kPersistExtraCtas;
+  }
+  void* args[] = {(void*)&set};
   const size_t smem = sizeof(Shared);
   const void* fn = nullptr;
   if (BM == 96 && BN == 96) fn = (const void*)k_persist<96, 96>;
@@ -1524,8 +1544,7 @@ cudaError_t launch_persist(const PersistParams& p, int BM, int BN, cudaStream_t 
   else return cudaErrorInvalidValue;
   cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  return cudaLaunchCooperativeKernel(fn, dim3(p.TR * p.TC + kPersistExtraCtas), dim3(persist_threads(BM, BN)), args,
-                                     smem, s);
+  return cudaLaunchCooperativeKernel(fn, dim3(set.first[count]), dim3(persist_threads(BM, BN)), args, smem, s);
 }
 
 }  // namespace rgf

@@ -82,6 +82,9 @@ cudaError_t launch_persist_gang(const PersistParams* params, const int* ctas, in
 size_t persist_smem_bytes();
 int persist_threads(int BM, int BN);
 bool persist_choose_tile(int64_t R, int64_t C, int sms, int* BM, int* BN, bool prefer_large = false);
-cudaError_t launch_persist(const PersistParams& p, int BM, int BN, cudaStream_t s);
+// up to kPersistMaxParts independent sweeps in one cooperative launch, each on
+// CTAs of its own (the sum of TR * TC + kPersistExtraCtas must fit the GPU)
+constexpr int kPersistMaxParts = 16;
+cudaError_t launch_persist(const PersistParams* p, int count, int BM, int BN, cudaStream_t s);
 
 }  // namespace rgf

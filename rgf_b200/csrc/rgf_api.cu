@@ -61,6 +61,7 @@ struct GangBatch {
   int device = 0, sms = 0;
   cudaStream_t stream = nullptr;
   int64_t launches = 0;
+  bool halves = false;  // the launch has room for two sweeps per structure
 };
 
 
@@ -93,6 +94,11 @@ struct rgf_handle_s {
   std::string prof_kernel;
   double probe = 0.0;
   DevBuf gepp;  // scratch of the whole-column pivoting (per-step engine)
+  // a structure swept in parts: augmented matrices, exchange buffers, flags,
+  // probe tables; per chain of joins (left, right) operands and matrices
+  DevBuf sp_m, sp_x, sp_sync, sp_tab, sp_t[2], sp_f[2], sp_q[2][2], sp_p[2], sp_w[2], sp_s[2];
+  cudaStream_t aux_stream = nullptr;  // the right chain's joins
+  cudaEvent_t aux_ev[2] = {nullptr, nullptr};
   // tuned tile table of the persistent engine: rows Rp <= tile_rmax[i] use
   // tile tile_bm[i] (first match) when its grid fits the GPU
   std::vector<int64_t> tile_rmax;
@@ -516,13 +522,13 @@ void gang_arrive_locked(GangBatch* g) {
   }
 }
 
-// a worker's sweep: wait until the gang launch has run it
-cudaError_t gang_run(GangBatch* g, const PersistParams& pp, int BM, int ctas) {
+// a worker's sweeps: wait until the gang launch has run them
+cudaError_t gang_run(GangBatch* g, const PersistParams* pp, int count) {
   std::unique_lock<std::mutex> lock(g->mu);
   // cost estimate (seconds) for the queue order and the scheduler's bound:
   // steps x ~25 us per step on 96 x 96 tiles
-  g->subs.push_back({pp, ctas, (double)pp.L * pp.NB * 25e-6});
-  (void)BM;
+  for (int q = 0; q < count; q++)
+    g->subs.push_back({pp[q], pp[q].TR * pp[q].TC + kPersistExtraCtas, (double)pp[q].L * pp[q].NB * 25e-6});
   gang_arrive_locked(g);
   g->cv.wait(lock, [&] { return g->done; });
   return g->result;
@@ -544,6 +550,9 @@ constexpr double kProbeRetry = 1e-10;
 constexpr double kProbeIllcond = 1e-8;
 // internal status of smatrix_run: recompute with engine 1
 constexpr rgf_status kRetryWholeColumn = static_cast<rgf_status>(1000);
+// internal status of smatrix_run: a part of a split sweep failed its check, or
+// did not fit; recompute as one sweep
+constexpr rgf_status kRetryUnsplit = static_cast<rgf_status>(1001);
 
 // Segment sweep of an L-split S-matrix: the slices [0, cut) swept from the
 // left lead (side 0) or [cut, L) from the right lead (side 1), carrying only
@@ -557,8 +566,360 @@ struct SegReq {
   rgf_cplx* state;
 };
 
+void set_waits(rgf_handle h, PersistParams* pp) {
+  const int clk_khz = clock_khz(h->device);
+  // bound of every device-side wait: ~4 s, or RGF_WAIT_TIMEOUT_MS
+  const char* tmo_env = getenv("RGF_WAIT_TIMEOUT_MS");
+  const double tmo_ms = (tmo_env && atof(tmo_env) > 0) ? atof(tmo_env) : 4000.0;
+  pp->timeout_cycles = (long long)(clk_khz * tmo_ms);
+  // RGF_TEST_WITHHOLD_T=1 (failure-detection tests): the T-server never
+  // releases its T flag, so every dependent wait runs out
+  const char* wh_env = getenv("RGF_TEST_WITHHOLD_T");
+  pp->withhold_t = (wh_env && atoi(wh_env) == 1) ? 1 : 0;
+  pp->trace = nullptr;  // per-step event timestamps: a development aid, off in the library
+  pp->trace_steps = 0;
+}
+
+// ---------------------------------------------------------------------------
+// A structure cut along its length into parts swept side by side.
+//
+// A sweep is a chain of L ceil(N / 32) pivot blocks, ~15 us each whatever the
+// matrix's size, and below N ~ 700 its tiles leave most SMs idle.  So the
+// slices are cut: the outer parts start from their leads as the unsplit sweep
+// does, carrying their own side's channels; an inner part starts from a lead of
+// its half's side that is not there, and carries the unit sources of its first
+// slice, so that its state holds the four blocks
+//     [[g', X'], [Z', Y']] = [[G'_ee, G'_ea], [G'_ae, G'_aa]]
+// of its own Green's function between its first slice a and last slice e.  All
+// parts run in one cooperative launch.  Then, from each lead inwards, the state
+// [[g, X], [Z, Y]] of what has been joined so far takes in the next inner part:
+// the true self-energy of slice a is g, not the absent lead's G0, so with
+// D = G0 - g
+//     G = G' - G'_{.a} (1 + D Y')^{-1} D G'_{a.},
+// and X, Z, Y follow over the hopping between the parts.  All of it is the
+// corner of one sweep (N pivots, whole-column pivoting) of
+//     [[1 + D Y',  D Z',  -X],
+//      [X',        g',     0],
+//      [Z Y',      Z Z',   Y]].
+// The two halves meet as in segment_merge.  The absent leads keep every slice
+// matrix as well conditioned as in the unsplit sweep (an isolated part could
+// resonate); every slice inverse is probed as there, and a part that fails its
+// check sends the call to the unsplit sweep.
+// ---------------------------------------------------------------------------
+struct SplitPlan {
+  int parts = 1, left = 0;  // parts in all, those of the left half (outer one included)
+  int tile = 0;
+};
+
+struct SplitProblem {
+  int64_t N, L;
+  int ni[2], no[2];          // requested channels, left / right
+  const int *in_idx[2], *out_idx[2];
+  const SideDev* side[2];
+  const double2* G0[2];
+  const double2* phi;
+  const int* st_col;
+  const double2* st_val;
+  const double2* eps;
+  double2 k2;
+  int* status;
+  unsigned long long* probe;
+};
+
+int64_t part_cols(int64_t N, int ni) { return ((N + ni + 1) & ~(int64_t)1) + 2; }
+int64_t part_ctas(int64_t N, int no, int ni, int tile) {
+  const int64_t R = N + no, C = part_cols(N, ni);
+  return ((R + tile - 1) / tile) * ((C + tile - 1) / tile) + kPersistExtraCtas;
+}
+
+// us of one slice of the persistent sweep with NB pivot blocks on tiles of
+// 96, 64, 32 (measured at N = 64, 157, 256, 512, 1000: 98, 146, 175, 302, 553;
+// 50, 93, 136, 253; 40, 85, 128), and of one join
+double slice_us(int tile, int64_t NB) {
+  return tile == 96 ? 66.0 + 15.0 * NB : tile == 64 ? 21.6 + 14.3 * NB : 11.3 + 14.55 * NB;
+}
+double join_us(int64_t NB) { return 40.0 + 45.0 * NB; }
+
+// The number of parts and the tile.  More parts shorten the chain of slices and
+// lengthen the chain of joins; smaller tiles run a slice faster and take more
+// CTAs.  Against the unsplit sweep (ms, best tile of each): N = 64, L = 200:
+// 8.5, 4.5 in two parts, 2.0 in seven, 1.9 in twelve; N = 157, L = 263: 22.6,
+// 11.8 in two, 5.5 in six; N = 576, L = 300: 88, 57 in two (no room for more);
+// the sums below pick within 5% of the fastest of these.  From N ~ 770 on not
+// even two grids fit the GPU.
+bool plan_split(const rgf_handle h, const SplitProblem& p, SplitPlan* plan) {
+  const int64_t NB = (p.N + 31) / 32;
+  const bool gang = h->gang != nullptr;  // throughput: only the two outer parts, on the gang launch's tile
+  if (gang && !h->gang->halves) return false;
+  if (!gj_step_fits(2 * p.N + std::max(p.no[0], p.no[1])) || !gj_step_fits(p.N + p.no[0] + p.no[1])) return false;
+  double best = 0.0;
+  for (int tile : {96, 64, 32}) {
+    if (gang && tile != 96) break;
+    const int64_t outer = part_ctas(p.N, p.no[0], p.ni[0], tile) + part_ctas(p.N, p.no[1], p.ni[1], tile);
+    const int64_t inner = part_ctas(p.N, (int)p.N, (int)p.N, tile);
+    for (int parts = 2; parts <= kPersistMaxParts && parts * 2 <= p.L; parts++) {
+      if (outer + (parts - 2) * inner > h->sms || (gang && parts > 2)) break;
+      const double t = (double)((p.L + parts - 1) / parts) * slice_us(tile, NB) + join_us(NB) * (1 + (parts - 1) / 2);
+      if (plan->tile == 0 || t < best) {
+        best = t;
+        plan->tile = tile;
+        plan->parts = parts;
+        plan->left = (parts + 1) / 2;
+      }
+    }
+  }
+  // the unsplit sweep on the tile it would take, and its far lead
+  double whole = 0.0;
+  for (int tile : {96, 64, 32}) {
+    if (gang && tile != 96) break;
+    if (part_ctas(p.N, p.no[1], p.ni[1], tile) > h->sms) continue;
+    const double t = (double)p.L * slice_us(tile, NB) + join_us(NB);
+    if (whole == 0.0 || t < whole) whole = t;
+  }
+  return plan->tile != 0 && best < whole;
+}
+
+// one part: its matrix, and its exchange buffers on tiles of T x T
+struct PartBuf {
+  int64_t R, ldm, pc1, TR, TC;
+  int64_t matrix, exchange, flags, cons;  // sizes (double2, double2, int, int)
+};
+PartBuf part_buf(int64_t N, int no, int ni, int T) {
+  PartBuf b;
+  b.R = N + no;
+  b.pc1 = (N + ni + 1) & ~(int64_t)1;
+  b.ldm = b.pc1 + 2;
+  b.TR = (b.R + T - 1) / T;
+  b.TC = (b.ldm + T - 1) / T;
+  b.matrix = b.R * b.ldm;
+  b.exchange = 2 * b.TR * T * 32 + 6 * b.TC * 32 * T + 11 * 32 * 32;
+  b.flags = (persist_flag_words((int)b.TR, (int)b.TC) + 31) & ~31;
+  b.cons = (persist_cons_words((int)b.TR, (int)b.TC) + 1 + 31) & ~31;
+  return b;
+}
+
+// sweep of the slices first, first + step, .. (n of them) of a part
+PersistParams part_params(rgf_handle h, const SplitProblem& p, const PartBuf& b, int T, int64_t first, int step, int64_t n,
+                          double2* M, double2* x, int* flags, int* cons) {
+  PersistParams w;
+  w.N = (int)p.N;
+  w.R = (int)b.R;
+  w.C = (int)b.ldm;
+  w.TR = (int)b.TR;
+  w.TC = (int)b.TC;
+  w.NB = (int)((p.N + sweep_block_width() - 1) / sweep_block_width());
+  w.L = (int)n;
+  w.M = M;
+  w.ldm = b.ldm;
+  w.eps = p.eps;
+  w.eps_first = first;
+  w.eps_step = step;
+  w.k2 = p.k2;
+  w.st_col = p.st_col;
+  w.st_val = p.st_val;
+  w.pc1 = (int)b.pc1;
+  w.probe = as<double2>(h->sp_tab);
+  w.pcbuf = x;
+  w.rowbuf = w.pcbuf + 2 * b.TR * T * 32;
+  w.prebuf = w.rowbuf + 2 * b.TC * 32 * T;
+  w.ubuf = w.prebuf + 2 * b.TC * 32 * T;
+  w.tbuf = w.ubuf + 2 * b.TC * 32 * T;
+  w.djjbuf = w.tbuf + 2 * 32 * 32;
+  w.srvbuf = w.tbuf + 3 * 32 * 32;
+  w.ybuf = w.tbuf + 7 * 32 * 32;
+  w.flags = flags;
+  w.cons = cons;
+  w.abort = cons + persist_cons_words((int)b.TR, (int)b.TC);
+  w.snap = nullptr;
+  w.snap_mod = 1;
+  w.snap_ld = b.matrix;
+  w.status = p.status;
+  w.probe_max = p.probe;
+  set_waits(h, &w);
+  return w;
+}
+
+// the stream and events of work that runs beside the handle's stream
+rgf_status second_stream(rgf_handle h) {
+  if (h->aux_stream) return RGF_OK;
+  for (cudaEvent_t& ev : h->aux_ev) RGF_CUDA_TRY(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+  RGF_CUDA_TRY(cudaStreamCreateWithFlags(&h->aux_stream, cudaStreamNonBlocking));
+  return RGF_OK;
+}
+
+// sweep of a join matrix Q (R x C, leading dimension C): N pivots over the
+// whole column with the buffers of chain c; only the corner is kept up to date
+// unless `whole`
+rgf_status join_sweep(rgf_handle h, const SplitProblem& p, double2* Q, int64_t R, int64_t C, int c, bool whole,
+                      cudaStream_t s) {
+  const int kSwW = sweep_block_width();
+  for (int64_t j0 = 0; j0 < p.N; j0 += kSwW) {
+    const int jn = (int)std::min<int64_t>(kSwW, p.N - j0);
+    RGF_CUDA_TRY(launch_gj_panel(Q, C, R, p.N, j0, jn, !whole, as<double2>(h->sp_p[c]), h->sp_s[c].p, p.status, s));
+    launch_gj_update(Q, C, R, p.N, C, j0, jn, !whole, as<double2>(h->sp_p[c]), as<double2>(h->sp_w[c]), h->sp_s[c].p, s);
+    h->launches += 3;
+  }
+  if (whole) {
+    RGF_CUDA_TRY(launch_gepp_unpermute(Q, C, R, p.N, h->sp_s[c].p, s));
+    h->launches += 2;
+  }
+  return RGF_OK;
+}
+
+SplitPart init_part(const rgf_handle h, const SplitProblem& p, const PartBuf& b, int side, bool inner, int64_t first,
+                    double2* M) {
+  SplitPart sp;
+  sp.M = M;
+  sp.ldm = b.ldm;
+  sp.eps = p.eps + first * p.N;
+  sp.G0 = p.G0[side];
+  sp.g0v = as<double2>(h->sp_tab) + (2 + side) * p.N;
+  sp.inner = inner;
+  sp.ni = inner ? (int)p.N : p.ni[side];
+  sp.no = inner ? (int)p.N : p.no[side];
+  sp.pc1 = (int)b.pc1;
+  sp.prop = p.side[side]->prop;
+  sp.lam = p.side[side]->lam;
+  sp.mu = p.side[side]->sqrtmu;
+  sp.in_idx = p.in_idx[side];
+  sp.out_idx = p.out_idx[side];
+  return sp;
+}
+
+rgf_status split_sweep(rgf_handle h, const SplitProblem& p, const SplitPlan& plan, const double2** Q_out,
+                       int64_t* ldQ_out) {
+  rgf_status st;
+  const int64_t N = p.N, L = p.L;
+  const int kSwW = sweep_block_width(), P = plan.parts, T = plan.tile;
+  struct Part {
+    int side, inner;
+    int64_t lo, n;  // physical slices [lo, lo + n)
+    PartBuf b;
+    double2* M;
+  };
+  std::vector<Part> part(P);
+  int64_t m_sz = 0, x_sz = 0, nflag = 0, ncons = 0;
+  for (int q = 0; q < P; q++) {  // in physical order, left to right
+    Part& a = part[q];
+    a.side = q < plan.left ? 0 : 1;
+    a.inner = q != 0 && q != P - 1;
+    a.lo = L * q / P;
+    a.n = L * (q + 1) / P - a.lo;
+    a.b = part_buf(N, a.inner ? (int)N : p.no[a.side], a.inner ? (int)N : p.ni[a.side], T);
+    m_sz += a.b.matrix;
+    x_sz += a.b.exchange;
+    nflag += a.b.flags;
+    ncons += a.b.cons;
+  }
+  if ((st = ensure(h, h->sp_m, sizeof(double2) * m_sz))) return st;
+  if ((st = ensure(h, h->sp_x, sizeof(double2) * x_sz))) return st;
+  if ((st = ensure(h, h->sp_sync, sizeof(int) * (nflag + ncons)))) return st;
+  if ((st = ensure(h, h->sp_tab, sizeof(double2) * 4 * N))) return st;
+  const int64_t n_out = p.no[0] + p.no[1], n_in = p.ni[0] + p.ni[1];
+  for (int c = 0; c < 2; c++) {
+    const int inners = (c == 0 ? plan.left : P - plan.left) - 1;
+    const int64_t Ri = 2 * N + p.no[c], Ci = 2 * N + p.ni[c];
+    const int64_t Rm = c == 0 ? std::max(Ri, N + n_out) : Ri, Cm = c == 0 ? std::max(Ci, N + n_in) : Ci;
+    if (inners == 0 && c == 1) continue;  // the halves are joined with the left chain's buffers
+    const int64_t f_sz = std::max((N + p.no[c]) * 2 * N, c == 0 ? (N + p.no[1]) * (N + p.ni[0]) : 0);
+    if ((st = ensure(h, h->sp_f[c], sizeof(double2) * f_sz))) return st;
+    if ((st = ensure(h, h->sp_t[c], sizeof(double2) * (N + p.no[c]) * N))) return st;
+    for (int k = 0; k < 2; k++)
+      if ((st = ensure(h, h->sp_q[c][k], sizeof(double2) * Rm * Cm))) return st;
+    if ((st = ensure(h, h->sp_p[c], sizeof(double2) * Rm * kSwW))) return st;
+    if ((st = ensure(h, h->sp_w[c], sizeof(double2) * Cm * kSwW))) return st;
+    if ((st = ensure(h, h->sp_s[c], gepp_scratch_bytes(N)))) return st;
+  }
+  double2* tab = as<double2>(h->sp_tab);
+  launch_split_tables(p.st_col, p.st_val, N, p.G0[0], p.G0[1], tab, h->stream);
+  int* flags = as<int>(h->sp_sync);
+  int* cons = flags + nflag;
+  RGF_CUDA_TRY(cudaMemsetAsync(flags, 0xFF, sizeof(int) * nflag, h->stream));
+  RGF_CUDA_TRY(cudaMemsetAsync(cons, 0, sizeof(int) * ncons, h->stream));
+  SplitInit init;
+  init.N = N;
+  init.phi = p.phi;
+  init.st_col = p.st_col;
+  init.st_val = p.st_val;
+  init.k2 = p.k2;
+  init.tab = tab;
+  std::vector<PersistParams> pp(P);
+  double2* m = as<double2>(h->sp_m);
+  double2* x = as<double2>(h->sp_x);
+  for (int q = 0; q < P; q++) {
+    Part& a = part[q];
+    const int64_t first = a.side == 0 ? a.lo : a.lo + a.n - 1;
+    a.M = m;
+    init.part[q] = init_part(h, p, a.b, a.side, a.inner, first, m);
+    pp[q] = part_params(h, p, a.b, T, first, a.side == 0 ? 1 : -1, a.n, m, x, flags, cons);
+    m += a.b.matrix;
+    x += a.b.exchange;
+    flags += a.b.flags;
+    cons += a.b.cons;
+  }
+  launch_split_init(init, P, h->stream);
+  h->launches += 2;
+  cudaError_t e;
+  if (h->gang) {
+    RGF_CUDA_TRY(cudaStreamSynchronize(h->stream));
+    h->gang_submitted = true;
+    e = gang_run(h->gang, pp.data(), P);
+  } else {
+    e = launch_persist(pp.data(), P, T, T, h->stream);
+  }
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return kRetryUnsplit;  // e.g. the cooperative launch does not fit
+  }
+  h->launches++;
+
+  // ---- join from the leads inwards ----
+  const double2* state[2];
+  int64_t lds[2];
+  const bool two = P - plan.left > 1 && plan.left > 1;  // both halves have inner parts
+  if (two) {
+    if ((st = second_stream(h))) return st;
+    RGF_CUDA_TRY(cudaEventRecord(h->aux_ev[0], h->stream));
+    RGF_CUDA_TRY(cudaStreamWaitEvent(h->aux_stream, h->aux_ev[0], 0));
+  }
+  int flip[2] = {0, 0};
+  for (int c = 0; c < 2; c++) {
+    const cudaStream_t s = c == 1 && two ? h->aux_stream : h->stream;
+    const int outer = c == 0 ? 0 : P - 1, step = c == 0 ? 1 : -1, n = (c == 0 ? plan.left : P - plan.left) - 1;
+    state[c] = part[outer].M;
+    lds[c] = part[outer].b.ldm;
+    for (int k = 1; k <= n; k++) {
+      const Part& in = part[outer + step * k];
+      double2* Q = as<double2>(h->sp_q[c][flip[c]]);
+      flip[c] ^= 1;
+      const int64_t ldQ = 2 * N + p.ni[c];
+      launch_join_inner(state[c], lds[c], in.M, in.b.ldm, p.G0[c], N, p.ni[c], p.no[c], as<double2>(h->sp_t[c]),
+                        as<double2>(h->sp_f[c]), Q, ldQ, s);
+      h->launches += 3;
+      if ((st = join_sweep(h, p, Q, 2 * N + p.no[c], ldQ, c, false, s))) return st;
+      state[c] = Q + N * ldQ + N;
+      lds[c] = ldQ;
+    }
+  }
+  if (two) {
+    RGF_CUDA_TRY(cudaEventRecord(h->aux_ev[1], h->aux_stream));
+    RGF_CUDA_TRY(cudaStreamWaitEvent(h->stream, h->aux_ev[1], 0));
+  }
+  double2* Q = as<double2>(h->sp_q[0][flip[0]]);
+  const int64_t ldQ = N + n_in;
+  launch_join_ends(state[0], lds[0], state[1], lds[1], N, p.ni[0], p.ni[1], p.no[0], p.no[1], as<double2>(h->sp_f[0]), Q,
+                   ldQ, h->stream);
+  h->launches += 2;
+  if ((st = join_sweep(h, p, Q, N + n_out, ldQ, 0, false, h->stream))) return st;
+  if ((st = check_launch())) return st;
+  *Q_out = Q;
+  *ldQ_out = ldQ;
+  return RGF_OK;
+}
+
 rgf_status smatrix_run(rgf_handle h, const Problem& p, const rgf_request* req, const rgf_options* opt, rgf_cplx* S,
-                       int64_t ldS, rgf_channels* ch, const GradReq* gr, int engine, const SegReq* seg) {
+                       int64_t ldS, rgf_channels* ch, const GradReq* gr, int engine, const SegReq* seg,
+                       bool may_split) {
   rgf_status st;
   h->launches = 0;
   h->probe = 0.0;
@@ -681,6 +1042,9 @@ rgf_status smatrix_run(rgf_handle h, const Problem& p, const rgf_request* req, c
   in_lr.insert(in_lr.end(), rq.in[1].begin(), rq.in[1].end());
   out_lr.insert(out_lr.end(), rq.out[1].begin(), rq.out[1].end());
   size_t o_in_lr = push(in_lr), o_out_lr = push(out_lr);
+  std::vector<int> ident(h->arena ? 0 : std::max(n_out, n_in));  // rows and columns in S's own order (split sweep)
+  for (size_t q = 0; q < ident.size(); q++) ident[q] = (int)q;
+  const size_t o_ident = push(ident);
   if ((st = ensure(h, h->idx, sizeof(int) * (idx.size() + 1)))) return st;
   int* idx_d = as<int>(h->idx);
   RGF_CUDA_TRY(cudaMemcpyAsync(idx_d, idx.data(), sizeof(int) * idx.size(), cudaMemcpyHostToDevice, h->stream));
@@ -788,10 +1152,69 @@ rgf_status smatrix_run(rgf_handle h, const Problem& p, const rgf_request* req, c
     h->mx_fallback = 1;  // S from the FP64 form
   }
 
-  // (6) initial augmented matrix
-  double2* M = as<double2>(h->aug);
   const int* st_col = as<int>(h->st_col);
   const double2* st_val = as<double2>(h->st_val);
+
+  // (5c) parts swept side by side where that is faster
+  if (may_split && engine == 0 && L > 0 && !gr && !seg && !h->arena && !h->sm_budget && !(opt && opt->profile > 0)) {
+    SplitProblem sp;
+    SplitPlan plan;
+    sp.N = N;
+    sp.L = L;
+    const size_t lr[4] = {s == 0 ? o_in_s : o_in_e, s == 0 ? o_in_e : o_in_s, s == 0 ? o_out_s : o_out_e,
+                          s == 0 ? o_out_e : o_out_s};
+    for (int q = 0; q < 2; q++) {
+      sp.ni[q] = (int)rq.in[q].size();
+      sp.no[q] = (int)rq.out[q].size();
+      sp.in_idx[q] = idx_d + lr[q];
+      sp.out_idx[q] = idx_d + lr[2 + q];
+      sp.side[q] = &ci.side[q];
+      sp.G0[q] = q == s ? g0s : g0e;
+    }
+    sp.phi = phi;
+    sp.st_col = st_col;
+    sp.st_val = st_val;
+    sp.eps = eps_d;
+    sp.k2 = k2;
+    sp.status = status;
+    if (plan_split(h, sp, &plan)) {
+      if ((st = ensure(h, h->xprobe, sizeof(unsigned long long)))) return st;
+      sp.probe = as<unsigned long long>(h->xprobe);
+      RGF_CUDA_TRY(cudaMemsetAsync(sp.probe, 0, sizeof(unsigned long long), h->stream));
+      const double2* Q = nullptr;
+      int64_t ldQ = 0;
+      if ((st = split_sweep(h, sp, plan, &Q, &ldQ))) return st;
+      double2* Sd = S_dev ? reinterpret_cast<double2*>(S) : as<double2>(h->sdev);
+      launch_extract(Q, ldQ, N, idx_d + o_ident, n_out, idx_d + o_ident, n_in, Sd, S_dev ? ldS : n_out, idx_d + o_pairs,
+                     npairs, h->stream);
+      h->launches += 1 + (npairs > 0 ? 1 : 0);
+      if ((st = check_launch())) return st;
+      if (!S_dev)
+        RGF_CUDA_TRY(cudaMemcpy2DAsync(S, sizeof(rgf_cplx) * ldS, Sd, sizeof(double2) * n_out,
+                                       sizeof(double2) * n_out, n_in, cudaMemcpyDeviceToHost, h->stream));
+      int hstatus = 0;
+      unsigned long long bits = 0;
+      RGF_CUDA_TRY(cudaMemcpyAsync(&hstatus, status, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+      RGF_CUDA_TRY(cudaMemcpyAsync(&bits, sp.probe, sizeof(bits), cudaMemcpyDeviceToHost, h->stream));
+      RGF_CUDA_TRY(cudaStreamSynchronize(h->stream));
+      memcpy(&h->probe, &bits, sizeof(double));
+      h->prof_n = 0;
+      h->prof_ms = h->prof_flops = 0.0;
+      if (hstatus & kStatusNonfinite) {
+        set_error("syst.epsilon contains NaN or Inf");
+        return RGF_ERR_NONFINITE;
+      }
+      if (hstatus & kStatusTimeout) {
+        set_error("a device-side wait timed out");
+        return RGF_ERR_TIMEOUT;
+      }
+      if ((hstatus & kStatusSingular) || !(h->probe <= kProbeRetry)) return kRetryUnsplit;
+      return copy_channels_out(h, tr, ci, ch);
+    }
+  }
+
+  // (6) initial augmented matrix
+  double2* M = as<double2>(h->aug);
   const double2 eps_e = d2(e == 0 ? p.epsL : p.epsR);
   launch_fill_init(M, ldm, N, phi, N, sd_s.prop, sd_s.lam, sd_s.sqrtmu, idx_d + o_in_s, ni_s, idx_d + o_out_s,
                    no_s, h->stream);
@@ -946,17 +1369,7 @@ rgf_status smatrix_run(rgf_handle h, const Problem& p, const rgf_request* req, c
       pp.snap_ld = Rp * ldm;
       pp.status = status;
       pp.probe_max = probe_d;
-      const int clk_khz = clock_khz(h->device);
-      // bound of every device-side wait: ~4 s, or RGF_WAIT_TIMEOUT_MS
-      const char* tmo_env = getenv("RGF_WAIT_TIMEOUT_MS");
-      const double tmo_ms = (tmo_env && atof(tmo_env) > 0) ? atof(tmo_env) : 4000.0;
-      pp.timeout_cycles = (long long)(clk_khz * tmo_ms);
-      // RGF_TEST_WITHHOLD_T=1 (failure-detection tests): the T-server never
-      // releases its T flag, so every dependent wait runs out
-      const char* wh_env = getenv("RGF_TEST_WITHHOLD_T");
-      pp.withhold_t = (wh_env && atoi(wh_env) == 1) ? 1 : 0;
-      pp.trace = nullptr;  // per-step event timestamps: a development aid, off in the library
-      pp.trace_steps = 0;
+      set_waits(h, &pp);
       const bool timed = prof_every > 0;
       if (timed) {
         while (h->ev.size() < ev_used + 2) {
@@ -983,9 +1396,9 @@ rgf_status smatrix_run(rgf_handle h, const Problem& p, const rgf_request* req, c
         // smaller tiles sweeps on its own before the gang launch
         RGF_CUDA_TRY(cudaStreamSynchronize(h->stream));
         h->gang_submitted = true;
-        e = gang_run(h->gang, pp, BMp, need);
+        e = gang_run(h->gang, &pp, 1);
       } else {
-        e = launch_persist(pp, BMp, BNp, h->stream);
+        e = launch_persist(&pp, 1, BMp, BNp, h->stream);
       }
       if (h->sm_budget) {
         const cudaError_t se = cudaStreamSynchronize(h->stream);
@@ -1238,12 +1651,17 @@ rgf_status smatrix(rgf_handle h, const Problem& p, const rgf_request* req, const
   h->fallback = 0;
   h->mx_form = RGF_FP64;
   h->mx_fallback = 0;
-  rgf_status st = smatrix_run(h, p, req, opt, S, ldS, ch, gr, engine, seg);
+  rgf_status st = smatrix_run(h, p, req, opt, S, ldS, ch, gr, engine, seg, true);
+  if (st == kRetryUnsplit) {
+    rgf_options o1 = opt ? *opt : rgf_options{};
+    o1.precision = RGF_FP64;
+    st = smatrix_run(h, p, req, &o1, S, ldS, ch, gr, engine, seg, false);
+  }
   if (st == kRetryWholeColumn) {
     const double probe0 = h->probe;
     rgf_options o2 = opt ? *opt : rgf_options{};
     o2.precision = RGF_FP64;  // a split-precision attempt, if any, has already been made
-    st = smatrix_run(h, p, req, &o2, S, ldS, ch, gr, 1, seg);
+    st = smatrix_run(h, p, req, &o2, S, ldS, ch, gr, 1, seg, false);
     h->fallback = 1;
     h->probe_first = probe0;
   }
@@ -1504,6 +1922,13 @@ rgf_status rgf_destroy(rgf_handle h) {
     if (b->p) cudaFree(b->p);
   for (DevBuf& b : h->mx)
     if (b.p) cudaFree(b.p);
+  for (DevBuf* b : {&h->sp_m, &h->sp_x, &h->sp_sync, &h->sp_tab, &h->sp_t[0], &h->sp_t[1], &h->sp_f[0], &h->sp_f[1],
+                    &h->sp_q[0][0], &h->sp_q[0][1], &h->sp_q[1][0], &h->sp_q[1][1], &h->sp_p[0], &h->sp_p[1],
+                    &h->sp_w[0], &h->sp_w[1], &h->sp_s[0], &h->sp_s[1]})
+    if (b->p) cudaFree(b->p);
+  for (cudaEvent_t ev : h->aux_ev)
+    if (ev) cudaEventDestroy(ev);
+  if (h->aux_stream) cudaStreamDestroy(h->aux_stream);
   for (cudaEvent_t ev : h->ev) cudaEventDestroy(ev);
   if (h->own_stream) cudaStreamDestroy(h->own_stream);
   for (rgf_handle_s* w : h->workers) rgf_destroy(w);
@@ -1562,6 +1987,7 @@ static rgf_status batch_one_launch(rgf_handle h, int64_t count, const rgf_syst2d
     gb[c]->stream = h->stream;
   }
   for (int64_t r = 0; r < count; r++) gb[r % nch]->pending++;
+  for (auto& g : gb) g->halves = 2 * g->pending <= kGangMaxItems;
   std::vector<rgf_handle> ws(count, nullptr);
   std::vector<std::thread> pool;
   for (int64_t r = 0; r < count; r++) {

@@ -131,6 +131,99 @@ __global__ void __launch_bounds__(128) k_zgemm(int64_t M, int64_t N, int64_t K, 
   }
 }
 
+// The same product on 32 x 32 tiles (4 warps of 16 x 16) for outputs that would
+// leave most SMs without a 64 x 64 tile; the next K chunk is read into
+// registers under the products of the current one.
+template <int kOpA, int kOpB>
+__global__ void __launch_bounds__(128) k_zgemm_small(int64_t M, int64_t N, int64_t K, double2 alpha, ZOp A, ZOp B,
+                                                     double2* C, int64_t ldc, ZAdd add) {
+  __shared__ double2 As[32][kBK + 4], Bs[kBK][32 + 2];
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5, wr = warp >> 1, wc = warp & 1;
+  const int64_t m0 = (int64_t)blockIdx.y * 32, n0 = (int64_t)blockIdx.x * 32;
+  double acc[2][2][4];
+#pragma unroll
+  for (int i = 0; i < 2; i++)
+#pragma unroll
+    for (int j = 0; j < 2; j++)
+#pragma unroll
+      for (int q = 0; q < 4; q++) acc[i][j][q] = 0.0;
+  const ZOp oa{A.p, A.ld, kOpA}, ob{B.p, B.ld, kOpB};
+  double2 va[8], vb[8];
+  auto fetch = [&](int64_t k0) {
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+      const int x = lane, y = warp + 4 * i;  // x along the contiguous axis of each operand
+      const int64_t ar = m0 + (kOpA == 0 ? y : x), ak = k0 + (kOpA == 0 ? x : y);
+      const int64_t bk = k0 + (kOpB == 0 ? y : x), bc = n0 + (kOpB == 0 ? x : y);
+      va[i] = (ar < M && ak < K) ? zop_load(oa, ar, ak) : cmk(0.0, 0.0);
+      vb[i] = (bk < K && bc < N) ? zop_load(ob, bk, bc) : cmk(0.0, 0.0);
+    }
+  };
+  fetch(0);
+  for (int64_t k0 = 0; k0 < K; k0 += kBK) {
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+      const int x = lane, y = warp + 4 * i;
+      As[kOpA == 0 ? y : x][kOpA == 0 ? x : y] = va[i];
+      Bs[kOpB == 0 ? y : x][kOpB == 0 ? x : y] = vb[i];
+    }
+    __syncthreads();
+    if (k0 + kBK < K) fetch(k0 + kBK);
+#pragma unroll
+    for (int kk = 0; kk < kBK / 4; kk++) {
+      double2 a[2], b[2];
+#pragma unroll
+      for (int i = 0; i < 2; i++) {
+        a[i] = As[wr * 16 + i * 8 + (lane >> 2)][kk * 4 + (lane & 3)];
+        b[i] = Bs[kk * 4 + (lane & 3)][wc * 16 + i * 8 + (lane >> 2)];
+      }
+#pragma unroll
+      for (int i = 0; i < 2; i++)
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+          dmma884(acc[i][j][0], acc[i][j][1], a[i].x, b[j].x);
+          dmma884(acc[i][j][2], acc[i][j][3], a[i].x, b[j].y);
+        }
+#pragma unroll
+      for (int i = 0; i < 2; i++)
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+          dmma884(acc[i][j][0], acc[i][j][1], -a[i].y, b[j].y);
+          dmma884(acc[i][j][2], acc[i][j][3], a[i].y, b[j].x);
+        }
+    }
+    __syncthreads();
+  }
+#pragma unroll
+  for (int i = 0; i < 2; i++) {
+    const int64_t r = m0 + wr * 16 + i * 8 + (lane >> 2);
+    if (r >= M) continue;
+#pragma unroll
+    for (int j = 0; j < 2; j++)
+#pragma unroll
+      for (int h = 0; h < 2; h++) {
+        const int64_t c = n0 + wc * 16 + j * 8 + (lane & 3) * 2 + h;
+        if (c >= N) continue;
+        double2 v = cmul(alpha, cmk(acc[i][j][h], acc[i][j][2 + h]));
+        if (add.p && r < add.rows && c < add.cols) v = cadd(v, add.p[r * add.ld + c]);
+        C[r * ldc + c] = v;
+      }
+  }
+}
+
+// 64 x 64 tiles below this many: a 32 x 32 tile takes a quarter of the time, and
+// four times as many still run at once (64^3: 28 us against 9 us)
+constexpr int64_t kSmallTiles = 75;
+static bool zgemm_small(int64_t M, int64_t N, int64_t K, double2 alpha, ZOp A, ZOp B, double2* C, int64_t ldc, ZAdd add,
+                        cudaStream_t s) {
+  if (((M + kBM - 1) / kBM) * ((N + kBN - 1) / kBN) >= kSmallTiles || A.op != 0) return false;
+  const dim3 grid((unsigned)((N + 31) / 32), (unsigned)((M + 31) / 32));
+  if (B.op == 0) k_zgemm_small<0, 0><<<grid, 128, 0, s>>>(M, N, K, alpha, A, B, C, ldc, add);
+  else if (B.op == 1) k_zgemm_small<0, 1><<<grid, 128, 0, s>>>(M, N, K, alpha, A, B, C, ldc, add);
+  else k_zgemm_small<0, 2><<<grid, 128, 0, s>>>(M, N, K, alpha, A, B, C, ldc, add);
+  return true;
+}
+
 static void zgemm_attr() {
   static bool attr = false;
   if (!attr) {
@@ -142,6 +235,7 @@ static void zgemm_attr() {
 
 void launch_zgemm(int64_t M, int64_t N, int64_t K, double2 alpha, ZOp A, ZOp B, double2 beta,
                   double2* C, int64_t ldc, cudaStream_t s) {
+  if (beta.x == 0.0 && beta.y == 0.0 && zgemm_small(M, N, K, alpha, A, B, C, ldc, ZAdd{nullptr, 0, 0, 0}, s)) return;
   zgemm_attr();
   dim3 grid((unsigned)((N + kBN - 1) / kBN), (unsigned)((M + kBM - 1) / kBM));
   k_zgemm<false><<<grid, 128, kGemmSmem, s>>>(M, N, K, alpha, A, B, beta, C, ldc, 0, 0, ZAdd{nullptr, 0, 0, 0});
@@ -150,6 +244,7 @@ void launch_zgemm(int64_t M, int64_t N, int64_t K, double2 alpha, ZOp A, ZOp B, 
 // C = A B + add (add read in its rows x cols corner, zero elsewhere)
 void launch_zgemm_add(int64_t M, int64_t N, int64_t K, ZOp A, ZOp B, ZAdd add, double2* C, int64_t ldc,
                       cudaStream_t s) {
+  if (zgemm_small(M, N, K, cmk(1.0, 0.0), A, B, C, ldc, add, s)) return;
   zgemm_attr();
   dim3 grid((unsigned)((N + kBN - 1) / kBN), (unsigned)((M + kBM - 1) / kBM));
   k_zgemm<false><<<grid, 128, kGemmSmem, s>>>(M, N, K, cmk(1.0, 0.0), A, B, cmk(0.0, 0.0), C, ldc, 0, 0, add);
@@ -716,44 +811,48 @@ __global__ void __launch_bounds__(256) k_pivot_rows(double2* W, int64_t ldm, int
   }
 }
 
-// W <- W_mod + P Wr on rows [r0, R) and columns [c0, Cc).  The old W goes
-// straight into the accumulators while the operands come by cp.async, and
-// three CTAs share an SM, so that one's loads run under another's products.
-__global__ void __launch_bounds__(128, 3) k_gj_update(double2* W, int64_t ldm, int64_t r0, int64_t R, int64_t c0,
-                                                      int64_t Cc, int64_t j0, int jn, const double2* __restrict__ P,
-                                                      const double2* __restrict__ Wr) {
+// W <- W_mod + P Wr on rows [r0, R) and columns [c0, Cc); tiles of 16 kT x 16 kT
+// (4 warps).  The old W goes straight into the accumulators while the operands
+// come by cp.async, and three CTAs of 64 x 64 share an SM, so that one's loads
+// run under another's products (78 us to 35 us at 1600 x 1600); matrices of few
+// 64 x 64 tiles take 32 x 32 ones.
+template <int kT>
+__global__ void __launch_bounds__(128, kT == 4 ? 3 : 4)
+    k_gj_update(double2* W, int64_t ldm, int64_t r0, int64_t R, int64_t c0, int64_t Cc, int64_t j0, int jn,
+                const double2* __restrict__ P, const double2* __restrict__ Wr) {
+  constexpr int kTile = 16 * kT, kBst = kTile + 2;
   extern __shared__ double2 gj_sm[];
-  double2* As = gj_sm;               // [kBM][kAS]
-  double2* Bs = gj_sm + kBM * kAS;   // [kBK][kBS]
+  double2* As = gj_sm;               // [kTile][kAS]
+  double2* Bs = gj_sm + kTile * kAS; // [kBK][kBst]
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5, wr = warp >> 1, wc = warp & 1;
-  const int64_t m0 = r0 + (int64_t)blockIdx.y * kBM, n0 = c0 + (int64_t)blockIdx.x * kBN;
+  const int64_t m0 = r0 + (int64_t)blockIdx.y * kTile, n0 = c0 + (int64_t)blockIdx.x * kTile;
   auto copy16 = [](double2* d, const double2* g, bool in) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(gj_smem(d)), "l"(g), "r"(in ? 16 : 0)
                  : "memory");
   };
 #pragma unroll 4
-  for (int e = t; e < kBM * kBK; e += 128) {
-    const int r = e >> 5, k = e & 31;
+  for (int e = t; e < kTile * kBK; e += 128) {
+    const int r = e / kBK, k = e % kBK;
     const bool in = m0 + r < R;
     copy16(As + r * kAS + k, in ? P + (m0 + r) * kSw + k : P, in);
   }
 #pragma unroll 4
-  for (int e = t; e < kBK * kBN; e += 128) {
-    const int k = e >> 6, c = e & 63;
+  for (int e = t; e < kBK * kTile; e += 128) {
+    const int k = e / kTile, c = e % kTile;
     const bool in = n0 + c < Cc;
-    copy16(Bs + k * kBS + c, in ? Wr + (int64_t)k * ldm + n0 + c : Wr, in);
+    copy16(Bs + k * kBst + c, in ? Wr + (int64_t)k * ldm + n0 + c : Wr, in);
   }
   asm volatile("cp.async.commit_group;" ::: "memory");
-  double acc[4][4][4];
+  double acc[kT][kT][4];
 #pragma unroll
-  for (int mi = 0; mi < 4; mi++) {
-    const int64_t r = m0 + wr * 32 + mi * 8 + (lane >> 2);
+  for (int mi = 0; mi < kT; mi++) {
+    const int64_t r = m0 + wr * 8 * kT + mi * 8 + (lane >> 2);
     const bool rin = r < R && !(r >= j0 && r < j0 + jn);
 #pragma unroll
-    for (int ni = 0; ni < 4; ni++)
+    for (int ni = 0; ni < kT; ni++)
 #pragma unroll
       for (int h = 0; h < 2; h++) {
-        const int64_t c = n0 + wc * 32 + ni * 8 + (lane & 3) * 2 + h;
+        const int64_t c = n0 + wc * 8 * kT + ni * 8 + (lane & 3) * 2 + h;
         const double2 v = (rin && c < Cc && !(c >= j0 && c < j0 + jn)) ? __ldcg(W + r * ldm + c) : cmk(0.0, 0.0);
         acc[mi][ni][h] = v.x;
         acc[mi][ni][2 + h] = v.y;
@@ -763,33 +862,33 @@ __global__ void __launch_bounds__(128, 3) k_gj_update(double2* W, int64_t ldm, i
   __syncthreads();
 #pragma unroll
   for (int kk = 0; kk < kBK / 4; kk++) {
-    double2 b[4];
+    double2 b[kT];
 #pragma unroll
-    for (int ni = 0; ni < 4; ni++) b[ni] = Bs[(kk * 4 + (lane & 3)) * kBS + wc * 32 + ni * 8 + (lane >> 2)];
+    for (int ni = 0; ni < kT; ni++) b[ni] = Bs[(kk * 4 + (lane & 3)) * kBst + wc * 8 * kT + ni * 8 + (lane >> 2)];
 #pragma unroll
-    for (int mi = 0; mi < 4; mi++) {
-      const double2 a = As[(wr * 32 + mi * 8 + (lane >> 2)) * kAS + kk * 4 + (lane & 3)];
+    for (int mi = 0; mi < kT; mi++) {
+      const double2 a = As[(wr * 8 * kT + mi * 8 + (lane >> 2)) * kAS + kk * 4 + (lane & 3)];
 #pragma unroll
-      for (int ni = 0; ni < 4; ni++) {
+      for (int ni = 0; ni < kT; ni++) {
         dmma884(acc[mi][ni][0], acc[mi][ni][1], a.x, b[ni].x);
         dmma884(acc[mi][ni][2], acc[mi][ni][3], a.x, b[ni].y);
       }
 #pragma unroll
-      for (int ni = 0; ni < 4; ni++) {
+      for (int ni = 0; ni < kT; ni++) {
         dmma884(acc[mi][ni][0], acc[mi][ni][1], -a.y, b[ni].y);
         dmma884(acc[mi][ni][2], acc[mi][ni][3], a.y, b[ni].x);
       }
     }
   }
 #pragma unroll
-  for (int mi = 0; mi < 4; mi++) {
-    const int64_t r = m0 + wr * 32 + mi * 8 + (lane >> 2);
+  for (int mi = 0; mi < kT; mi++) {
+    const int64_t r = m0 + wr * 8 * kT + mi * 8 + (lane >> 2);
     if (r >= R) continue;
 #pragma unroll
-    for (int ni = 0; ni < 4; ni++)
+    for (int ni = 0; ni < kT; ni++)
 #pragma unroll
       for (int h = 0; h < 2; h++) {
-        const int64_t c = n0 + wc * 32 + ni * 8 + (lane & 3) * 2 + h;
+        const int64_t c = n0 + wc * 8 * kT + ni * 8 + (lane & 3) * 2 + h;
         if (c < Cc) __stcg(W + r * ldm + c, cmk(acc[mi][ni][h], acc[mi][ni][2 + h]));
       }
   }
@@ -876,15 +975,20 @@ void launch_gj_update(double2* W, int64_t ldm, int64_t R, int64_t N, int64_t Cc,
   const int64_t lo = trailing ? j0 + jn : 0;
   if (lo >= Cc || lo >= R) return;
   k_pivot_rows<<<(unsigned)((Cc - lo + 31) / 32), 256, 0, s>>>(W, ldm, lo, Cc, j0, jn, src, src + kSw, Wr);
+  if (((Cc - lo + kBN - 1) / kBN) * ((R - lo + kBM - 1) / kBM) < kSmallTiles) {
+    const dim3 grid((unsigned)((Cc - lo + 31) / 32), (unsigned)((R - lo + 31) / 32));
+    k_gj_update<2><<<grid, 128, sizeof(double2) * (32 * kAS + kBK * 34), s>>>(W, ldm, lo, R, lo, Cc, j0, jn, P, Wr);
+    return;
+  }
   static std::atomic<bool> attr[kMaxDevices];
   int dev = 0;
   cudaGetDevice(&dev);
   if (!attr[dev & (kMaxDevices - 1)].load()) {
-    cudaFuncSetAttribute(k_gj_update, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGemmSmem);
+    cudaFuncSetAttribute(k_gj_update<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGemmSmem);
     attr[dev & (kMaxDevices - 1)].store(true);
   }
   const dim3 grid((unsigned)((Cc - lo + kBN - 1) / kBN), (unsigned)((R - lo + kBM - 1) / kBM));
-  k_gj_update<<<grid, 128, kGemmSmem, s>>>(W, ldm, lo, R, lo, Cc, j0, jn, P, Wr);
+  k_gj_update<4><<<grid, 128, kGemmSmem, s>>>(W, ldm, lo, R, lo, Cc, j0, jn, P, Wr);
 }
 
 size_t gepp_scratch_bytes(int64_t N) {
@@ -1140,6 +1244,178 @@ double2* probe_tables(void* scratch) { return reinterpret_cast<double2*>(scratch
 
 void launch_probe_tables(const int* st_col, const double2* st_val, int64_t N, void* scratch, cudaStream_t s) {
   k_probe_tables<<<(unsigned)((N + 127) / 128), 128, 0, s>>>(st_col, st_val, N, probe_tables(scratch));
+}
+
+// ---------------------------------------------------------------------------
+// A structure cut along its length into parts swept side by side (split_sweep
+// in rgf_api.cu has the algebra).
+// ---------------------------------------------------------------------------
+// tab: v, A0 v, G0_L v, G0_R v (N entries each), one warp per row
+__global__ void k_split_tables(const int* __restrict__ st_col, const double2* __restrict__ st_val, int64_t N,
+                               const double2* __restrict__ G0L, const double2* __restrict__ G0R,
+                               double2* __restrict__ tab) {
+  const int64_t i = blockIdx.x * (int64_t)(blockDim.x / 32) + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
+  if (i >= N) return;
+  double2 l = cmk(0.0, 0.0), r = cmk(0.0, 0.0);
+  for (int64_t j = lane; j < N; j += 32) {
+    const double2 v = probe_v(j);
+    l = cadd(l, cmul(G0L[i * N + j], v));
+    r = cadd(r, cmul(G0R[i * N + j], v));
+  }
+  for (int off = 16; off > 0; off >>= 1) {
+    l.x += __shfl_xor_sync(0xffffffffu, l.x, off);
+    l.y += __shfl_xor_sync(0xffffffffu, l.y, off);
+    r.x += __shfl_xor_sync(0xffffffffu, r.x, off);
+    r.y += __shfl_xor_sync(0xffffffffu, r.y, off);
+  }
+  if (lane) return;
+  double2 s = cmk(0.0, 0.0);
+  for (int q = 0; q < kMaxStencil; q++) {
+    const int c = st_col[i * kMaxStencil + q];
+    if (c >= 0) s = cadd(s, cmul(st_val[i * kMaxStencil + q], probe_v(c)));
+  }
+  tab[i] = probe_v(i);
+  tab[N + i] = s;
+  tab[2 * N + i] = l;
+  tab[3 * N + i] = r;
+}
+
+void launch_split_tables(const int* st_col, const double2* st_val, int64_t N, const double2* G0L, const double2* G0R,
+                         double2* tab, cudaStream_t s) {
+  k_split_tables<<<(unsigned)((N + 3) / 4), 128, 0, s>>>(st_col, st_val, N, G0L, G0R, tab);
+}
+
+// first augmented slice matrix of every part (grid.z): A - G0 of the part's
+// own side, its carriers (those of the lead's channels, or for an inner part
+// the identity: X = I, -Z = -I, Y = 0) and the probe pair
+__global__ void k_split_init(const __grid_constant__ SplitInit a) {
+  const SplitPart& p = a.part[blockIdx.z];
+  const int64_t N = a.N, j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (j >= p.ldm) return;
+  const double2 zero = cmk(0.0, 0.0);
+  for (int64_t i = blockIdx.y; i < N + p.no; i += gridDim.y) {
+    double2 v = zero;
+    if (j < N) {
+      if (i < N) {
+        v = cneg(p.G0[i * N + j]);
+        for (int q = 0; q < kMaxStencil; q++)
+          if (a.st_col[i * kMaxStencil + q] == j) v = cadd(v, a.st_val[i * kMaxStencil + q]);
+        if (i == j) v = csub(v, cmul(a.k2, p.eps[i]));
+      } else if (p.inner) {
+        v = cmk(i - N == j ? -1.0 : 0.0, 0.0);
+      } else {
+        const int c = p.prop[p.out_idx[i - N]];
+        v = cneg(cmul(cmul(p.mu[c], p.lam[c]), cconj(a.phi[j * N + c])));
+      }
+    } else if (j < N + p.ni) {
+      const int64_t o = i - N, b = j - N;
+      if (p.inner) {
+        v = cmk(i == b ? 1.0 : 0.0, 0.0);
+      } else {
+        const int c = p.prop[p.in_idx[b]];
+        if (i < N) {
+          v = cmul(a.phi[i * N + c], cmul(p.lam[c], p.mu[c]));
+        } else {
+          const int d = p.prop[p.out_idx[o]];
+          v = d == c ? cmul(cmul(p.mu[d], p.lam[d]), p.mu[c]) : zero;
+        }
+      }
+    } else if (j == p.pc1 || j == p.pc1 + 1) {
+      if (i < N) {
+        const double2 pv = a.tab[i];
+        v = j == p.pc1 ? pv : csub(csub(a.tab[N + i], cmul(cmul(a.k2, p.eps[i]), pv)), p.g0v[i]);
+      }
+    }
+    p.M[i * p.ldm + j] = v;
+  }
+}
+
+void launch_split_init(const SplitInit& a, int parts, cudaStream_t s) {
+  int64_t ld = 1, rows = 1;
+  for (int q = 0; q < parts; q++) {
+    ld = std::max(ld, a.part[q].ldm);
+    rows = std::max<int64_t>(rows, a.N + a.part[q].no);
+  }
+  const dim3 grid((unsigned)((ld + 127) / 128), (unsigned)std::min<int64_t>(rows, 4096), (unsigned)parts);
+  k_split_init<<<grid, 128, 0, s>>>(a);
+}
+
+// T = [G0 - g; Z] of an end part's state E = [[g, X], [Z, Y]]
+__global__ void k_join_delta(const double2* __restrict__ E, int64_t ldE, const double2* __restrict__ G0, int64_t N,
+                             int64_t rows, double2* __restrict__ T) {
+  const int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (j >= N) return;
+  for (int64_t i = blockIdx.y; i < rows; i += gridDim.y) {
+    const double2 e = E[i * ldE + j];
+    T[i * N + j] = i < N ? csub(G0[i * N + j], e) : e;
+  }
+}
+
+// the matrix whose sweep joins an end part (state E) with the inner part next
+// to it (state I), F = [G0 - g; Z] [Z_I, Y_I]:
+//   [[1 + (G0 - g) Y_I, (G0 - g) Z_I, -X], [X_I, g_I, 0], [Z Y_I, Z Z_I, Y]]
+__global__ void k_join_inner(const double2* __restrict__ E, int64_t ldE, const double2* __restrict__ I, int64_t ldI,
+                             const double2* __restrict__ F, int64_t N, int ni, int no, double2* __restrict__ Q,
+                             int64_t ldQ) {
+  const int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (j >= 2 * N + ni) return;
+  for (int64_t i = blockIdx.y; i < 2 * N + no; i += gridDim.y) {
+    double2 v;
+    if (i >= N && i < 2 * N) {
+      const double2* row = I + (i - N) * ldI;
+      v = j < N ? row[N + j] : j < 2 * N ? row[j - N] : cmk(0.0, 0.0);
+    } else {
+      const int64_t r = i < N ? i : i - N;  // row of F and of E
+      if (j < 2 * N) {
+        v = F[r * 2 * N + (j < N ? N + j : j - N)];
+        if (i == j) v.x += 1.0;
+      } else {
+        v = E[r * ldE + j - N];
+        if (i < N) v = cneg(v);
+      }
+    }
+    Q[i * ldQ + j] = v;
+  }
+}
+
+// the matrix whose sweep joins the left and the right state (segment_merge has
+// the algebra), F = [g_R; Z_R] [g_L, X_L]
+__global__ void k_join_ends(const double2* __restrict__ L, int64_t ldL, const double2* __restrict__ R, int64_t ldR,
+                            const double2* __restrict__ F, int64_t N, int niL, int niR, int noL, int noR,
+                            double2* __restrict__ Q, int64_t ldQ) {
+  const int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (j >= N + niL + niR) return;
+  const int64_t ldF = N + niL;
+  for (int64_t i = blockIdx.y; i < N + noL + noR; i += gridDim.y) {
+    double2 v;
+    if (i >= N && i < N + noL) {
+      v = j < ldF ? L[i * ldL + j] : cmk(0.0, 0.0);
+      if (j < N) v = cneg(v);
+    } else {
+      const int64_t r = i < N ? i : i - noL;  // row of F and of R
+      v = j < ldF ? F[r * ldF + j] : R[r * ldR + j - niL];
+      if (j < N) v = cmk((i == j ? 1.0 : 0.0) - v.x, -v.y);
+    }
+    Q[i * ldQ + j] = v;
+  }
+}
+
+static dim3 join_grid(int64_t rows, int64_t cols) {
+  return dim3((unsigned)((cols + 127) / 128), (unsigned)std::min<int64_t>(rows, 4096));
+}
+
+void launch_join_inner(const double2* E, int64_t ldE, const double2* I, int64_t ldI, const double2* G0, int64_t N, int ni,
+                       int no, double2* T, double2* F, double2* Q, int64_t ldQ, cudaStream_t s) {
+  k_join_delta<<<join_grid(N + no, N), 128, 0, s>>>(E, ldE, G0, N, N + no, T);
+  launch_zgemm(N + no, 2 * N, N, cmk(1.0, 0.0), ZOp{T, N, 0}, ZOp{I + N * ldI, ldI, 0}, cmk(0.0, 0.0), F, 2 * N, s);
+  k_join_inner<<<join_grid(2 * N + no, 2 * N + ni), 128, 0, s>>>(E, ldE, I, ldI, F, N, ni, no, Q, ldQ);
+}
+
+void launch_join_ends(const double2* L, int64_t ldL, const double2* R, int64_t ldR, int64_t N, int niL, int niR, int noL,
+                      int noR, double2* F, double2* Q, int64_t ldQ, cudaStream_t s) {
+  launch_zgemm(N + noR, N + niL, N, cmk(1.0, 0.0), ZOp{R, ldR, 0}, ZOp{L, ldL, 0}, cmk(0.0, 0.0), F, N + niL, s);
+  k_join_ends<<<join_grid(N + noL + noR, N + niL + niR), 128, 0, s>>>(L, ldL, R, ldR, F, N, niL, niR, noL, noR, Q, ldQ);
 }
 
 // ---------------------------------------------------------------------------

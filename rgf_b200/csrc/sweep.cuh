@@ -86,4 +86,32 @@ void launch_grad_step(const double2* W, int64_t ld, int64_t N, int n_in, int n_o
 void launch_grad_slice(const double2* Phi, const double2* Et, int64_t N, int64_t n_out, double2 coef, double2* g,
                        cudaStream_t s);
 
+// ---- a structure cut along its length (split_sweep in rgf_api.cu) ----
+constexpr int kSplitMaxParts = 16;
+struct SplitPart {
+  double2* M;            // R x ldm augmented matrix, R = N + no
+  int64_t ldm;
+  const double2* eps;    // its first slice in sweep order
+  const double2 *G0, *g0v;  // lead of its side, and G0 v
+  int inner, ni, no, pc1;
+  const int *prop, *in_idx, *out_idx;  // an end part's channels
+  const double2 *lam, *mu;
+};
+struct SplitInit {
+  int64_t N;
+  const double2* phi;
+  const int* st_col;
+  const double2* st_val;
+  double2 k2;
+  const double2* tab;
+  SplitPart part[kSplitMaxParts];
+};
+void launch_split_tables(const int* st_col, const double2* st_val, int64_t N, const double2* G0L, const double2* G0R,
+                         double2* tab, cudaStream_t s);
+void launch_split_init(const SplitInit& a, int parts, cudaStream_t s);
+void launch_join_inner(const double2* E, int64_t ldE, const double2* I, int64_t ldI, const double2* G0, int64_t N, int ni,
+                       int no, double2* T, double2* F, double2* Q, int64_t ldQ, cudaStream_t s);
+void launch_join_ends(const double2* L, int64_t ldL, const double2* R, int64_t ldR, int64_t N, int niL, int niR, int noL,
+                      int noR, double2* F, double2* Q, int64_t ldQ, cudaStream_t s);
+
 }  // namespace rgf
