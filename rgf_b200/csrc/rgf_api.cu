@@ -97,6 +97,7 @@ struct rgf_handle_s {
   // a structure swept in parts: augmented matrices, exchange buffers, flags,
   // probe tables; per chain of joins (left, right) operands and matrices
   DevBuf sp_m, sp_x, sp_sync, sp_tab, sp_t[2], sp_f[2], sp_q[2][2], sp_p[2], sp_w[2], sp_s[2];
+  DevBuf sp_ck[2], sp_m0, sp_seg, sp_g[2];  // gradient and fields of a split structure
   cudaStream_t aux_stream = nullptr;  // the right chain's joins
   cudaEvent_t aux_ev[2] = {nullptr, nullptr};
   // tuned tile table of the persistent engine: rows Rp <= tile_rmax[i] use
@@ -917,6 +918,296 @@ rgf_status split_sweep(rgf_handle h, const SplitProblem& p, const SplitPlan& pla
   return RGF_OK;
 }
 
+// ---------------------------------------------------------------------------
+// Permittivity gradient and fields of a structure cut in two halves.
+//
+// The backward recursions only need, at every slice, its Green's function
+// connected to one lead and the carriers of that lead, and start from the
+// responses Psi = G B and Phi = C G on the two slices at the cut, a (right) and
+// b (left).  Swept whole, the matrix that joins the halves holds, beside S in
+// its corner, Psi_a in its top rows and Phi_b in its left columns, and
+//     Psi_b = [X_L, 0] + g_L Psi_a,    Phi_a = [0; Z_R] + Phi_b g_R.
+// The left half runs
+//     Psi_k = [X_k, 0] + g_k Psi_{k+1},    Phi_k = [Z_k; 0] + Phi_{k+1} g_k
+// down from (Psi_a, Phi_a) to its lead, the right half its mirror image up from
+// (Psi_b, Phi_b), each with its own side's channels first.  Both forward sweeps,
+// and then the recomputed segments of both halves, as many as fit the GPU, are
+// one launch; the two recursions run on two streams.
+// ---------------------------------------------------------------------------
+struct GradPlan {
+  int tile = 0, group = 1;  // segments of a half recomputed side by side
+  int64_t cut = 0, K = 1;   // checkpoint interval
+};
+
+// extra memory that recomputing several segments side by side may take
+constexpr double kGradSegBytes = 1024.0 * (1 << 20);
+
+bool plan_grad(const rgf_handle h, const SplitProblem& p, int64_t checkpoint, GradPlan* plan) {
+  const int64_t NB = (p.N + 31) / 32;
+  if (p.L < 4 || !gj_step_fits(p.N + p.no[0] + p.no[1])) return false;
+  double best = 0.0, whole = 0.0;
+  plan->cut = p.L / 2;
+  for (int tile : {96, 64, 32}) {
+    const int64_t both = part_ctas(p.N, p.no[0], p.ni[0], tile) + part_ctas(p.N, p.no[1], p.ni[1], tile);
+    const double us = (double)p.L * slice_us(tile, NB);
+    if (std::max(part_ctas(p.N, p.no[0], p.ni[0], tile), part_ctas(p.N, p.no[1], p.ni[1], tile)) <= h->sms &&
+        (whole == 0.0 || us < whole))
+      whole = us;
+    if (both > h->sms) continue;
+    const PartBuf b0 = part_buf(p.N, p.no[0], p.ni[0], tile), b1 = part_buf(p.N, p.no[1], p.ni[1], tile);
+    const double per_slice = sizeof(double2) * 0.5 * (double)(b0.matrix + b1.matrix);
+    // as in the one-sweep form: every slice when those snapshots take at most 2 GiB
+    const int64_t K = checkpoint > 0 ? std::min(checkpoint, p.L)
+                      : (double)p.L * per_slice <= 2.0 * (1 << 30) ? 1
+                                                                   : (int64_t)ceil(sqrt((double)p.L));
+    const int64_t segs = (plan->cut + K - 1) / K;
+    int group = 1;
+    while (K > 1 && group + 1 <= segs && 2 * (group + 1) <= kPersistMaxParts && both * (group + 1) <= h->sms &&
+           (double)(group + 1) * 2.0 * (double)K * per_slice <= kGradSegBytes)
+      group++;
+    double t = 0.5 * us;
+    if (K > 1) t += (double)((segs + group - 1) / group) * (double)K * slice_us(tile, NB);
+    if (plan->tile == 0 || t < best) {
+      best = t;
+      plan->tile = tile;
+      plan->group = group;
+      plan->K = K;
+    }
+  }
+  return plan->tile != 0 && 0.5 * (double)p.L * slice_us(plan->tile, NB) + join_us(NB) < whole;
+}
+
+rgf_status split_grad(rgf_handle h, const SplitProblem& p, const GradPlan& plan, const rgf_cplx* D, int64_t ldD, bool dev,
+                      double2* gout, double2* fout, const int* const col_of[2], const double2** Q_out, int64_t* ldQ_out) {
+  rgf_status st;
+  const int64_t N = p.N, L = p.L, K = plan.K, G = plan.group;
+  const int T = plan.tile, kSwW = sweep_block_width();
+  const int64_t nO = p.no[0] + p.no[1], nI = p.ni[0] + p.ni[1];
+  const PartBuf b[2] = {part_buf(N, p.no[0], p.ni[0], T), part_buf(N, p.no[1], p.ni[1], T)};
+  const int64_t n[2] = {plan.cut, L - plan.cut};
+  // slice k of a half in sweep order
+  auto phys = [&](int c, int64_t k) { return c == 0 ? k : L - 1 - k; };
+  const bool again = K > 1;  // segments are recomputed
+  if ((st = ensure(h, h->sp_m, sizeof(double2) * G * (b[0].matrix + b[1].matrix)))) return st;
+  if ((st = ensure(h, h->sp_x, sizeof(double2) * G * (b[0].exchange + b[1].exchange)))) return st;
+  const int64_t nflag = G * (b[0].flags + b[1].flags), ncons = G * (b[0].cons + b[1].cons);
+  if ((st = ensure(h, h->sp_sync, sizeof(int) * (nflag + ncons)))) return st;
+  if ((st = ensure(h, h->sp_tab, sizeof(double2) * 4 * N))) return st;
+  if ((st = ensure(h, h->sp_f[0], sizeof(double2) * (N + p.no[1]) * (N + p.ni[0])))) return st;
+  if ((st = ensure(h, h->sp_q[0][0], sizeof(double2) * (N + nO) * (N + nI)))) return st;
+  if ((st = ensure(h, h->sp_p[0], sizeof(double2) * (N + nO) * kSwW))) return st;
+  if ((st = ensure(h, h->sp_w[0], sizeof(double2) * (N + nI) * kSwW))) return st;
+  if ((st = ensure(h, h->sp_s[0], gepp_scratch_bytes(N)))) return st;
+  for (int c = 0; c < 2; c++) {
+    if ((st = ensure(h, h->sp_ck[c], sizeof(double2) * b[c].matrix * std::max<int64_t>(1, n[c] / K)))) return st;
+    // Psi, Phi (two each), the contraction's operand, the weights
+    if ((st = ensure(h, h->sp_g[c], sizeof(double2) * (2 * N * nI + 3 * nO * N + nO * nI)))) return st;
+  }
+  if (again) {
+    if ((st = ensure(h, h->sp_m0, sizeof(double2) * (b[0].matrix + b[1].matrix)))) return st;
+    if ((st = ensure(h, h->sp_seg, sizeof(double2) * G * K * (b[0].matrix + b[1].matrix)))) return st;
+  }
+  if ((st = second_stream(h))) return st;
+  const cudaStream_t str[2] = {h->stream, h->aux_stream};
+
+  double2* tab = as<double2>(h->sp_tab);
+  launch_split_tables(p.st_col, p.st_val, N, p.G0[0], p.G0[1], tab, h->stream);
+  // launches `count` parts (half, first slice, slices, matrix, snapshots)
+  struct Run {
+    int c;
+    int64_t lo, n;
+    double2 *M, *snap;
+    int64_t mod;
+  };
+  auto sweep_parts = [&](const std::vector<Run>& runs) -> rgf_status {
+    int* flags = as<int>(h->sp_sync);
+    int* cons = flags + nflag;
+    RGF_CUDA_TRY(cudaMemsetAsync(flags, 0xFF, sizeof(int) * nflag, h->stream));
+    RGF_CUDA_TRY(cudaMemsetAsync(cons, 0, sizeof(int) * ncons, h->stream));
+    double2* x = as<double2>(h->sp_x);
+    std::vector<PersistParams> pp;
+    for (const Run& r : runs) {
+      pp.push_back(part_params(h, p, b[r.c], T, phys(r.c, r.lo), r.c == 0 ? 1 : -1, r.n, r.M, x, flags, cons));
+      pp.back().snap = r.snap;
+      pp.back().snap_mod = (int)r.mod;
+      x += b[r.c].exchange;
+      flags += b[r.c].flags;
+      cons += b[r.c].cons;
+    }
+    const cudaError_t e = launch_persist(pp.data(), (int)pp.size(), T, T, h->stream);
+    if (e != cudaSuccess) {
+      cudaGetLastError();
+      return kRetryUnsplit;
+    }
+    h->launches++;
+    return RGF_OK;
+  };
+  // ---- forward ----
+  double2* M[2] = {as<double2>(h->sp_m), as<double2>(h->sp_m) + b[0].matrix};
+  double2* M0[2] = {as<double2>(h->sp_m0), as<double2>(h->sp_m0) + b[0].matrix};
+  SplitInit init;
+  init.N = N;
+  init.phi = p.phi;
+  init.st_col = p.st_col;
+  init.st_val = p.st_val;
+  init.k2 = p.k2;
+  init.tab = tab;
+  for (int c = 0; c < 2; c++) init.part[c] = init_part(h, p, b[c], c, false, phys(c, 0), M[c]);
+  launch_split_init(init, 2, h->stream);
+  h->launches += 2;
+  if (again)
+    RGF_CUDA_TRY(cudaMemcpyAsync(M0[0], M[0], sizeof(double2) * (b[0].matrix + b[1].matrix), cudaMemcpyDeviceToDevice,
+                                 h->stream));
+  std::vector<Run> runs;
+  for (int c = 0; c < 2; c++) runs.push_back({c, 0, n[c], M[c], as<double2>(h->sp_ck[c]), K});
+  if ((st = sweep_parts(runs))) return st;
+  // ---- join, and the responses on both sides of the cut ----
+  double2* Q = as<double2>(h->sp_q[0][0]);
+  const int64_t ldQ = N + nI;
+  launch_join_ends(M[0], b[0].ldm, M[1], b[1].ldm, N, p.ni[0], p.ni[1], p.no[0], p.no[1], as<double2>(h->sp_f[0]), Q, ldQ,
+                   h->stream);
+  h->launches += 2;
+  if ((st = join_sweep(h, p, Q, N + nO, ldQ, 0, true, h->stream))) return st;
+  double2 *psi[2][2], *phv[2][2], *Et[2], *Dd[2];
+  for (int c = 0; c < 2; c++) {
+    double2* base = as<double2>(h->sp_g[c]);
+    for (int k = 0; k < 2; k++) {
+      psi[c][k] = base + k * N * nI;
+      phv[c][k] = base + 2 * N * nI + k * nO * N;
+    }
+    Et[c] = base + 2 * N * nI + 2 * nO * N;
+    Dd[c] = Et[c] + nO * N;
+  }
+  // left half: Psi_a in S's order; right half: Phi_b with the right side's channels first
+  auto cols = [&](double2* d, int64_t ldd, const double2* q, int64_t ldq, int64_t rows, int64_t w) {
+    launch_block_copy(d, ldd, q, ldq, rows, w, 1.0, h->stream);
+    h->launches++;
+  };
+  cols(psi[0][0], nI, Q + N, ldQ, N, nI);
+  cols(phv[1][0], N, Q + (N + p.no[0]) * ldQ, ldQ, p.no[1], N);
+  cols(phv[1][0] + p.no[1] * N, N, Q + N * ldQ, ldQ, p.no[0], N);
+  // Psi_b = [X_L, 0] + g_L Psi_a, reordered; Phi_a = [Z_R; 0] + Phi_b g_R (right first), reordered
+  launch_zgemm_add(N, nI, N, ZOp{M[0], b[0].ldm, 0}, ZOp{psi[0][0], nI, 0}, ZAdd{M[0] + N, b[0].ldm, N, p.ni[0]},
+                   psi[0][1], nI, h->stream);
+  cols(psi[1][0], nI, psi[0][1] + p.ni[0], nI, N, p.ni[1]);
+  cols(psi[1][0] + p.ni[1], nI, psi[0][1], nI, N, p.ni[0]);
+  launch_zgemm_add(nO, N, N, ZOp{phv[1][0], N, 0}, ZOp{M[1], b[1].ldm, 0},
+                   ZAdd{M[1] + N * b[1].ldm, b[1].ldm, p.no[1], N}, phv[1][1], N, h->stream);
+  cols(phv[0][0] + p.no[0] * N, N, phv[1][1], N, p.no[1], N);
+  cols(phv[0][0], N, phv[1][1] + p.no[1] * N, N, p.no[0], N);
+  h->launches += 2;
+  // the weights in each half's order
+  std::vector<rgf_cplx> Du((size_t)nO * nI), Da[2];
+  if (gout) {
+    if (dev) {
+      RGF_CUDA_TRY(cudaMemcpy2DAsync(Du.data(), sizeof(rgf_cplx) * nO, D, sizeof(rgf_cplx) * ldD, sizeof(rgf_cplx) * nO,
+                                     nI, cudaMemcpyDeviceToHost, h->stream));
+      RGF_CUDA_TRY(cudaStreamSynchronize(h->stream));
+    } else {
+      for (int64_t i = 0; i < nI; i++)
+        for (int64_t o = 0; o < nO; o++) Du[o + i * nO] = D[o + i * ldD];
+    }
+    for (int c = 0; c < 2; c++) {
+      Da[c].resize((size_t)nO * nI);
+      for (int64_t i = 0; i < nI; i++)
+        for (int64_t o = 0; o < nO; o++) {
+          const int64_t r = c == 0 ? o : o < p.no[0] ? p.no[1] + o : o - p.no[0];
+          const int64_t q = c == 0 ? i : i < p.ni[0] ? p.ni[1] + i : i - p.ni[0];
+          Da[c][(size_t)(r * nI + q)] = Du[o + i * nO];
+        }
+      RGF_CUDA_TRY(cudaMemcpyAsync(Dd[c], Da[c].data(), sizeof(double2) * nO * nI, cudaMemcpyHostToDevice, h->stream));
+    }
+  }
+  // ---- backward: groups of segments of both halves, the last ones first ----
+  const double2 coef = cmul(cmk(0.0, -2.0), p.k2);
+  const double2 one = cmk(1.0, 0.0), zero = cmk(0.0, 0.0);
+  int cur[2] = {0, 0};
+  auto back = [&](int c, int64_t k, const double2* W) {
+    const int64_t ld = b[c].ldm, at = phys(c, k);
+    const int nx = cur[c] ^ 1;
+    const cudaStream_t s = str[c];
+    if (grad_step_fits((int)nI, (int)nO)) {
+      launch_grad_step(W, ld, N, (int)nI, (int)nO, p.ni[c], p.no[c], psi[c][cur[c]], phv[c][cur[c]], Dd[c], coef,
+                       psi[c][nx], phv[c][nx], gout ? gout + at * N : nullptr, s);
+      h->launches++;
+    } else {
+      launch_zgemm_add(N, nI, N, ZOp{W, ld, 0}, ZOp{psi[c][cur[c]], nI, 0}, ZAdd{W + N, ld, N, p.ni[c]}, psi[c][nx], nI, s);
+      h->launches++;
+      if (gout) {
+        launch_zgemm_add(nO, N, N, ZOp{phv[c][cur[c]], N, 0}, ZOp{W, ld, 0}, ZAdd{W + N * ld, ld, p.no[c], N}, phv[c][nx],
+                         N, s);
+        if (nO * nI <= 1024) {
+          launch_grad_fused(phv[c][nx], psi[c][nx], Dd[c], N, (int)nO, (int)nI, coef, gout + at * N, s);
+          h->launches += 2;
+        } else {
+          launch_zgemm(nO, N, nI, one, ZOp{Dd[c], nI, 0}, ZOp{psi[c][nx], nI, 1}, zero, Et[c], N, s);
+          launch_grad_slice(phv[c][nx], Et[c], N, nO, coef, gout + at * N, s);
+          h->launches += 3;
+        }
+      }
+    }
+    if (fout) {
+      launch_store_field(psi[c][nx], col_of[c], N, (int)nI, fout + at * N, N * L, s);
+      h->launches++;
+    }
+    cur[c] = nx;
+  };
+  auto fork = [&]() -> rgf_status {
+    RGF_CUDA_TRY(cudaEventRecord(h->aux_ev[0], h->stream));
+    RGF_CUDA_TRY(cudaStreamWaitEvent(h->aux_stream, h->aux_ev[0], 0));
+    return RGF_OK;
+  };
+  auto join = [&]() -> rgf_status {
+    RGF_CUDA_TRY(cudaEventRecord(h->aux_ev[1], h->aux_stream));
+    RGF_CUDA_TRY(cudaStreamWaitEvent(h->stream, h->aux_ev[1], 0));
+    return RGF_OK;
+  };
+  if (!again) {
+    if ((st = fork())) return st;
+    for (int64_t k = std::max(n[0], n[1]) - 1; k >= 0; k--)
+      for (int c = 0; c < 2; c++)
+        if (k < n[c]) back(c, k, as<double2>(h->sp_ck[c]) + k * b[c].matrix);
+    if ((st = check_launch())) return st;
+    if ((st = join())) return st;
+  } else {
+    int64_t left[2] = {(n[0] + K - 1) / K, (n[1] + K - 1) / K};  // segments not yet done
+    while (left[0] > 0 || left[1] > 0) {
+      runs.clear();
+      double2* m = as<double2>(h->sp_m);
+      double2* seg = as<double2>(h->sp_seg);
+      for (int c = 0; c < 2; c++)
+        for (int64_t g = 0; g < G && left[c] > 0; g++) {
+          const int64_t sg = --left[c], lo = sg * K, hi = std::min(n[c], lo + K);
+          const size_t bytes = sizeof(double2) * b[c].matrix;
+          if (sg == 0) {
+            RGF_CUDA_TRY(cudaMemcpyAsync(m, M0[c], bytes, cudaMemcpyDeviceToDevice, h->stream));
+          } else {
+            RGF_CUDA_TRY(cudaMemcpyAsync(m, as<double2>(h->sp_ck[c]) + (sg - 1) * b[c].matrix, bytes,
+                                         cudaMemcpyDeviceToDevice, h->stream));
+            launch_assemble(m, b[c].ldm, N, b[c].R, m, b[c].ldm, nullptr, 0, p.st_col, p.st_val, p.k2,
+                            p.eps + phys(c, lo) * N, zero, h->stream);
+            launch_probe_init(m, b[c].ldm, N, b[c].R, b[c].pc1, h->stream);
+            h->launches += 2;
+          }
+          runs.push_back({c, lo, hi - lo, m, seg, 1});
+          m += b[c].matrix;
+          seg += K * b[c].matrix;
+        }
+      if ((st = sweep_parts(runs))) return st;
+      if ((st = fork())) return st;
+      for (int c = 0; c < 2; c++)
+        for (const Run& r : runs)
+          if (r.c == c)
+            for (int64_t k = r.n - 1; k >= 0; k--) back(c, r.lo + k, r.snap + k * b[c].matrix);
+      if ((st = check_launch())) return st;
+      if ((st = join())) return st;
+    }
+  }
+  *Q_out = Q;
+  *ldQ_out = ldQ;
+  return RGF_OK;
+}
+
 rgf_status smatrix_run(rgf_handle h, const Problem& p, const rgf_request* req, const rgf_options* opt, rgf_cplx* S,
                        int64_t ldS, rgf_channels* ch, const GradReq* gr, int engine, const SegReq* seg,
                        bool may_split) {
@@ -1045,6 +1336,9 @@ rgf_status smatrix_run(rgf_handle h, const Problem& p, const rgf_request* req, c
   std::vector<int> ident(h->arena ? 0 : std::max(n_out, n_in));  // rows and columns in S's own order (split sweep)
   for (size_t q = 0; q < ident.size(); q++) ident[q] = (int)q;
   const size_t o_ident = push(ident);
+  std::vector<int> right_first(h->arena ? 0 : n_in);  // columns of S with the right side's channels first
+  for (size_t q = 0; q < right_first.size(); q++) right_first[q] = (int)q < niL ? niR + (int)q : (int)q - niL;
+  const size_t o_right = push(right_first);
   if ((st = ensure(h, h->idx, sizeof(int) * (idx.size() + 1)))) return st;
   int* idx_d = as<int>(h->idx);
   RGF_CUDA_TRY(cudaMemcpyAsync(idx_d, idx.data(), sizeof(int) * idx.size(), cudaMemcpyHostToDevice, h->stream));
@@ -1156,7 +1450,7 @@ rgf_status smatrix_run(rgf_handle h, const Problem& p, const rgf_request* req, c
   const double2* st_val = as<double2>(h->st_val);
 
   // (5c) parts swept side by side where that is faster
-  if (may_split && engine == 0 && L > 0 && !gr && !seg && !h->arena && !h->sm_budget && !(opt && opt->profile > 0)) {
+  if (may_split && engine == 0 && L > 0 && !seg && !h->arena && !h->sm_budget && !(opt && opt->profile > 0)) {
     SplitProblem sp;
     SplitPlan plan;
     sp.N = N;
@@ -1177,13 +1471,25 @@ rgf_status smatrix_run(rgf_handle h, const Problem& p, const rgf_request* req, c
     sp.eps = eps_d;
     sp.k2 = k2;
     sp.status = status;
-    if (plan_split(h, sp, &plan)) {
+    GradPlan gplan;
+    if (gr ? plan_grad(h, sp, gr->checkpoint, &gplan) : plan_split(h, sp, &plan)) {
       if ((st = ensure(h, h->xprobe, sizeof(unsigned long long)))) return st;
       sp.probe = as<unsigned long long>(h->xprobe);
       RGF_CUDA_TRY(cudaMemsetAsync(sp.probe, 0, sizeof(unsigned long long), h->stream));
       const double2* Q = nullptr;
       int64_t ldQ = 0;
-      if ((st = split_sweep(h, sp, plan, &Q, &ldQ))) return st;
+      const bool g_host = gr && gr->D && !S_dev, f_host = gr && gr->psi && !S_dev;
+      if (gr) {
+        if (g_host && (st = ensure(h, h->gg, sizeof(double2) * N * L))) return st;
+        if (f_host && (st = ensure(h, h->gf, sizeof(double2) * N * L * n_in))) return st;
+        double2* gout = !gr->D ? nullptr : S_dev ? reinterpret_cast<double2*>(gr->g) : as<double2>(h->gg);
+        double2* fout = !gr->psi ? nullptr : S_dev ? reinterpret_cast<double2*>(gr->psi) : as<double2>(h->gf);
+        const int* const col_of[2] = {idx_d + o_ident, idx_d + o_right};
+        st = split_grad(h, sp, gplan, gr->D, gr->ldD, S_dev, gout, fout, col_of, &Q, &ldQ);
+      } else {
+        st = split_sweep(h, sp, plan, &Q, &ldQ);
+      }
+      if (st) return st;
       double2* Sd = S_dev ? reinterpret_cast<double2*>(S) : as<double2>(h->sdev);
       launch_extract(Q, ldQ, N, idx_d + o_ident, n_out, idx_d + o_ident, n_in, Sd, S_dev ? ldS : n_out, idx_d + o_pairs,
                      npairs, h->stream);
@@ -1192,6 +1498,10 @@ rgf_status smatrix_run(rgf_handle h, const Problem& p, const rgf_request* req, c
       if (!S_dev)
         RGF_CUDA_TRY(cudaMemcpy2DAsync(S, sizeof(rgf_cplx) * ldS, Sd, sizeof(double2) * n_out,
                                        sizeof(double2) * n_out, n_in, cudaMemcpyDeviceToHost, h->stream));
+      if (g_host)
+        RGF_CUDA_TRY(cudaMemcpyAsync(gr->g, h->gg.p, sizeof(double2) * N * L, cudaMemcpyDeviceToHost, h->stream));
+      if (f_host)
+        RGF_CUDA_TRY(cudaMemcpyAsync(gr->psi, h->gf.p, sizeof(double2) * N * L * n_in, cudaMemcpyDeviceToHost, h->stream));
       int hstatus = 0;
       unsigned long long bits = 0;
       RGF_CUDA_TRY(cudaMemcpyAsync(&hstatus, status, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
@@ -1924,7 +2234,8 @@ rgf_status rgf_destroy(rgf_handle h) {
     if (b.p) cudaFree(b.p);
   for (DevBuf* b : {&h->sp_m, &h->sp_x, &h->sp_sync, &h->sp_tab, &h->sp_t[0], &h->sp_t[1], &h->sp_f[0], &h->sp_f[1],
                     &h->sp_q[0][0], &h->sp_q[0][1], &h->sp_q[1][0], &h->sp_q[1][1], &h->sp_p[0], &h->sp_p[1],
-                    &h->sp_w[0], &h->sp_w[1], &h->sp_s[0], &h->sp_s[1]})
+                    &h->sp_w[0], &h->sp_w[1], &h->sp_s[0], &h->sp_s[1], &h->sp_ck[0], &h->sp_ck[1], &h->sp_m0,
+                    &h->sp_seg, &h->sp_g[0], &h->sp_g[1]})
     if (b->p) cudaFree(b->p);
   for (cudaEvent_t ev : h->aux_ev)
     if (ev) cudaEventDestroy(ev);

@@ -111,3 +111,62 @@ def test_nonfinite_permittivity_is_refused():
     s["epsilon"][5, 50] = np.nan
     with pytest.raises(Exception, match="NaN or Inf"):
         rgf_b200.cal_smatrix_RGF(s, FULL, FULL)
+
+
+@pytest.mark.parametrize("checkpoint", [0, 1, 2, 7, 100])
+@pytest.mark.parametrize("ny,nx", [(1, 4), (20, 5), (33, 31), (70, 12), (130, 9)])
+def test_gradient_of_two_halves(ny, nx, checkpoint):
+    """Odd cuts, short last segments, several segments side by side, and (at
+    ny = 130, full S) the separate contraction for many channels; 1e-10 on the
+    gradient, as for the one-sweep form."""
+    from oracle.adjoint import grad_rgf_2d
+    form = ("full", "transmission", "back", "from_left", "full")[[1, 20, 33, 70, 130].index(ny)]
+    out, in_ = REQUESTS[form]
+    s = structure(ny, nx, "periodic" if ny != 33 else "Neumann", eps_R=1.0 if ny == 130 else 2.0, lossy=nx == 31)
+    rng = np.random.default_rng(ny)
+    shape = cal_smatrix_RGF(s, out, in_)[0].shape
+    D = rng.standard_normal(shape) + 1j * rng.standard_normal(shape)
+    S0, g0 = grad_rgf_2d(s, out, in_, D)
+    S, g = rgf_b200.smatrix_grad_RGF(s, out, in_, D, checkpoint=checkpoint)
+    assert rel(S, S0) <= TOL_S
+    assert np.abs(g - g0).max() <= 1e-10 * np.abs(g0).max()
+
+
+@pytest.mark.parametrize("form", sorted(REQUESTS))
+@pytest.mark.parametrize("ny,nx", [(20, 4), (34, 11)])
+def test_fields_of_two_halves(ny, nx, form):
+    from oracle.dense_fdfd import fields_dense_2d
+    out, in_ = REQUESTS[form]
+    s = structure(ny, nx, 0.4, eps_R=1.7)
+    _, psi0 = fields_dense_2d(s, out, in_)
+    for checkpoint in (0, 3):
+        S, psi = rgf_b200.fields_RGF(s, out, in_, checkpoint=checkpoint)
+        assert np.linalg.norm(psi - psi0) <= TOL_S * np.linalg.norm(psi0)
+
+
+def test_gradient_on_the_device_in_two_halves():
+    """S, weights, gradient and fields as device buffers, one handle for calls of changing size."""
+    import ctypes
+
+    import torch
+    from rgf_b200.api import _request
+    h = _abi.Handle(0)
+    for ny, nx in ((48, 21), (16, 40), (90, 8)):
+        s = structure(ny, nx)
+        req, keep = _request(FULL, FULL)
+        S0, _ = cal_smatrix_RGF(s, FULL, FULL)
+        n = S0.shape[0]
+        eps = torch.from_numpy(np.ascontiguousarray(np.asarray(s["epsilon"], complex).ravel(order="F"))).cuda()
+        sy = _abi.Syst2D(ny, nx, eps.data_ptr(), 1, _abi.cplx(1.0), _abi.cplx(1.0), _abi.cplx(s["k0dx"]),
+                         _abi.BC_PERIODIC, 0.0)
+        D = torch.from_numpy(np.ascontiguousarray(np.conj(S0).T)).cuda()
+        S = torch.zeros((n, n), dtype=torch.complex128, device="cuda")
+        g = torch.zeros((nx, ny), dtype=torch.complex128, device="cuda")
+        opt = _abi.Options(_abi.RGF_FP64, 0, 1, 0)
+        torch.cuda.synchronize()
+        _abi.check(h.lib.rgf_smatrix_grad_2d(h.h, ctypes.byref(sy), ctypes.byref(req), ctypes.byref(opt), D.data_ptr(), n,
+                                             S.data_ptr(), n, g.data_ptr(), 4))
+        host = rgf_b200.smatrix_grad_RGF(s, FULL, FULL, np.conj(S0), checkpoint=4)
+        assert rel(S.cpu().numpy().T, S0) <= TOL_S
+        assert rel(g.cpu().numpy().T, host[1]) <= 1e-12
+        del keep
