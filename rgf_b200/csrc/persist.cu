@@ -29,10 +29,10 @@
 //    a3 = W^{(x-2)}(J_{x-1},J_x) (from the panels' pivot rows) in shared
 //    memory; its 8 math warps form the next pivot block by the Schur update
 //        W^{(s-1)}(J_s,J_s) = y0 - y1 (T_{s-1} a3)
-//    and invert it by register-resident Gauss-Jordan with partial pivoting
-//    (owner warps run ahead with per-row release counters, redux.sync pivot
-//    search, implicit row interchanges, rows scaled once at the end); the
-//    first pivot block of every slice comes straight from the slice assembly.
+//    and invert it by Gauss-Jordan with partial pivoting in panels of four
+//    columns (one warp, redux.sync pivot search, implicit row interchanges) and
+//    rank-4 updates on the FP64 tensor cores; the first pivot block of every
+//    slice comes straight from the slice assembly.
 // setmaxnreg moves registers from the panel warpgroup (88) to the math
 // warpgroups (208) so the 96x96 complex tile (144 registers/thread) fits.
 // Exchange buffers are double-buffered by step parity; each has a publication
@@ -71,10 +71,13 @@ struct Cfg {
 
 // Named barriers in their non-.aligned form (per-thread arrival), preceded
 // by a warp reconvergence, so that no barrier depends on the compiler having
-// reconverged a warp after lane-divergent code.
+// reconverged a warp after lane-divergent code; and followed by one, so that a
+// lane that polled a flag before the barrier does not run what follows apart
+// from its warp.
 __device__ __forceinline__ void bar_sync(int id, int n) {
   __syncwarp();
   asm volatile("barrier.sync %0, %1;" ::"r"(id), "r"(n) : "memory");
+  __syncwarp();
 }
 // CTA-uniform OR over the threads of a named barrier
 __device__ __forceinline__ int bar_or(int id, int n, int pred) {
@@ -85,6 +88,7 @@ __device__ __forceinline__ int bar_or(int id, int n, int pred) {
       : "=r"(r)
       : "r"(id), "r"(n), "r"(pred)
       : "memory");
+  __syncwarp();
   return r;
 }
 __device__ __forceinline__ int ld_acquire(const int* p) {
@@ -145,17 +149,12 @@ struct Shared {
   int panel_abort;
   Blk T;   // panel role: T_s
   Blk Mr;  // panel role: my columns of the pivot rows
-  // T-server Gauss-Jordan: pivot q's multipliers are in srv.v[q][r]; per row r
-  // its pivot index copy, release counter, and the reciprocal of the pivot
-  // it became
-  int gpiv[kPB][kPB];
-  int gflag[kPB];
-  double2 drow[kPB];
-  int gj_fail;  // a Gauss-Jordan wait gave up
+  // T-server Gauss-Jordan: the swept four columns of a panel, the row chosen at every pivot
+  double2 gpan[kPB][5];
+  alignas(16) int gpv[kPB];
   int asig[2];  // T-server: step whose a3[parity] block is staged (prep -> server)
   int ysig[2];  // T-server: step whose y[parity] blocks are ready (prep -> server)
   int ycons;    // T-server: last step whose y blocks the server has read
-  int perm[kPB], pinv[kPB];
 };
 
 __device__ __forceinline__ void trace_ev(const PersistParams& p, int s, int ev) {
@@ -911,103 +910,116 @@ __device__ void panel_role(const PersistParams& p, Shared& sh, const Sync& sy, i
 // ---------------------------------------------------------------------------
 // T-server CTA
 // ---------------------------------------------------------------------------
-// Gauss-Jordan inversion of the 32x32 pivot block with partial pivoting,
-// register resident: lane r of warp w holds row r, columns [4w, 4w+4).  The
-// block is padded with the identity beyond its jn valid rows and columns, so
-// all 32 pivots run (a padding column is a unit vector whose pivot is its
-// own padding row; the result is the inverse padded with the identity).
+// Gauss-Jordan inversion of the 32x32 pivot block with partial pivoting by the
+// 8 server warps, in eight panels of four columns.  The block is padded with
+// the identity beyond its jn valid rows and columns, so all 32 pivots run (a
+// padding column is a unit vector whose pivot is its own padding row; the result
+// is the inverse padded with the identity).
 //
-// Rows are kept unscaled: after pivot q (row pv, reciprocal d of the pivot
-// value, multipliers m(r) = a(r,q) d for r != pv, m(pv) = 0) every column c
-// of every warp takes the one complex FMA  a(r,c) -= m(r) a(pv,c), the pivot
-// column becomes (-m, with 1 in row pv), and row r is multiplied by the d of
-// the pivot it became only at the end.
+// Warp 0 sweeps a panel in registers (lane = row): for each of its pivots one
+// redux.sync over the high words of max(|re|, |im|) packed with the lane index,
+// the reciprocal formed speculatively by every lane meanwhile, and one complex
+// FMA per element.  The panel P it leaves, [-W(i,J) T (i not chosen); T], turns
+// the other 28 columns into  W_mod + P W(J, :)  (J the rows chosen, W_mod W with
+// those rows read as zero), one m8n8k4 k-step on every warp's 16 x 8 piece,
+// which stays in its accumulators; the panel's own columns take unit columns for
+// W(J, :).  The matrix before and after a panel alternate between two blocks
+// of shared memory, read by the next panel and for the rows J.
 //
-// Warp w chooses the pivots of its own four columns and runs ahead: for each
-// one it publishes m(r), pv (and d in lane pv) with a release store of its
-// own row's counter, lane by lane, and goes on at once; every warp applies
-// the pivots in order, each lane waiting (bounded) on its own row's counter,
-// so the chain from one pivot to the next crosses warps only at the
-// four-column block boundaries.  Pivot search: one redux.sync over
-// single-precision magnitudes packed with the lane index, the reciprocal
-// formed speculatively by every lane meanwhile.  Row interchanges are
-// implicit:  inv[pinv[r]][perm[c]] = a(r, c),  perm[q] = row chosen at q.
-// Returns false in every lane if a wait gave up (abort or timeout).
-__device__ __forceinline__ bool gj_ahead(const PersistParams& p, Shared& sh, double2 (&a)[4], int t) {
-  constexpr int NC = 4;
+// The chain of 32 pivots bounds it, at 220 cycles a pivot (the shuffles of a
+// pivot take 6 cycles each to issue) and 600 for the rank-4 update of a panel:
+// 7.8 us, against 9.7 us for eight warps of four columns that pass every pivot
+// on through flags in shared memory (a flag takes 220 cycles from warp to warp,
+// a barrier 30).  The pivot loop stays rolled: unrolled, a panel is 10% faster,
+// but the first one of a slice, whose code has gone cold, takes 8 us more.  A
+// slice of N = 256 (32 x 32 tiles) went from 128 to 108 us, of N = 512 (64 x 64)
+// from 254 to 218 us.  Row interchanges are implicit: the inverse is
+//     T[q][pv[c]] = W(pv[q], c),   pv[q] = row chosen at pivot q.
+// The block is in A on entry, its inverse there at the end; B is scratch.
+__device__ __forceinline__ double2 shfl_c(double2 v, int src) {
+  return cmk(__shfl_sync(kFull, v.x, src), __shfl_sync(kFull, v.y, src));
+}
+
+__device__ __forceinline__ void gj_block(const PersistParams& p, Shared& sh, int s, Blk* A, Blk* B, int t) {
   const int lane = t & 31, warp = t >> 5;
+  const int r0 = 16 * (warp & 1) + (lane >> 2), cb = 8 * (warp >> 1), lc = (lane & 3) * 2;
   unsigned used = 0;
-  bool sing = false, ok = true;
-  for (int b = 0; b < kPB / NC; b++) {
-    if (warp == b) {
+  bool sing = false;
+  const Blk* W = A;
+  double acc[2][4];
 #pragma unroll
-      for (int cq = 0; cq < NC; cq++) {
-        const int q = b * NC + cq;
-        const double2 vq = a[cq];
-        const double2 dq = crecip_nr(vq);  // speculative: used only if this lane wins
-        const float fx = (float)vq.x, fy = (float)vq.y;
-        const float mag = fx * fx + fy * fy;
-        const bool elig = !((used >> lane) & 1u);
-        const unsigned key = elig ? ((__float_as_uint(mag) & ~63u) | (unsigned)(32 - lane)) : 0u;
+  for (int rt = 0; rt < 2; rt++)
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      const double2 v = (*W)[r0 + 8 * rt][cb + lc + h];
+      acc[rt][h] = v.x;
+      acc[rt][2 + h] = v.y;
+    }
+  Blk* out = B;
+#pragma unroll 1
+  for (int b = 0; b < kPB / 4; b++) {
+    if (warp == 0) {
+      double2 a[4];
+#pragma unroll
+      for (int k = 0; k < 4; k++) a[k] = (*W)[lane][4 * b + k];
+#pragma unroll 1
+      for (int k = 0; k < 4; k++) {  // the pivot's column in a[0]: a pivot rotates the registers by one
+        const double2 dq = crecip_nr(a[0]);  // speculative: used only if this lane wins
+        const unsigned mag = max((unsigned)__double2hiint(a[0].x) & 0x7fffffffu,
+                                 (unsigned)__double2hiint(a[0].y) & 0x7fffffffu);
+        const unsigned key = ((used >> lane) & 1u) ? 0u : ((mag & ~63u) | (unsigned)(32 - lane));
         const unsigned best = __reduce_max_sync(kFull, key);
         const int pv = 32 - (int)(best & 63u);
-        const double2 d = cmk(__shfl_sync(kFull, dq.x, pv), __shfl_sync(kFull, dq.y, pv));
+        const double2 p1 = shfl_c(a[1], pv);  // the next pivot's column first
+        const double2 d = shfl_c(dq, pv);
+        const double2 p2 = shfl_c(a[2], pv), p3 = shfl_c(a[3], pv);
         const bool me = lane == pv;
-        const double2 m = me ? cmk(0.0, 0.0) : cmul(vq, d);
-        sh.srv.v[q][lane] = m;
-        sh.gpiv[q][lane] = pv;
-        if (me) {
-          sh.drow[lane] = d;
-          sh.pinv[lane] = q;
-        }
-        if (lane == 0) sh.perm[q] = pv;
-        st_release_cta(&sh.gflag[lane], q + 1);
-        // a zero reciprocal of a nonzero pivot (|z|^2 beyond the range of
-        // rcp.approx.ftz) is as unusable as a non-finite one
-        sing = sing || (best >> 6) == 0u || !isfinite(d.x) || !isfinite(d.y) || (d.x == 0.0 && d.y == 0.0);
+        const double2 m = me ? cneg(d) : cmul(a[0], d);
         used |= 1u << pv;
-#pragma unroll
-        for (int c = 0; c < NC; c++) {
-          if (c == cq) {
-            a[c] = me ? cmk(1.0, 0.0) : cneg(m);
-          } else {
-            const double2 pr = cmk(__shfl_sync(kFull, a[c].x, pv), __shfl_sync(kFull, a[c].y, pv));
-            a[c] = cmk(fma(-m.x, pr.x, fma(m.y, pr.y, a[c].x)), fma(-m.x, pr.y, fma(-m.y, pr.x, a[c].y)));
-          }
-        }
+        if (lane == 0) sh.gpv[4 * b + k] = pv;
+        sing = sing || (best >> 6) == 0u || !isfinite(d.x) || !isfinite(d.y);
+        auto swept = [&](double2 x, double2 pr) {
+          const double2 o = me ? cmk(0.0, 0.0) : x;
+          return cmk(fma(-m.x, pr.x, fma(m.y, pr.y, o.x)), fma(-m.x, pr.y, fma(-m.y, pr.x, o.y)));
+        };
+        a[0] = swept(a[1], p1);
+        a[1] = swept(a[2], p2);
+        a[2] = swept(a[3], p3);
+        a[3] = cneg(m);
       }
-    } else {
 #pragma unroll
-      for (int cq = 0; cq < NC; cq++) {
-        const int q = b * NC + cq;
-        if (ld_acquire_cta(&sh.gflag[lane]) <= q) {
-          const long long t0 = clock64();
-          for (int spins = 1;; spins++) {
-            if (ld_acquire_cta(&sh.gflag[lane]) > q) break;
-            if ((spins & 63) == 0 && give_up(p, t0)) {
-              ok = false;
-              break;
-            }
-          }
-        }
-        const double2 m = sh.srv.v[q][lane];
-        const int pv = sh.gpiv[q][lane] & 31;
-        used |= 1u << pv;
-#pragma unroll
-        for (int c = 0; c < NC; c++) {
-          const double2 pr = cmk(__shfl_sync(kFull, a[c].x, pv), __shfl_sync(kFull, a[c].y, pv));
-          a[c] = cmk(fma(-m.x, pr.x, fma(m.y, pr.y, a[c].x)), fma(-m.x, pr.y, fma(-m.y, pr.x, a[c].y)));
-        }
-      }
+      for (int k = 0; k < 4; k++) sh.gpan[lane][k] = a[k];
     }
-  }
-  // every lane has acquired its own row's counter for all 32 pivots, so the
-  // reciprocal of the pivot its row became is visible to it
-  const double2 dr = sh.drow[lane];
+    bar_sync(kBarMath, kServerThreads);
+    const int k = lane & 3, cB = cb + (lane >> 2);
+    const int4 p4 = *reinterpret_cast<const int4*>(&sh.gpv[4 * b]);
+    const int pvk = k == 0 ? p4.x : k == 1 ? p4.y : k == 2 ? p4.z : p4.w;
+    const double2 A0 = sh.gpan[r0][k], A1 = sh.gpan[r0 + 8][k];
+    double2 bv = (*W)[pvk][cB];
+    if ((cB >> 2) == b) bv = cmk((cB & 3) == k ? 1.0 : 0.0, 0.0);
+    const unsigned chosen = (1u << p4.x) | (1u << p4.y) | (1u << p4.z) | (1u << p4.w);
+    const bool own = ((cb + lc) >> 2) == b;  // this thread's two columns lie in the panel
 #pragma unroll
-  for (int c = 0; c < NC; c++) a[c] = cmul(a[c], dr);
-  if (sing && lane == 0) atomicOr(p.status, kStatusSingular);
-  return __all_sync(kFull, ok);
+    for (int rt = 0; rt < 2; rt++)
+      if (own || ((chosen >> (r0 + 8 * rt)) & 1u)) acc[rt][0] = acc[rt][1] = acc[rt][2] = acc[rt][3] = 0.0;
+    dmma(acc[0][0], acc[0][1], A0.x, bv.x);
+    dmma(acc[0][2], acc[0][3], A0.x, bv.y);
+    dmma(acc[1][0], acc[1][1], A1.x, bv.x);
+    dmma(acc[1][2], acc[1][3], A1.x, bv.y);
+    dmma(acc[0][0], acc[0][1], -A0.y, bv.y);
+    dmma(acc[0][2], acc[0][3], A0.y, bv.x);
+    dmma(acc[1][0], acc[1][1], -A1.y, bv.y);
+    dmma(acc[1][2], acc[1][3], A1.y, bv.x);
+#pragma unroll
+    for (int rt = 0; rt < 2; rt++)
+#pragma unroll
+      for (int h = 0; h < 2; h++) (*out)[r0 + 8 * rt][cb + lc + h] = cmk(acc[rt][h], acc[rt][2 + h]);
+    bar_sync(kBarMath, kServerThreads);
+    if (t == 0) trace_ev(p, s, kTrSrvGroup0 + b);
+    W = out;
+    out = out == B ? A : B;
+  }
+  if (sing && t == 0) atomicOr(p.status, kStatusSingular);
 }
 
 // Cout = Cin + alpha * A B for padded 32x32 complex blocks in shared memory
@@ -1081,34 +1093,32 @@ __device__ void server_role(const PersistParams& p, Shared& sh, const Sync& sy, 
       bad = !wait_cta_ge(p, &sh.ysig[par], s);
       trace_ev(p, s, kTrPanelTin);
     }
-    if (t < kPB) sh.gflag[t] = 0;
-    if (t == 0) sh.gj_fail = 0;
     if (bar_or(kBarMath, kServerThreads, bad)) return;
     if (t == 0) trace_ev(p, s, kTrSrvLoaded);
     if (k != 0) {  // W^{(s-1)}(J_s,J_s) = y0 - y1 V
       blk_gemm(sh.srv.y[par][1], sh.srv.v, &sh.srv.y[par][0], -1.0, sh.srv.a1, t);
-      bar_sync(kBarMath, kServerThreads);
-    }
-    if (t == 0) trace_ev(p, s, kTrSrvSchur);
-    double2 a[4];
-    const Blk& a0 = (k != 0) ? sh.srv.a1 : sh.srv.y[par][0];
+    } else {
 #pragma unroll
-    for (int c = 0; c < 4; c++) a[c] = a0[lane][warp * 4 + c];
-    if (!gj_ahead(p, sh, a, t)) sh.gj_fail = 1;
+      for (int q = 0; q < 4; q++) sh.srv.a1[warp * 4 + q][lane] = sh.srv.y[par][0][warp * 4 + q][lane];
+    }
+    bar_sync(kBarMath, kServerThreads);
+    if (t == 0) trace_ev(p, s, kTrSrvSchur);
+    gj_block(p, sh, s, &sh.srv.a1, &sh.srv.v, t);
     if (t == 0) {
       trace_ev(p, s, kTrSrvGJ);
       sh.panel_abort = tcons_ok ? 0 : !wait_ge(p, sy.t_cons + par, ntiles * (s >> 1));
-      st_release_cta(&sh.ycons, s);  // y[par] was read before the Gauss-Jordan started
+      st_release_cta(&sh.ycons, s);  // y[par] was read before the Gauss-Jordan ended
     }
     bar_sync(kBarMath, kServerThreads);
-    if (sh.panel_abort || sh.gj_fail) return;
+    if (sh.panel_abort) return;
     double2* tb = p.tbuf + (size_t)par * kPB * kPB;
-    const int rr = sh.pinv[lane];
+    const int cc = sh.gpv[lane];
 #pragma unroll
-    for (int c = 0; c < 4; c++) {
-      const int cc = sh.perm[warp * 4 + c];
-      __stcg(tb + rr * kPB + cc, a[c]);
-      sh.srv.tprev[rr][cc] = a[c];
+    for (int q = 0; q < 4; q++) {
+      const int r = warp * 4 + q;
+      const double2 v = sh.srv.a1[sh.gpv[r]][lane];
+      __stcg(tb + r * kPB + cc, v);
+      sh.srv.tprev[r][cc] = v;
     }
     bar_sync(kBarMath, kServerThreads);
     if (t == 0) {
@@ -1276,14 +1286,26 @@ struct PersistSet {
   PersistParams p[kPersistMaxParts];
 };
 
-template <int BM, int BN>
-__global__ void __launch_bounds__(Cfg<BM, BN>::Threads, 1) k_persist(const __grid_constant__ PersistSet set) {
-  extern __shared__ __align__(128) unsigned char smem_raw[];
-  Shared& sh = *reinterpret_cast<Shared*>(smem_raw);
+// the part of this CTA and its place there.  One sweep takes its parameters as
+// they are: indexed, they cost the 96 x 96 tiles 26 us of a 553 us slice
+// (N = 1000; every use a load instead of a constant operand, and spills).
+__device__ __forceinline__ const PersistParams& part_of(const PersistParams& one, int& local) {
+  local = (int)blockIdx.x;
+  return one;
+}
+__device__ __forceinline__ const PersistParams& part_of(const PersistSet& set, int& local) {
   int part = 0;
   while (part + 1 < set.count && (int)blockIdx.x >= set.first[part + 1]) part++;
-  const PersistParams& p = set.p[part];
-  const int local = (int)blockIdx.x - set.first[part];
+  local = (int)blockIdx.x - set.first[part];
+  return set.p[part];
+}
+
+template <int BM, int BN, class Params>
+__global__ void __launch_bounds__(Cfg<BM, BN>::Threads, 1) k_persist(const __grid_constant__ Params params) {
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  Shared& sh = *reinterpret_cast<Shared*>(smem_raw);
+  int local;
+  const PersistParams& p = part_of(params, local);
   const int I = local / p.TC, Cq = local % p.TC;
   Sync sy(p);
   if (threadIdx.x == 0) {
@@ -1526,6 +1548,14 @@ bool persist_choose_tile(int64_t R, int64_t C, int sms, int* BM, int* BN, bool p
   return false;
 }
 
+template <class Params>
+static const void* persist_kernel(int BM, int BN) {
+  if (BM == 96 && BN == 96) return (const void*)k_persist<96, 96, Params>;
+  if (BM == 64 && BN == 64) return (const void*)k_persist<64, 64, Params>;
+  if (BM == 32 && BN == 32) return (const void*)k_persist<32, 32, Params>;
+  return nullptr;
+}
+
 cudaError_t launch_persist(const PersistParams* p, int count, int BM, int BN, cudaStream_t s) {
   if (count < 1 || count > kPersistMaxParts) return cudaErrorInvalidValue;
   PersistSet set;
@@ -1535,13 +1565,10 @@ cudaError_t launch_persist(const PersistParams* p, int count, int BM, int BN, cu
     set.p[q] = p[q];
     set.first[q + 1] = set.first[q] + p[q].TR * p[q].TC + kPersistExtraCtas;
   }
-  void* args[] = {(void*)&set};
+  void* args[] = {count == 1 ? (void*)&set.p[0] : (void*)&set};
   const size_t smem = sizeof(Shared);
-  const void* fn = nullptr;
-  if (BM == 96 && BN == 96) fn = (const void*)k_persist<96, 96>;
-  else if (BM == 64 && BN == 64) fn = (const void*)k_persist<64, 64>;
-  else if (BM == 32 && BN == 32) fn = (const void*)k_persist<32, 32>;
-  else return cudaErrorInvalidValue;
+  const void* fn = count == 1 ? persist_kernel<PersistParams>(BM, BN) : persist_kernel<PersistSet>(BM, BN);
+  if (!fn) return cudaErrorInvalidValue;
   cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   return cudaLaunchCooperativeKernel(fn, dim3(set.first[count]), dim3(persist_threads(BM, BN)), args, smem, s);

@@ -54,7 +54,7 @@ enum { kTrMathStart = 0, kTrMathOperands, kTrMathCopied, kTrMathPublished, kTrMa
        kTrSrvLoaded, kTrSrvSchur, kTrSrvGJ,
        // publication of the pivot rows / columns and of the server blocks (lead warp)
        kTrGlobEnter, kTrGlobStored, kTrSrvPubEnter, kTrSrvPubStored, kTrSrvPubDone,
-       // T-server: end of the factorization of each 4-pivot group
+       // T-server: end of each four-column panel and its update
        kTrSrvGroup0, kTraceEvents = kTrSrvGroup0 + 8 };
 
 inline int persist_flag_words(int TR, int TC) { return TR + 2 * TC + 1 + TR * TC + 1 + 2 + 1 + TR * TC + 2 + 3; }
