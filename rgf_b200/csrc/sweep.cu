@@ -1286,9 +1286,10 @@ void launch_split_tables(const int* st_col, const double2* st_val, int64_t N, co
   k_split_tables<<<(unsigned)((N + 3) / 4), 128, 0, s>>>(st_col, st_val, N, G0L, G0R, tab);
 }
 
-// first augmented slice matrix of every part (grid.z): A - G0 of the part's
-// own side, its carriers (those of the lead's channels, or for an inner part
-// the identity: X = I, -Z = -I, Y = 0) and the probe pair
+// first augmented slice matrix of every part (grid.z): A less the self-energy it
+// starts behind (its lead's G0, or i for an inner part), its carriers (those of
+// the lead's channels, or for an inner part the identity: X = I, -Z = -I, Y = 0)
+// and the probe pair
 __global__ void k_split_init(const __grid_constant__ SplitInit a) {
   const SplitPart& p = a.part[blockIdx.z];
   const int64_t N = a.N, j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -1298,7 +1299,7 @@ __global__ void k_split_init(const __grid_constant__ SplitInit a) {
     double2 v = zero;
     if (j < N) {
       if (i < N) {
-        v = cneg(p.G0[i * N + j]);
+        v = p.inner ? cmk(0.0, i == j ? -1.0 : 0.0) : cneg(p.G0[i * N + j]);
         for (int q = 0; q < kMaxStencil; q++)
           if (a.st_col[i * kMaxStencil + q] == j) v = cadd(v, a.st_val[i * kMaxStencil + q]);
         if (i == j) v = csub(v, cmul(a.k2, p.eps[i]));
@@ -1323,8 +1324,8 @@ __global__ void k_split_init(const __grid_constant__ SplitInit a) {
       }
     } else if (j == p.pc1 || j == p.pc1 + 1) {
       if (i < N) {
-        const double2 pv = a.tab[i];
-        v = j == p.pc1 ? pv : csub(csub(a.tab[N + i], cmul(cmul(a.k2, p.eps[i]), pv)), p.g0v[i]);
+        const double2 pv = a.tab[i], sv = p.inner ? cmk(-pv.y, pv.x) : p.g0v[i];
+        v = j == p.pc1 ? pv : csub(csub(a.tab[N + i], cmul(cmul(a.k2, p.eps[i]), pv)), sv);
       }
     }
     p.M[i * p.ldm + j] = v;
@@ -1341,20 +1342,20 @@ void launch_split_init(const SplitInit& a, int parts, cudaStream_t s) {
   k_split_init<<<grid, 128, 0, s>>>(a);
 }
 
-// T = [G0 - g; Z] of an end part's state E = [[g, X], [Z, Y]]
-__global__ void k_join_delta(const double2* __restrict__ E, int64_t ldE, const double2* __restrict__ G0, int64_t N,
-                             int64_t rows, double2* __restrict__ T) {
+// T = [i - g; Z] of an end part's state E = [[g, X], [Z, Y]]
+__global__ void k_join_delta(const double2* __restrict__ E, int64_t ldE, int64_t N, int64_t rows,
+                             double2* __restrict__ T) {
   const int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (j >= N) return;
   for (int64_t i = blockIdx.y; i < rows; i += gridDim.y) {
     const double2 e = E[i * ldE + j];
-    T[i * N + j] = i < N ? csub(G0[i * N + j], e) : e;
+    T[i * N + j] = i < N ? cmk(-e.x, (i == j ? 1.0 : 0.0) - e.y) : e;
   }
 }
 
 // the matrix whose sweep joins an end part (state E) with the inner part next
-// to it (state I), F = [G0 - g; Z] [Z_I, Y_I]:
-//   [[1 + (G0 - g) Y_I, (G0 - g) Z_I, -X], [X_I, g_I, 0], [Z Y_I, Z Z_I, Y]]
+// to it (state I), F = [i - g; Z] [Z_I, Y_I]:
+//   [[1 + (i - g) Y_I, (i - g) Z_I, -X], [X_I, g_I, 0], [Z Y_I, Z Z_I, Y]]
 __global__ void k_join_inner(const double2* __restrict__ E, int64_t ldE, const double2* __restrict__ I, int64_t ldI,
                              const double2* __restrict__ F, int64_t N, int ni, int no, double2* __restrict__ Q,
                              int64_t ldQ) {
@@ -1405,9 +1406,9 @@ static dim3 join_grid(int64_t rows, int64_t cols) {
   return dim3((unsigned)((cols + 127) / 128), (unsigned)std::min<int64_t>(rows, 4096));
 }
 
-void launch_join_inner(const double2* E, int64_t ldE, const double2* I, int64_t ldI, const double2* G0, int64_t N, int ni,
-                       int no, double2* T, double2* F, double2* Q, int64_t ldQ, cudaStream_t s) {
-  k_join_delta<<<join_grid(N + no, N), 128, 0, s>>>(E, ldE, G0, N, N + no, T);
+void launch_join_inner(const double2* E, int64_t ldE, const double2* I, int64_t ldI, int64_t N, int ni, int no, double2* T,
+                       double2* F, double2* Q, int64_t ldQ, cudaStream_t s) {
+  k_join_delta<<<join_grid(N + no, N), 128, 0, s>>>(E, ldE, N, N + no, T);
   launch_zgemm(N + no, 2 * N, N, cmk(1.0, 0.0), ZOp{T, N, 0}, ZOp{I + N * ldI, ldI, 0}, cmk(0.0, 0.0), F, 2 * N, s);
   k_join_inner<<<join_grid(2 * N + no, 2 * N + ni), 128, 0, s>>>(E, ldE, I, ldI, F, N, ni, no, Q, ldQ);
 }

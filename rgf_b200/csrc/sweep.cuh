@@ -109,8 +109,8 @@ struct SplitInit {
 void launch_split_tables(const int* st_col, const double2* st_val, int64_t N, const double2* G0L, const double2* G0R,
                          double2* tab, cudaStream_t s);
 void launch_split_init(const SplitInit& a, int parts, cudaStream_t s);
-void launch_join_inner(const double2* E, int64_t ldE, const double2* I, int64_t ldI, const double2* G0, int64_t N, int ni,
-                       int no, double2* T, double2* F, double2* Q, int64_t ldQ, cudaStream_t s);
+void launch_join_inner(const double2* E, int64_t ldE, const double2* I, int64_t ldI, int64_t N, int ni, int no, double2* T,
+                       double2* F, double2* Q, int64_t ldQ, cudaStream_t s);
 void launch_join_ends(const double2* L, int64_t ldL, const double2* R, int64_t ldR, int64_t N, int niL, int niR, int noL,
                       int noR, double2* F, double2* Q, int64_t ldQ, cudaStream_t s);
 
