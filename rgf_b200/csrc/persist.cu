@@ -335,12 +335,11 @@ __device__ void math_role(const PersistParams& p, Shared& sh, const Sync& sy, in
   // works on its own accumulators only.  The probe pair is the column pair
   // (pc1, pc1 + 1), pc1 even, so one thread holds both as h = 0, 1.
   // Returns the largest probe residual this thread saw.
-  // No step of the sweep runs meanwhile, so what counts is the latency of the
-  // slowest warp: v and A0 v come from tables, the slice's eps is read by the
-  // warps on the diagonal or the probe pair only, all rows at once, and the
-  // stencil by the warps that hold one of its entries (a slice of N = 1000 went
-  // from 575 to 553 us, of N = 64 on 32 x 32 tiles from 42.1 to 40.4 us).
-  const bool on_diag = t.r_base < t.c_base + Tile::WC && t.c_base < t.r_base + Tile::WR;
+  // No step of the sweep runs meanwhile, and code that runs once a slice has gone
+  // cold (a fetch costs ~270 cycles per 128 bytes): the unrolled work on the
+  // accumulators is kept to sign flips, what needs more sits behind branches that
+  // most warps jump over, v and A0 v come from tables, and the slice's eps and
+  // the stencil are read by the warps that hold one of its entries only.
   const bool on_probe = p.pc1 >= t.c_base && p.pc1 < t.c_base + Tile::WC;
   bool on_stencil = false;
   for (int e = t.lane; e < Tile::WR * kMaxStencil; e += 32) {
@@ -351,24 +350,35 @@ __device__ void math_role(const PersistParams& p, Shared& sh, const Sync& sy, in
   on_stencil = __any_sync(kFull, on_stencil);
   auto boundary_regs = [&](const double2* eps_next, double2* snap) {
     double pmax = 0.0;
+    if (snap) {
+#pragma unroll
+      for (int mi = 0; mi < MI; mi++)
+#pragma unroll
+        for (int ni = 0; ni < NI; ni++)
+#pragma unroll
+          for (int h = 0; h < 2; h++) {
+            const int i = t.row(mi), j = t.col(ni, h);
+            if (i < p.R && j < p.pc1) __stcg(snap + (int64_t)i * p.ldm + j, cmk(t.acc[mi][ni][h], t.acc[mi][ni][2 + h]));
+          }
+    }
     double2 ke[MI];
 #pragma unroll
-    for (int mi = 0; mi < MI; mi++) {
-      const int i = t.row(mi);
-      ke[mi] = (eps_next && (on_diag || on_probe) && i < p.N) ? __ldg(eps_next + i) : cmk(0.0, 0.0);
+    for (int mi = 0; mi < MI; mi++) ke[mi] = cmk(0.0, 0.0);
+    if (eps_next && (on_stencil || on_probe)) {
+#pragma unroll
+      for (int mi = 0; mi < MI; mi++) ke[mi] = t.row(mi) < p.N ? __ldg(eps_next + t.row(mi)) : cmk(0.0, 0.0);
+#pragma unroll
+      for (int mi = 0; mi < MI; mi++) ke[mi] = cmul(p.k2, ke[mi]);
     }
-#pragma unroll
-    for (int mi = 0; mi < MI; mi++) ke[mi] = cmul(p.k2, ke[mi]);
-#pragma unroll
-    for (int mi = 0; mi < MI; mi++) {
-      const int i = t.row(mi);
-      if (i >= p.R) continue;
+    if (on_probe) {
 #pragma unroll
       for (int ni = 0; ni < NI; ni++) {
-        const int j0c = t.col(ni, 0);  // even; j0c + 1 is the h = 1 column
-        if (j0c >= p.C) continue;
-        double* a = t.acc[mi][ni];
-        if (j0c == p.pc1) {
+        if ((unsigned)(p.pc1 - (t.c_base + ni * 8)) >= 8u) continue;  // the same for the whole warp
+#pragma unroll
+        for (int mi = 0; mi < MI; mi++) {
+          const int i = t.row(mi);
+          if (t.col(ni, 0) != p.pc1 || i >= p.R) continue;
+          double* a = t.acc[mi][ni];
           if (i < p.N) {
             const double2 v = __ldg(p.probe + i);
             const double rr = sqrt(cabs2(csub(cmk(a[1], a[3]), v)));
@@ -383,29 +393,35 @@ __device__ void math_role(const PersistParams& p, Shared& sh, const Sync& sy, in
           } else if (eps_next) {
             a[0] = a[1] = a[2] = a[3] = 0.0;
           }
-          continue;
-        }
-#pragma unroll
-        for (int h = 0; h < 2; h++) {
-          const int j = j0c + h;
-          if (j >= p.C) continue;
-          if (snap) __stcg(snap + (int64_t)i * p.ldm + j, cmk(a[h], a[2 + h]));
-          if (!eps_next || j >= p.N) continue;  // X columns and the Y block are carried unchanged
-          a[h] = -a[h];  // -G_n, or the -Z rows
-          a[2 + h] = -a[2 + h];
-          if (i == j) {
-            a[h] -= ke[mi].x;
-            a[2 + h] -= ke[mi].y;
-          }
         }
       }
-      // + A0 (stencil entries of row i), one entry at a time
-      if (!eps_next || !on_stencil || i >= p.N) continue;
+    }
+    if (!eps_next) return pmax;
+    // -G_n, and the -Z rows; X columns, the Y block and the probe pair keep their sign
+#pragma unroll
+    for (int ni = 0; ni < NI; ni++)
+#pragma unroll
+      for (int h = 0; h < 2; h++) {
+        const int flip = t.col(ni, h) < p.N ? (int)0x80000000 : 0;
+#pragma unroll
+        for (int mi = 0; mi < MI; mi++) {
+          double* a = t.acc[mi][ni];
+          a[h] = __hiloint2double(__double2hiint(a[h]) ^ flip, __double2loint(a[h]));
+          a[2 + h] = __hiloint2double(__double2hiint(a[2 + h]) ^ flip, __double2loint(a[2 + h]));
+        }
+      }
+    if (!on_stencil) return pmax;
+    // + A0 - k0dx^2 eps (stencil entries of row i), one entry at a time
+#pragma unroll
+    for (int mi = 0; mi < MI; mi++) {
+      const int i = t.row(mi);
+      if (i >= p.N) continue;
 #pragma unroll 1
       for (int q = 0; q < kMaxStencil; q++) {
         const int cq = __ldg(p.st_col + (int64_t)i * kMaxStencil + q);
         if (cq < t.c_base || cq >= t.c_base + Tile::WC) continue;
-        const double2 v = __ldg(p.st_val + (int64_t)i * kMaxStencil + q);
+        double2 v = __ldg(p.st_val + (int64_t)i * kMaxStencil + q);
+        if (cq == i) v = csub(v, ke[mi]);
 #pragma unroll
         for (int ni = 0; ni < NI; ni++)
 #pragma unroll
@@ -447,37 +463,33 @@ __device__ void math_role(const PersistParams& p, Shared& sh, const Sync& sy, in
       }
     }
   };
+  // The publications below copy accumulators as they are wherever they can:
+  // padding beyond the last pivot row or column is the readers' business, so that
+  // the code, cold whenever a CTA comes to hold the next pieces, stays short.
+  //
   // 32x32 block (rows in window wr_, columns in window wc_) of W into a
-  // row-major [32][32] buffer; rows / columns at or beyond `lim` are padded
-  // with the identity (pad_id) or zeros
-  auto store_block = [&](double2* dst, int wr_, int wc_, int lim_r, int lim_c, bool pad_id) {
+  // row-major [32][32] buffer
+  auto store_block = [&](double2* dst, int wr_, int wc_) {
+    double2* q0 = dst + (t.r_base + lr - wr_) * kPB + t.c_base + lc - wc_;
 #pragma unroll
     for (int mi = 0; mi < MI; mi++) {
       if (!row_in(mi, wr_)) continue;
-      const int r = t.r_base + mi * 8 + lr - wr_;
 #pragma unroll
       for (int ni = 0; ni < NI; ni++) {
         if (!col_in(ni, wc_)) continue;
-        const int c0 = t.c_base + ni * 8 + lc - wc_;
 #pragma unroll
-        for (int h = 0; h < 2; h++) {
-          const int c = c0 + h;
-          const bool in = r < lim_r && c < lim_c;
-          const double2 v = in ? cmk(t.acc[mi][ni][h], t.acc[mi][ni][2 + h])
-                               : cmk((pad_id && r == c) ? 1.0 : 0.0, 0.0);
-          __stcg(dst + r * kPB + c, v);
-        }
+        for (int h = 0; h < 2; h++)
+          __stcg(q0 + mi * 8 * kPB + ni * 8 + h, cmk(t.acc[mi][ni][h], t.acc[mi][ni][2 + h]));
       }
     }
   };
   // the first pivot block of a slice -> djjbuf for the T-server
   auto publish_djj = [&](int s1) {
     const int w0 = (s1 % p.NB) * kPB;
-    const int jnn = min(kPB, p.N - w0);
     int ok = 1;
     if (t.lane == 0 && s1 >= p.NB) ok = wait_ge(p, sy.d_used, s1 - p.NB);  // previous slice's was loaded
     ok = __shfl_sync(kFull, ok, 0);
-    if (ok) store_block(p.djjbuf, w0, w0, jnn, jnn, true);
+    if (ok) store_block(p.djjbuf, w0, w0);
     int lead;
     const int n = pub_set(kSetDjj, s1, &lead);
     const int all_ok = !bar_or(kBarDjj, n * 32, !ok);
@@ -504,10 +516,21 @@ __device__ void math_role(const PersistParams& p, Shared& sh, const Sync& sy, in
       // Pc = [-W(i, J) ; +I on the pivot rows], zero beyond the last pivot
       // column and below row R, stored in the swizzled [BM][32] layout
       double2* pcb = p.pcbuf + ((size_t)par * p.TR + I) * (BM * kPB) + (t.r_base - tr0 + lr) * kPB;
+      // most warps: no pivot rows, no padding
+      const bool plain = jnn == kPB && t.r_base + Tile::WR <= p.R && (t.r_base + Tile::WR <= w0 || t.r_base >= w0 + kPB);
 #pragma unroll
       for (int ni = 0; ni < NI; ni++) {
         if (!col_in(ni, w0)) continue;
-        const int kc = t.c_base + ni * 8 - w0;  // multiple of 8: the swizzle acts on lc + h only
+        double2* q = pcb + t.c_base + ni * 8 - w0;  // multiple of 8: the swizzle acts on lc + h only
+        if (plain) {
+#pragma unroll
+          for (int mi = 0; mi < MI; mi++)
+#pragma unroll
+            for (int h = 0; h < 2; h++)
+              __stcg(q + mi * 8 * kPB + ((lc + h) ^ sw), cmk(-t.acc[mi][ni][h], -t.acc[mi][ni][2 + h]));
+          continue;
+        }
+        const int kc = t.c_base + ni * 8 - w0;
 #pragma unroll
         for (int mi = 0; mi < MI; mi++) {
           const int i = t.r_base + mi * 8 + lr;
@@ -518,7 +541,7 @@ __device__ void math_role(const PersistParams& p, Shared& sh, const Sync& sy, in
             if (k >= jnn || i >= p.R) wv = cmk(0.0, 0.0);
             else if (i >= w0 && i < w0 + jnn) wv = cmk((i - w0 == k) ? 1.0 : 0.0, 0.0);
             else wv = cmk(-t.acc[mi][ni][h], -t.acc[mi][ni][2 + h]);
-            __stcg(pcb + mi * 8 * kPB + kc + ((lc + h) ^ sw), wv);
+            __stcg(q + mi * 8 * kPB + ((lc + h) ^ sw), wv);
           }
         }
       }
@@ -530,11 +553,10 @@ __device__ void math_role(const PersistParams& p, Shared& sh, const Sync& sy, in
       trace_ev(p, s1 - 1, kTrMathPublished);
     }
   };
-  // rows J_x of the current W (prebuf[x & 1][Cq][k][c - tc0], zero beyond the
-  // last pivot row) for the panels of tile column Cq
+  // rows J_x of the current W (prebuf[x & 1][Cq][k][c - tc0]) for the panels of
+  // tile column Cq
   auto publish_pre = [&](int x, int bar_id) {
     const int w0 = (x % p.NB) * kPB;
-    const int jnn = min(kPB, p.N - w0);
     const int par = x & 1;
     int lead;
     const int n = pub_set(kSetPre, x, &lead);
@@ -542,31 +564,27 @@ __device__ void math_role(const PersistParams& p, Shared& sh, const Sync& sy, in
     if (t.lane == 0 && x >= 2) ok = wait_ge(p, sy.pre_cons + par * p.TC + Cq, p.TR * (x >> 1));
     ok = __shfl_sync(kFull, ok, 0);
     if (ok) {
-      double2* rowb = p.prebuf + ((size_t)par * p.TC + Cq) * (kPB * BN) + (t.c_base - tc0 + lc);
+      double2* rowb = p.prebuf + ((size_t)par * p.TC + Cq) * (kPB * BN) + (t.c_base - tc0 + lc) +
+                      (t.r_base + lr - w0) * BN;
 #pragma unroll
       for (int mi = 0; mi < MI; mi++) {
         if (!row_in(mi, w0)) continue;
-        const int kr = t.r_base + mi * 8 + lr - w0;
-        const bool valid = kr < jnn;
-        double2* q = rowb + kr * BN;
 #pragma unroll
         for (int ni = 0; ni < NI; ni++)
 #pragma unroll
           for (int h = 0; h < 2; h++)
-            __stcg(q + ni * 8 + h, valid ? cmk(t.acc[mi][ni][h], t.acc[mi][ni][2 + h]) : cmk(0.0, 0.0));
+            __stcg(rowb + mi * 8 * BN + ni * 8 + h, cmk(t.acc[mi][ni][h], t.acc[mi][ni][2 + h]));
       }
     }
     const int all_ok = !bar_or(bar_id, n * 32, !ok);
     if (warp == lead && t.lane == 0 && all_ok) st_release(sy.pre_flag + par * p.TC + Cq, x);
   };
-  // blocks (J_s2, J_s2) (padded with the identity beyond the last pivot row)
-  // and (J_s2, J_s1) (zero rows there) of the current W, s2 = s1+1, for the
-  // T-server's prep warps, which update them by step s2-2 (unless s2 is the
-  // second step of its slice) into the blocks of the Schur update of step s2
+  // blocks (J_s2, J_s2) and (J_s2, J_s1) of the current W, s2 = s1+1, for the
+  // prep CTA, which updates them by step s2-2 (unless s2 is the second step of
+  // its slice) into the blocks of the Schur update of step s2
   auto publish_srv = [&](int s1, int bar_id) {
     const int s2 = s1 + 1;
     const int w1 = (s1 % p.NB) * kPB, w2 = w1 + kPB;
-    const int jn2 = min(kPB, p.N - w2);
     const int par = s2 & 1;
     int lead;
     const int n = pub_set(kSetSrv, s1, &lead);
@@ -575,8 +593,8 @@ __device__ void math_role(const PersistParams& p, Shared& sh, const Sync& sy, in
     if (t.lane == 0 && s2 >= 2) ok = wait_ge(p, sy.srv_cons + par, s2 >> 1);
     ok = __shfl_sync(kFull, ok, 0);
     if (ok) {
-      store_block(p.srvbuf + (size_t)par * 2 * kPB * kPB, w2, w2, jn2, jn2, true);
-      store_block(p.srvbuf + ((size_t)par * 2 + 1) * kPB * kPB, w2, w1, jn2, kPB, false);
+      store_block(p.srvbuf + (size_t)par * 2 * kPB * kPB, w2, w2);
+      store_block(p.srvbuf + ((size_t)par * 2 + 1) * kPB * kPB, w2, w1);
     }
     if (warp == lead && t.lane == 0) trace_ev(p, s1 - 1, kTrSrvPubStored);
     const int all_ok = !bar_or(bar_id, n * 32, !ok);
@@ -1148,12 +1166,13 @@ __device__ void yprep_role(const PersistParams& p, Shared& sh, const Sync& sy, i
   constexpr int kPer = kPB * kPB / kServerThreads;
   // bounded load of a 32x32 block (row stride ld; entries outside rows x cols
   // zero; column c read at col_of(c)) into a padded shared block
-  auto load_blk = [&](Blk& dst, const double2* src, int ld, int rows, int cols, auto col_of) {
+  auto load_blk = [&](Blk& dst, const double2* src, int ld, int rows, int cols, auto col_of, bool pad_id = false) {
     double2 v[kPer];
 #pragma unroll
     for (int u = 0; u < kPer; u++) {
       const int e = t + u * kServerThreads, q = e / kPB, c = e % kPB;
-      v[u] = (q < rows && c < cols) ? __ldcg(src + (size_t)q * ld + col_of(q, c)) : cmk(0.0, 0.0);
+      v[u] = (q < rows && c < cols) ? __ldcg(src + (size_t)q * ld + col_of(q, c))
+                                    : cmk(pad_id && q == c ? 1.0 : 0.0, 0.0);
     }
 #pragma unroll
     for (int u = 0; u < kPer; u++) dst[(t + u * kServerThreads) / kPB][(t + u * kServerThreads) % kPB] = v[u];
@@ -1184,13 +1203,10 @@ __device__ void yprep_role(const PersistParams& p, Shared& sh, const Sync& sy, i
     }
     bar_sync(kBarMath, kServerThreads);
     if (sh.panel_abort) return;
-    if (k == 0) {
-      load_blk(y0, p.djjbuf, kPB, kPB, kPB, plain);
-    } else {
-      const double2* sb = p.srvbuf + (size_t)par * 2 * kPB * kPB;
-      load_blk(y0, sb, kPB, kPB, kPB, plain);
-      load_blk(y1, sb + kPB * kPB, kPB, kPB, kPB, plain);
-    }
+    // beyond jn the pivot block is padded with the identity, y1 with zero rows
+    const double2* sb = p.srvbuf + (size_t)par * 2 * kPB * kPB;
+    load_blk(y0, k == 0 ? p.djjbuf : sb, kPB, jn, jn, plain, true);
+    if (k != 0) load_blk(y1, sb + kPB * kPB, kPB, jn, kPB, plain);
     if (k >= 2) {
       // Pc_{x-2}(J_x, :), rows beyond jn zero -> sh.T; U_{x-2}(:, J_x), columns
       // beyond jn zero -> sh.Mr; U_{x-2}(:, J_{x-1}) -> srv.v
@@ -1495,20 +1511,16 @@ __global__ void __launch_bounds__(Cfg<BM, BN>::Threads, 1)
 size_t persist_smem_bytes() { return sizeof(Shared); }
 
 cudaError_t launch_persist_gang(const PersistParams* params, const int* ctas, int count, GangState* state, int grid,
-                                long long sched_timeout, int BM, int BN, cudaStream_t s) {
+                                long long sched_timeout, cudaStream_t s) {
   if (count > kGangMaxItems) return cudaErrorInvalidValue;
-  const void* fn = nullptr;
-  if (BM == 96 && BN == 96) fn = (const void*)k_persist_gang<96, 96>;
-  else if (BM == 64 && BN == 64) fn = (const void*)k_persist_gang<64, 64>;
-  else if (BM == 32 && BN == 32) fn = (const void*)k_persist_gang<32, 32>;
-  else return cudaErrorInvalidValue;
+  const void* fn = (const void*)k_persist_gang<kMaxTile, kMaxTile>;
   const size_t smem = sizeof(Shared);
   cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   e = cudaMemcpyToSymbolAsync(c_gang_p, params, sizeof(PersistParams) * count, 0, cudaMemcpyHostToDevice, s);
   if (e != cudaSuccess) return e;
   void* args[] = {(void*)&ctas, (void*)&count, (void*)&state, (void*)&sched_timeout};
-  return cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(persist_threads(BM, BN)), args, smem, s);
+  return cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(persist_threads(kMaxTile, kMaxTile)), args, smem, s);
 }
 
 int persist_threads(int BM, int BN) {

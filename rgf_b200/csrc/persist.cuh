@@ -66,7 +66,8 @@ inline int persist_cons_words(int TR, int TC) { return 2 * TR + 2 * TC + 2 + 2 *
 // work queue, see persist.cu).  params / ctas (host) are ordered by cost,
 // largest first; ctas[i] = TR * TC + kPersistExtraCtas <= grid; at most
 // kGangMaxItems structures.  Launches that share a device must not overlap
-// (the parameters live in one constant-memory array).
+// (the parameters live in one constant-memory array).  All sweeps of a gang
+// launch run on 96 x 96 tiles.
 constexpr int kGangMaxCtas = 1024;
 constexpr int kGangMaxItems = 160;  // structures per launch (constant memory)
 constexpr int kGangWindow = 16;     // queue positions a free pool may look ahead
@@ -77,7 +78,7 @@ struct GangState {  // zero-initialised before the launch
   int taken[kGangMaxItems];
 };
 cudaError_t launch_persist_gang(const PersistParams* params, const int* ctas, int count, GangState* state, int grid,
-                                long long sched_timeout, int BM, int BN, cudaStream_t s);
+                                long long sched_timeout, cudaStream_t s);
 
 size_t persist_smem_bytes();
 int persist_threads(int BM, int BN);

@@ -493,7 +493,7 @@ void gang_launch(GangBatch* g) {
   const double sched_s = std::max(30.0, 3.0 * est_s);
   const long long sched_cycles = (long long)(sched_s * 1e3 * clk_khz);
   if (e == cudaSuccess)
-    e = launch_persist_gang(params.data(), d_ctas, (int)ctas.size(), d_state, g->sms, sched_cycles, 96, 96,
+    e = launch_persist_gang(params.data(), d_ctas, (int)ctas.size(), d_state, g->sms, sched_cycles,
                             g->stream);
   int abort_word = 0;
   if (e == cudaSuccess)
