@@ -636,10 +636,10 @@ int64_t part_ctas(int64_t N, int no, int ni, int tile) {
 }
 
 // us of one slice of the persistent sweep with NB pivot blocks on tiles of
-// 96, 64, 32 (measured at N = 64, 157, 256, 512, 1000: 98, 146, 175, 302, 553;
-// 50, 93, 136, 253; 40, 85, 128), and of one join
+// 96, 64, 32 (measured at N = 64, 157, 256, 512, 1000: 90, 133, 160, 284, 522;
+// 47, 83, 114, 212; 36, 71, 107), and of one join
 double slice_us(int tile, int64_t NB) {
-  return tile == 96 ? 66.0 + 15.0 * NB : tile == 64 ? 21.6 + 14.3 * NB : 11.3 + 14.55 * NB;
+  return tile == 96 ? 60.0 + 14.2 * NB : tile == 64 ? 23.0 + 11.8 * NB : 13.0 + 11.7 * NB;
 }
 double join_us(int64_t NB) { return 40.0 + 45.0 * NB; }
 
