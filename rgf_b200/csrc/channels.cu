@@ -76,19 +76,17 @@ __global__ void k_transverse(Transverse tr, double* k0, double* k1) {
   if (tr.dim == 3 && a < tr.n1) k1[a] = transverse_k(tr.bc, tr.n1, ka1, a);
 }
 
-// One side (L or R) of setup_longitudinal for every channel a.
-__global__ void k_longitudinal(Transverse tr, const double* k0, const double* k1, double2 k2e,
-                               SideDev side) {
-  int64_t a = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (a >= tr.N) return;
+// setup_longitudinal for channel a of one side (L or R), transverse wave numbers
+// kx0 (fast axis) and ky0 (3D)
+__device__ __forceinline__ void longitudinal(const Transverse& tr, int64_t a, double kx0, double ky0, double2 k2e,
+                                             const SideDev& side) {
   const bool is_real = (k2e.y == 0.0);
   double2 z;
   if (tr.dim == 2) {
-    double s = sin(k0[a] / 2.0);
+    double s = sin(kx0 / 2.0);
     z = cmk(0.25 * k2e.x - s * s, 0.25 * k2e.y);  // setup_channels.m:185
   } else {
-    int64_t ax = a % tr.n0, ay = a / tr.n0;
-    double sx = sin(k0[ax] / 2.0), sy = sin(k1[ay] / 2.0);
+    double sx = sin(kx0 / 2.0), sy = sin(ky0 / 2.0);
     z = cmk((0.25 * k2e.x - sx * sx) - sy * sy, 0.25 * k2e.y);  // setup_channels_3D.m:152
   }
   if (is_real) z.y = 0.0;
@@ -118,9 +116,17 @@ __global__ void k_longitudinal(Transverse tr, const double* k0, const double* k1
   side.isprop[a] = (z.x > 0.0 && z.x < 1.0) ? 1 : 0;  // setup_channels.m:195
 }
 
+__global__ void k_longitudinal(Transverse tr, const double* k0, const double* k1, double2 k2e,
+                               SideDev side) {
+  int64_t a = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (a >= tr.N) return;
+  if (tr.dim == 2) longitudinal(tr, a, k0[a], 0.0, k2e, side);
+  else longitudinal(tr, a, k0[a % tr.n0], k1[a / tr.n0], k2e, side);
+}
+
 // Single-CTA ordered compaction of the propagating flags (MATLAB find) and
 // the reciprocity permutation ind_prop_conj (setup_channels.m:222-236).
-__global__ void k_compact_prop(int64_t N, SideDev side, int conj_mode, int64_t ind_zero0) {
+__device__ __forceinline__ void compact_prop(int64_t N, const SideDev& side, int conj_mode, int64_t ind_zero0) {
   __shared__ int64_t warp_tot[32];
   __shared__ int64_t base;
   if (threadIdx.x == 0) base = 0;
@@ -162,6 +168,29 @@ __global__ void k_compact_prop(int64_t N, SideDev side, int conj_mode, int64_t i
       else side.conj[p] = (p == Np - 1) ? (int)(Np - 1) : (int)(Np - 2 - p);
     }
   }
+}
+
+__global__ void k_compact_prop(int64_t N, SideDev side, int conj_mode, int64_t ind_zero0) {
+  compact_prop(N, side, conj_mode, ind_zero0);
+}
+
+// The whole set-up in one launch, a CTA per side: launches, not arithmetic, are
+// what a set-up of some thousand channels costs.
+__global__ void __launch_bounds__(1024) k_channels(Transverse tr, double* k0, double* k1, double2 k2eL, double2 k2eR,
+                                                   SideDev L, SideDev R, int conj_mode, int64_t ind_zero0) {
+  const SideDev& side = blockIdx.x == 0 ? L : R;
+  const double2 k2e = blockIdx.x == 0 ? k2eL : k2eR;
+  const double ka0 = (tr.bc == RGF_BC_BLOCH) ? tr.ka0 : 0.0, ka1 = (tr.bc == RGF_BC_BLOCH) ? tr.ka1 : 0.0;
+  for (int64_t a = threadIdx.x; a < tr.N; a += blockDim.x) {
+    const int64_t ax = tr.dim == 2 ? a : a % tr.n0, ay = tr.dim == 2 ? 0 : a / tr.n0;
+    const double kx0 = transverse_k(tr.bc, tr.n0, ka0, ax);
+    const double ky0 = tr.dim == 3 ? transverse_k(tr.bc, tr.n1, ka1, ay) : 0.0;
+    if (blockIdx.x == 0 && ay == 0) k0[ax] = kx0;
+    if (blockIdx.x == 0 && tr.dim == 3 && ax == 0) k1[ay] = ky0;
+    longitudinal(tr, a, kx0, ky0, k2e, side);
+  }
+  __syncthreads();
+  compact_prop(tr.N, side, conj_mode, ind_zero0);
 }
 
 // 1D transverse profile of mode a at site m (0-based), setup_channels.m:133-156
@@ -365,16 +394,24 @@ __global__ void k_laplacian_dense(int64_t n, int bc, double ka, double2* A) {
 }
 
 // ---- host-side launchers ----------------------------------------------------
-void launch_transverse(const Transverse& tr, double* k0, double* k1, cudaStream_t s) {
-  int64_t n = tr.n0 > tr.n1 ? tr.n0 : tr.n1;
+// One launch up to kOneLaunch channels (501 channels, two sides: 5 launches and 10
+// copies of 190 us became one and one of 50 us); beyond, a CTA's share of the
+// transcendental functions outweighs the launches and every channel gets a thread
+// of the whole GPU.
+constexpr int64_t kOneLaunch = 8192;
+int launch_channels(const Transverse& tr, double* k0, double* k1, const double2 k2e[2], const SideDev side[2], int sides,
+                    int conj_mode, int64_t ind_zero0, cudaStream_t s) {
+  if (tr.N <= kOneLaunch) {
+    k_channels<<<sides, 1024, 0, s>>>(tr, k0, k1, k2e[0], k2e[1], side[0], side[1], conj_mode, ind_zero0);
+    return 1;
+  }
+  const int64_t n = tr.n0 > tr.n1 ? tr.n0 : tr.n1;
   k_transverse<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(tr, k0, k1);
-}
-void launch_longitudinal(const Transverse& tr, const double* k0, const double* k1, double2 k2e,
-                         const SideDev& side, cudaStream_t s) {
-  k_longitudinal<<<(unsigned)((tr.N + 255) / 256), 256, 0, s>>>(tr, k0, k1, k2e, side);
-}
-void launch_compact(int64_t N, const SideDev& side, int conj_mode, int64_t ind_zero0, cudaStream_t s) {
-  k_compact_prop<<<1, 1024, 0, s>>>(N, side, conj_mode, ind_zero0);
+  for (int q = 0; q < sides; q++) {
+    k_longitudinal<<<(unsigned)((tr.N + 255) / 256), 256, 0, s>>>(tr, k0, k1, k2e[q], side[q]);
+    k_compact_prop<<<1, 1024, 0, s>>>(tr.N, side[q], conj_mode, ind_zero0);
+  }
+  return 1 + 2 * sides;
 }
 void launch_phi(const Transverse& tr, const double* k0, const double* k1, double2* phi, int64_t ld,
                 cudaStream_t s) {

@@ -15,10 +15,10 @@ struct SideDev {
   int* conj;        // ind_prop_conj (0-based), when defined
 };
 
-void launch_transverse(const Transverse& tr, double* k0, double* k1, cudaStream_t s);
-void launch_longitudinal(const Transverse& tr, const double* k0, const double* k1, double2 k2e,
-                         const SideDev& side, cudaStream_t s);
-void launch_compact(int64_t N, const SideDev& side, int conj_mode, int64_t ind_zero0, cudaStream_t s);
+// transverse and longitudinal wave numbers, propagating channels of `sides` leads;
+// returns the number of launches
+int launch_channels(const Transverse& tr, double* k0, double* k1, const double2 k2e[2], const SideDev side[2], int sides,
+                    int conj_mode, int64_t ind_zero0, cudaStream_t s);
 void launch_phi(const Transverse& tr, const double* k0, const double* k1, double2* phi, int64_t ld,
                 cudaStream_t s);
 void launch_stencil(const Transverse& tr, int* st_col, double2* st_val, cudaStream_t s);

@@ -78,7 +78,7 @@ struct rgf_handle_s {
   int64_t prof_n = 0;
   double prof_ms = 0.0, prof_flops = 0.0;
   // workspace (grow-only)
-  DevBuf k0, k1, kx[2], lam[2], mu[2], isprop[2], prop[2], conj[2], nprop, status;
+  DevBuf chan, status;  // chan: every channel array (ChanLayout)
   DevBuf phi, tmp, g0s, g0e, st_col, st_val, eps, aug, pc, u, idx, sdev;
   DevBuf xpc, xrow, xt, xu, xsync, xprobe;  // persistent-kernel exchange buffers
   DevBuf gck, gseg, gm0, gpsi, gphi, get, gd, gg;   // permittivity gradient (checkpoints, carriers)
@@ -197,43 +197,55 @@ rgf_status check_launch() {
 // ---------------------------------------------------------------------------
 // channels (setup_channels.m / setup_channels_3D.m)
 // ---------------------------------------------------------------------------
+// The channel arrays in one block: what the caller may ask for first, so that one
+// copy brings it to the host.
+struct ChanLayout {
+  size_t nprop = 0, k0, k1, kx[2], mu[2], prop[2], conj[2], lam[2], isprop[2], host, bytes;
+  explicit ChanLayout(const Transverse& tr, int sides) {
+    const size_t N = (size_t)tr.N;
+    size_t at = 16;
+    auto take = [&](size_t b) {
+      const size_t o = at;
+      at += (b + 15) & ~(size_t)15;
+      return o;
+    };
+    k0 = take(sizeof(double) * tr.n0);
+    k1 = take(sizeof(double) * tr.n1);
+    for (int s = 0; s < 2; s++) {
+      kx[s] = s < sides ? take(sizeof(double2) * N) : kx[0];
+      mu[s] = s < sides ? take(sizeof(double2) * N) : mu[0];
+      prop[s] = s < sides ? take(sizeof(int) * N) : prop[0];
+      conj[s] = s < sides ? take(sizeof(int) * N) : conj[0];
+    }
+    host = at;
+    for (int s = 0; s < 2; s++) {
+      lam[s] = s < sides ? take(sizeof(double2) * N) : lam[0];
+      isprop[s] = s < sides ? take(sizeof(int) * N) : isprop[0];
+    }
+    bytes = at;
+  }
+};
+
 struct ChanInfo {
   int64_t np[2] = {0, 0};
   bool same = false;   // R side aliases L (epsilon_R == epsilon_L, setup_channels.m:166)
   bool two_sided = true;
   bool has_conj = false;
   SideDev side[2];
+  double *k0 = nullptr, *k1 = nullptr;
+  std::vector<unsigned char> host;  // the block's host part, when asked for
 };
 
-SideDev side_of(rgf_handle h, int s) {
-  SideDev d;
-  d.kx = as<double2>(h->kx[s]);
-  d.lam = as<double2>(h->lam[s]);
-  d.sqrtmu = as<double2>(h->mu[s]);
-  d.isprop = as<int>(h->isprop[s]);
-  d.prop = as<int>(h->prop[s]);
-  d.nprop = as<int>(h->nprop) + s;
-  d.conj = as<int>(h->conj[s]);
-  return d;
-}
-
-rgf_status run_channels(rgf_handle h, const Transverse& tr, double2 k2eL, double2 k2eR, bool two_sided,
+// want_host: keep the arrays a caller may ask for (copy_channels_out)
+rgf_status run_channels(rgf_handle h, const Transverse& tr, double2 k2eL, double2 k2eR, bool two_sided, bool want_host,
                         ChanInfo* ci) {
-  const int64_t N = tr.N;
   rgf_status st;
-  if ((st = ensure(h, h->k0, sizeof(double) * tr.n0))) return st;
-  if ((st = ensure(h, h->k1, sizeof(double) * tr.n1))) return st;
-  for (int s = 0; s < 2; s++) {
-    if ((st = ensure(h, h->kx[s], sizeof(double2) * N))) return st;
-    if ((st = ensure(h, h->lam[s], sizeof(double2) * N))) return st;
-    if ((st = ensure(h, h->mu[s], sizeof(double2) * N))) return st;
-    if ((st = ensure(h, h->isprop[s], sizeof(int) * N))) return st;
-    if ((st = ensure(h, h->prop[s], sizeof(int) * N))) return st;
-    if ((st = ensure(h, h->conj[s], sizeof(int) * N))) return st;
-  }
-  if ((st = ensure(h, h->nprop, sizeof(int) * 2))) return st;
   ci->two_sided = two_sided;
   ci->same = !two_sided || (k2eL.x == k2eR.x && k2eL.y == k2eR.y);
+  const int sides = ci->same ? 1 : 2;
+  const ChanLayout lay(tr, sides);
+  if ((st = ensure(h, h->chan, lay.bytes))) return st;
+  unsigned char* base = as<unsigned char>(h->chan);
   int conj_mode = 0;
   int64_t ind_zero0 = -1;
   if (tr.dim == 2) {
@@ -245,33 +257,37 @@ rgf_status run_channels(rgf_handle h, const Transverse& tr, double2 k2eL, double
     }
   }
   ci->has_conj = conj_mode != 0;
-  launch_transverse(tr, as<double>(h->k0), as<double>(h->k1), h->stream);
-  h->launches++;
+  ci->k0 = reinterpret_cast<double*>(base + lay.k0);
+  ci->k1 = reinterpret_cast<double*>(base + lay.k1);
   for (int s = 0; s < 2; s++) {
-    ci->side[s] = side_of(h, s);
-    if (s == 1 && ci->same) {
-      ci->side[1] = ci->side[0];
-      continue;
-    }
-    launch_longitudinal(tr, as<double>(h->k0), as<double>(h->k1), s == 0 ? k2eL : k2eR, ci->side[s], h->stream);
-    launch_compact(N, ci->side[s], conj_mode, ind_zero0, h->stream);
-    h->launches += 2;
+    SideDev& d = ci->side[s];
+    d.kx = reinterpret_cast<double2*>(base + lay.kx[s]);
+    d.lam = reinterpret_cast<double2*>(base + lay.lam[s]);
+    d.sqrtmu = reinterpret_cast<double2*>(base + lay.mu[s]);
+    d.isprop = reinterpret_cast<int*>(base + lay.isprop[s]);
+    d.prop = reinterpret_cast<int*>(base + lay.prop[s]);
+    d.nprop = reinterpret_cast<int*>(base + lay.nprop) + (ci->same ? 0 : s);
+    d.conj = reinterpret_cast<int*>(base + lay.conj[s]);
   }
+  const double2 k2e[2] = {k2eL, k2eR};
+  h->launches += launch_channels(tr, ci->k0, ci->k1, k2e, ci->side, sides, conj_mode, ind_zero0, h->stream);
   if ((st = check_launch())) return st;
-  int np[2] = {0, 0};
-  RGF_CUDA_TRY(cudaMemcpyAsync(np, as<int>(h->nprop), sizeof(int) * 2, cudaMemcpyDeviceToHost, h->stream));
+  ci->host.resize(want_host ? lay.host : 2 * sizeof(int));
+  RGF_CUDA_TRY(cudaMemcpyAsync(ci->host.data(), base, ci->host.size(), cudaMemcpyDeviceToHost, h->stream));
   RGF_CUDA_TRY(cudaStreamSynchronize(h->stream));
+  const int* np = reinterpret_cast<const int*>(ci->host.data());
   ci->np[0] = np[0];
   ci->np[1] = ci->same ? np[0] : np[1];
   return RGF_OK;
 }
 
-rgf_status copy_channels_out(rgf_handle h, const Transverse& tr, const ChanInfo& ci, rgf_channels* ch) {
+rgf_status copy_channels_out(const Transverse& tr, const ChanInfo& ci, rgf_channels* ch) {
   if (!ch) return RGF_OK;
   const int64_t N = tr.N;
-  std::vector<double> k0(tr.n0), k1(tr.n1);
-  RGF_CUDA_TRY(cudaMemcpy(k0.data(), h->k0.p, sizeof(double) * tr.n0, cudaMemcpyDeviceToHost));
-  if (tr.dim == 3) RGF_CUDA_TRY(cudaMemcpy(k1.data(), h->k1.p, sizeof(double) * tr.n1, cudaMemcpyDeviceToHost));
+  const ChanLayout lay(tr, ci.same ? 1 : 2);
+  const unsigned char* base = ci.host.data();
+  const double* k0 = reinterpret_cast<const double*>(base + lay.k0);
+  const double* k1 = reinterpret_cast<const double*>(base + lay.k1);
   if (ch->kydx) {
     for (int64_t a = 0; a < N; a++) ch->kydx[a] = (tr.dim == 2) ? k0[a] : k1[a / tr.n0];
   }
@@ -280,25 +296,19 @@ rgf_status copy_channels_out(rgf_handle h, const Transverse& tr, const ChanInfo&
   }
   const int nsides = ci.two_sided ? 2 : 1;
   for (int s = 0; s < nsides; s++) {
-    const SideDev& sd = ci.side[s];
     rgf_cplx* kx = s == 0 ? ch->kxdx_L : ch->kxdx_R;
     rgf_cplx* mu = s == 0 ? ch->sqrt_mu_L : ch->sqrt_mu_R;
     int64_t* ip = s == 0 ? ch->ind_prop_L : ch->ind_prop_R;
     int64_t* ic = s == 0 ? ch->ind_prop_conj_L : ch->ind_prop_conj_R;
     const int64_t np = ci.np[s];
-    if (kx) RGF_CUDA_TRY(cudaMemcpy(kx, sd.kx, sizeof(double2) * N, cudaMemcpyDeviceToHost));
-    std::vector<int> prop(np > 0 ? np : 1), conj(np > 0 ? np : 1);
-    std::vector<double2> muall(N);
-    if (np > 0) RGF_CUDA_TRY(cudaMemcpy(prop.data(), sd.prop, sizeof(int) * np, cudaMemcpyDeviceToHost));
-    if (mu) {
-      RGF_CUDA_TRY(cudaMemcpy(muall.data(), sd.sqrtmu, sizeof(double2) * N, cudaMemcpyDeviceToHost));
-      for (int64_t p = 0; p < np; p++) mu[p] = rgf_cplx{muall[prop[p]].x, muall[prop[p]].y};
-    }
-    if (ip)
-      for (int64_t p = 0; p < np; p++) ip[p] = prop[p];
-    if (ic && ci.has_conj && np > 0) {
-      RGF_CUDA_TRY(cudaMemcpy(conj.data(), sd.conj, sizeof(int) * np, cudaMemcpyDeviceToHost));
-      for (int64_t p = 0; p < np; p++) ic[p] = conj[p];
+    const rgf_cplx* muall = reinterpret_cast<const rgf_cplx*>(base + lay.mu[s]);
+    const int* prop = reinterpret_cast<const int*>(base + lay.prop[s]);
+    const int* conj = reinterpret_cast<const int*>(base + lay.conj[s]);
+    if (kx) memcpy(kx, base + lay.kx[s], sizeof(double2) * N);
+    for (int64_t p = 0; p < np; p++) {
+      if (mu) mu[p] = muall[prop[p]];
+      if (ip) ip[p] = prop[p];
+      if (ic && ci.has_conj) ic[p] = conj[p];
     }
   }
   ch->N_prop_L = ci.np[0];
@@ -426,7 +436,7 @@ rgf_status smatrix_sizes(rgf_handle h, const Problem& p, const rgf_request* req,
   k2eps(p.k0dx, p.epsL, &k2, &k2eL);
   k2eps(p.k0dx, p.epsR, &k2, &k2eR);
   ChanInfo ci;
-  if ((st = run_channels(h, p.tr, k2eL, k2eR, true, &ci))) return st;
+  if ((st = run_channels(h, p.tr, k2eL, k2eR, true, false, &ci))) return st;
   Request r;
   if ((st = resolve_request(req, ci, &r))) return st;
   *n_out = (int64_t)(r.out[0].size() + r.out[1].size());
@@ -1238,7 +1248,7 @@ rgf_status smatrix_run(rgf_handle h, const Problem& p, const rgf_request* req, c
 
   // (1) channels, request resolution (cal_smatrix_RGF.m:98-178)
   ChanInfo ci;
-  if ((st = run_channels(h, tr, k2eL, k2eR, true, &ci))) return st;
+  if ((st = run_channels(h, tr, k2eL, k2eR, true, ch != nullptr, &ci))) return st;
   Request rq;
   if ((st = resolve_request(req, ci, &rq))) return st;
   const int noL = (int)rq.out[0].size(), noR = (int)rq.out[1].size();
@@ -1253,7 +1263,7 @@ rgf_status smatrix_run(rgf_handle h, const Problem& p, const rgf_request* req, c
       if (S_dev) RGF_CUDA_TRY(cudaMemsetAsync(gr->g, 0, sizeof(rgf_cplx) * N * L, h->stream));
       else memset(gr->g, 0, sizeof(rgf_cplx) * N * L);
     }
-    return copy_channels_out(h, tr, ci, ch);
+    return copy_channels_out(tr, ci, ch);
   }
   if (gr && gr->D && gr->ldD < n_out) {
     set_error("ldD must be >= the number of requested output channels");
@@ -1364,7 +1374,7 @@ rgf_status smatrix_run(rgf_handle h, const Problem& p, const rgf_request* req, c
   // (5) transverse profiles, slice stencil, lead surface Green's functions
   //     G0 = phi diag(exp(1i kx)) phi'  (cal_smatrix_RGF.m:187-209)
   double2* phi = as<double2>(h->phi);
-  launch_phi(tr, as<double>(h->k0), as<double>(h->k1), phi, N, h->stream);
+  launch_phi(tr, ci.k0, ci.k1, phi, N, h->stream);
   launch_stencil(tr, as<int>(h->st_col), as<double2>(h->st_val), h->stream);
   h->launches += 2;
   const SideDev& sd_s = ci.side[s];
@@ -1431,7 +1441,7 @@ rgf_status smatrix_run(rgf_handle h, const Problem& p, const rgf_request* req, c
         return RGF_ERR_NONFINITE;
       }
       h->mx_form = RGF_TF32X3;
-      return copy_channels_out(h, tr, ci, ch);
+      return copy_channels_out(tr, ci, ch);
     }
     if (st == RGF_ERR_OOM) {
       // the factor store does not fit: give its buffers back and take the
@@ -1521,7 +1531,7 @@ rgf_status smatrix_run(rgf_handle h, const Problem& p, const rgf_request* req, c
         return RGF_ERR_TIMEOUT;
       }
       if ((hstatus & kStatusSingular) || !(h->probe <= kProbeRetry)) return kRetryUnsplit;
-      return copy_channels_out(h, tr, ci, ch);
+      return copy_channels_out(tr, ci, ch);
     }
   }
 
@@ -1941,7 +1951,7 @@ rgf_status smatrix_run(rgf_handle h, const Problem& p, const rgf_request* req, c
     set_error("a slice matrix is singular (zero pivot under partial pivoting)");
     return RGF_ERR_SINGULAR;
   }
-  if ((st = copy_channels_out(h, tr, ci, ch))) return st;
+  if ((st = copy_channels_out(tr, ci, ch))) return st;
   if (!(h->probe <= kProbeIllcond)) {
     char msg[160];
     snprintf(msg, sizeof(msg),
@@ -2016,7 +2026,7 @@ rgf_status segment_merge(rgf_handle h, const Problem& p, const rgf_request* req,
   k2eps(p.k0dx, p.epsL, &k2, &k2eL);
   k2eps(p.k0dx, p.epsR, &k2, &k2eR);
   ChanInfo ci;
-  if ((st = run_channels(h, p.tr, k2eL, k2eR, true, &ci))) return st;
+  if ((st = run_channels(h, p.tr, k2eL, k2eR, true, false, &ci))) return st;
   Request rq;
   if ((st = resolve_request(req, ci, &rq))) return st;
   const int noL = (int)rq.out[0].size(), noR = (int)rq.out[1].size();
@@ -2222,9 +2232,7 @@ rgf_status rgf_create(int device, rgf_handle* out) {
 rgf_status rgf_destroy(rgf_handle h) {
   if (!h) return RGF_OK;
   cudaSetDevice(h->device);
-  DevBuf* bufs[] = {&h->k0,     &h->k1,     &h->kx[0],     &h->kx[1],     &h->lam[0],  &h->lam[1],
-                    &h->mu[0],  &h->mu[1],  &h->isprop[0], &h->isprop[1], &h->prop[0], &h->prop[1],
-                    &h->conj[0], &h->conj[1], &h->nprop,   &h->status,    &h->phi,     &h->tmp,
+  DevBuf* bufs[] = {&h->chan,    &h->status,    &h->phi,     &h->tmp,
                     &h->g0s,    &h->g0e,    &h->st_col,    &h->st_val,    &h->eps,     &h->aug,
                     &h->pc,     &h->u,      &h->idx,       &h->sdev,      &h->xpc,     &h->xrow,
                     &h->xt,     &h->xu,     &h->xsync,     &h->xprobe,    &h->gepp,    &h->gck,
@@ -2560,8 +2568,8 @@ static rgf_status setup_channels_common(rgf_handle h, const Transverse& tr, rgf_
   k2eps(k0dx, eL, &k2, &k2eL);
   k2eps(k0dx, two_sided ? eR : eL, &k2, &k2eR);
   ChanInfo ci;
-  if ((st = run_channels(h, tr, k2eL, k2eR, two_sided != 0, &ci))) return st;
-  return copy_channels_out(h, tr, ci, ch);
+  if ((st = run_channels(h, tr, k2eL, k2eR, two_sided != 0, ch != nullptr, &ci))) return st;
+  return copy_channels_out(tr, ci, ch);
 }
 
 rgf_status rgf_setup_channels_2d(rgf_handle h, int64_t ny, int32_t bc, double ka, rgf_cplx k0dx,
