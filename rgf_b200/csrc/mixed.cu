@@ -13,7 +13,7 @@
 // right-input ones).  Here:
 //
 // 1. factor: g_k = (H_kk - g_{k-1})^-1 for every slice in FP32 (complex64),
-//    each inverse by block Gauss-Jordan with 64-wide pivot blocks: the pivot
+//    each inverse by block Gauss-Jordan with 32-wide pivot blocks: the pivot
 //    block's inverse T by one CTA (register-resident GJ, diagonal pivots), the
 //    row panel U = T W'(J, :) in FP32, and the rank-64 update
 //    W <- W' - V U on the tensor cores (tcgen05.mma kind::tf32, 3xTF32, TMEM
@@ -470,71 +470,6 @@ __device__ unsigned int g_mx_tl_n[2];
   } while (0)
 #endif
 
-// X = M^-1 for a 16 x 16 complex block by one warp: Gauss-Jordan on diagonal
-// pivots with lane l holding row l/2, columns (l%2) + 2q; the pivot row, the
-// multiplier and the pivot come by shuffles, so no barrier is needed.  A zero
-// or non-finite pivot sets *bad.
-__device__ __forceinline__ void inv16_warp(const float2* M, int ldm, float2* X, int ldx, int lane, int* bad) {
-  const int r = lane >> 1, h = lane & 1;
-  float2 a[8];
-#pragma unroll
-  for (int q = 0; q < 8; q++) a[q] = M[r * ldm + h + 2 * q];
-  bool badl = false;
-#pragma unroll
-  for (int k = 0; k < 16; k++) {
-    float2 rk[8];
-#pragma unroll
-    for (int q = 0; q < 8; q++) {
-      rk[q].x = __shfl_sync(0xffffffffu, a[q].x, 2 * k + h);
-      rk[q].y = __shfl_sync(0xffffffffu, a[q].y, 2 * k + h);
-    }
-    const float2 src = a[k >> 1];
-    float2 f, p;
-    f.x = __shfl_sync(0xffffffffu, src.x, 2 * r + (k & 1));
-    f.y = __shfl_sync(0xffffffffu, src.y, 2 * r + (k & 1));
-    p.x = __shfl_sync(0xffffffffu, src.x, 2 * k + (k & 1));
-    p.y = __shfl_sync(0xffffffffu, src.y, 2 * k + (k & 1));
-    const float d = p.x * p.x + p.y * p.y;
-    float id;  // approximate reciprocal (one instruction): the factor only preconditions the refinement
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(id) : "f"(d));
-    if (!(d > 0.f) || !isfinite(id)) badl = true;
-    const float2 pinv = make_float2(p.x * id, -p.y * id);
-    const bool me = (r == k);
-    const float2 fp = fcmul(f, pinv);
-    const float2 coef = me ? make_float2(-pinv.x, -pinv.y) : fp;
-#pragma unroll
-    for (int q = 0; q < 8; q++) {
-      const float2 u = fcmul(coef, rk[q]);
-      const float2 base = me ? make_float2(0.f, 0.f) : a[q];
-      a[q] = make_float2(base.x - u.x, base.y - u.y);
-    }
-    if (h == (k & 1)) a[k >> 1] = me ? pinv : make_float2(-fp.x, -fp.y);
-  }
-#pragma unroll
-  for (int q = 0; q < 8; q++) X[r * ldx + h + 2 * q] = a[q];
-  if (badl) *bad = 1;
-}
-
-// C (16 x 16) = sign * A B (+ D), row-major with the given leading dimensions;
-// thread t of the block computes element (t / 16, t % 16)
-__device__ __forceinline__ void mm16(const float2* A, int lda_, const float2* B, int ldb, const float2* D, int ldd,
-                                     float sign, float2* C, int ldc, int t) {
-  const int i = t >> 4, j = t & 15;
-  float2 acc = make_float2(0.f, 0.f);
-#pragma unroll
-  for (int s = 0; s < 16; s++) {
-    const float2 u = fcmul(A[i * lda_ + s], B[s * ldb + j]);
-    acc.x += u.x;
-    acc.y += u.y;
-  }
-  float2 v = make_float2(sign * acc.x, sign * acc.y);
-  if (D) {
-    v.x += D[i * ldd + j].x;
-    v.y += D[i * ldd + j].y;
-  }
-  C[i * ldc + j] = v;
-}
-
 // C (32 x 32) = sign * A B (+ D) in shared memory (leading dimension 33) by
 // 256 threads: thread t computes rows i, i + 16 and columns c, c + 16
 // (i = t / 16, c = t % 16)
@@ -574,42 +509,123 @@ __device__ __forceinline__ void mm32(const float2* A, const float2* B, const flo
     }
 }
 
-// T = M^-1 for the identity-padded 32 x 32 pivot block M (shared memory,
-// leading dimension 33) by 2 x 2 blocks of 16 (A, B; C, D): X = A^-1,
-// S = D - C X B, Y = S^-1, T = [[X - X B T21, -X B Y], [-Y C X, Y]]; the two
-// 16 x 16 inverses by warp 0 (shuffles only), the products by all 256
-// threads.  tmp: 5 x 16 x 17 float2 of shared memory.  T is zeroed beyond jn.
-__device__ __forceinline__ void inv32_block(const float2* Mb, float2* Ts, float2* tmp, int jn, int tid, int* bad) {
-  constexpr int LD = NB + 1, L16 = 17;
-  const int warp = tid >> 5, lane = tid & 31;
-  float2* Xs = tmp;
-  float2* P1 = Xs + 16 * L16;
-  float2* P2 = P1 + 16 * L16;
-  float2* Ss = P2 + 16 * L16;
-  float2* Ys = Ss + 16 * L16;
-  if (warp == 0) inv16_warp(Mb, LD, Xs, L16, lane, bad);
-  __syncthreads();
-  mm16(Xs, L16, Mb + 16, LD, nullptr, 0, 1.f, P1, L16, tid);           // P1 = X B
-  mm16(Mb + 16 * LD, LD, Xs, L16, nullptr, 0, 1.f, P2, L16, tid);      // P2 = C X
-  __syncthreads();
-  mm16(Mb + 16 * LD, LD, P1, L16, Mb + 16 * LD + 16, LD, -1.f, Ss, L16, tid);  // S = D - C P1
-  __syncthreads();
-  if (warp == 0) inv16_warp(Ss, L16, Ys, L16, lane, bad);
-  __syncthreads();
-  mm16(P1, L16, Ys, L16, nullptr, 0, -1.f, Ts + 16, LD, tid);            // T12 = -P1 Y
-  mm16(Ys, L16, P2, L16, nullptr, 0, -1.f, Ts + 16 * LD, LD, tid);       // T21 = -Y P2
-  Ts[(16 + (tid >> 4)) * LD + 16 + (tid & 15)] = Ys[(tid >> 4) * L16 + (tid & 15)];  // T22 = Y
-  __syncthreads();
-  mm16(P1, L16, Ts + 16 * LD, LD, Xs, L16, -1.f, Ts, LD, tid);          // T11 = X - P1 T21
-  __syncthreads();
-  if (jn < NB) {
-    const int r = tid >> 3, cq = tid & 7;
+// T = M^-1 for the identity-padded 32 x 32 pivot block, in registers: lane =
+// row, warp w = columns 4w .. 4w + 3 (a[0..3]).  Gauss-Jordan on diagonal
+// pivots in eight panels of four columns: the panel's warp eliminates its
+// four pivots by shuffles alone and leaves its columns (the panel's transform
+// F) in shared memory, the other seven apply F to their four columns as one
+// rank-4 update (rows outside the panel a += F R, rows of the panel a = F R,
+// R = the panel's rows, which each warp keeps for itself).  One barrier per
+// panel; F alternates between two buffers, so the barrier of the next panel
+// also says that the last reader of a buffer is done.  Latency of the pivot
+// chain bounds it: 32 pivots of ~110 clocks and 8 exchanges; 3.3 us in the
+// step at N = 576, against 6.5 us for two 16 x 16 inverses of one warp each
+// with the block products between them.  The loop over
+// panels stays rolled: every launch runs this once on an SM whose instruction
+// cache the tile CTAs have filled, so code is paid by the line.
+// A zero or non-finite pivot sets *bad.
+struct Inv32Sm {
+  float4 F[2][2][32];
+  float4 R[8][4][2];
+};
+__device__ __forceinline__ void inv32_cols(float2 (&a)[4], Inv32Sm* sm, int warp, int lane, int* bad) {
+  bool badl = false;
+#pragma unroll 1
+  for (int p = 0; p < 8; p++) {
+    float4(*F)[32] = sm->F[p & 1];
+    float4 R[4][2];
+    if (warp == p) {
 #pragma unroll
-    for (int q = 0; q < 4; q++) {
-      const int c = cq + 8 * q;
-      if (r >= jn || c >= jn) Ts[r * LD + c] = make_float2(0.f, 0.f);
+      for (int k = 0; k < 4; k++) {
+        const int pl = 4 * p + k;
+        float2 rk[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++) {  // the pivot first: its reciprocal is the chain
+          const int c = (k + i) & 3;
+          rk[c].x = __shfl_sync(0xffffffffu, a[c].x, pl);
+          rk[c].y = __shfl_sync(0xffffffffu, a[c].y, pl);
+        }
+        const float d = rk[k].x * rk[k].x + rk[k].y * rk[k].y;
+        float id;  // approximate reciprocal (one instruction): the factor only preconditions the refinement
+        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(id) : "f"(d));
+        if (!(d > 0.f) || !isfinite(id)) badl = true;
+        const float2 pinv = make_float2(rk[k].x * id, -rk[k].y * id);
+        const bool me = lane == pl;
+        const float2 fp = fcmul(a[k], pinv);
+        const float2 coef = me ? make_float2(-pinv.x, -pinv.y) : fp;
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+          if (c == k) continue;
+          const float2 u = fcmul(coef, rk[c]);
+          const float2 base = me ? make_float2(0.f, 0.f) : a[c];
+          a[c] = make_float2(base.x - u.x, base.y - u.y);
+        }
+        a[k] = me ? pinv : make_float2(-fp.x, -fp.y);
+      }
+      F[0][lane] = make_float4(a[0].x, a[0].y, a[1].x, a[1].y);
+      F[1][lane] = make_float4(a[2].x, a[2].y, a[3].x, a[3].y);
+    } else {
+      if ((lane >> 2) == p) {
+        sm->R[warp][lane & 3][0] = make_float4(a[0].x, a[0].y, a[1].x, a[1].y);
+        sm->R[warp][lane & 3][1] = make_float4(a[2].x, a[2].y, a[3].x, a[3].y);
+      }
+      __syncwarp();
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        R[k][0] = sm->R[warp][k][0];
+        R[k][1] = sm->R[warp][k][1];
+      }
     }
     __syncthreads();
+    if (warp != p) {
+      const float4 f01 = F[0][lane], f23 = F[1][lane];
+      const float2 f[4] = {make_float2(f01.x, f01.y), make_float2(f01.z, f01.w), make_float2(f23.x, f23.y),
+                           make_float2(f23.z, f23.w)};
+      if ((lane >> 2) == p) {
+#pragma unroll
+        for (int c = 0; c < 4; c++) a[c] = make_float2(0.f, 0.f);
+      }
+#pragma unroll
+      for (int c = 0; c < 4; c++) {
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+          const float4 rr = R[k][c >> 1];
+          const float2 b = (c & 1) ? make_float2(rr.z, rr.w) : make_float2(rr.x, rr.y);
+          a[c].x = fmaf(f[k].x, b.x, fmaf(-f[k].y, b.y, a[c].x));
+          a[c].y = fmaf(f[k].x, b.y, fmaf(f[k].y, b.x, a[c].y));
+        }
+      }
+    }
+    __syncwarp();
+  }
+  if (badl) *bad = 1;
+}
+
+// Publish the pivot-block inverse held by inv32_cols' threads (zero beyond
+// jn), as float2 rows (Tout) and as the right operand of the step's U product
+// (U = T W'(J, :), computed on the tensor core as conj(U)^T in realified
+// form): image rows 2t = T(t, :) and 2t + 1 = i T(t, :), K = (re, im) of
+// column m, K-major with the 128-byte swizzle, 2 K-chunks of 64 rows; the tf32
+// hi image, then the lo image.  A thread's columns 2h, 2h + 1 fill one 16-byte
+// granule of an image row.
+__device__ __forceinline__ void publish_tu(float2 (&a)[4], int jn, float2* Tout, uint8_t* img, int warp, int lane) {
+#pragma unroll
+  for (int c = 0; c < 4; c++)
+    if (lane >= jn || 4 * warp + c >= jn) a[c] = make_float2(0.f, 0.f);
+  float4* to = reinterpret_cast<float4*>(Tout + lane * NB + 4 * warp);
+#pragma unroll
+  for (int h = 0; h < 2; h++) {
+    const float2 u = a[2 * h], v = a[2 * h + 1];
+    to[h] = make_float4(u.x, u.y, v.x, v.y);
+#pragma unroll
+    for (int rr = 0; rr < 2; rr++) {
+      const int n = 2 * lane + rr, gq = 2 * (warp & 3) + h;
+      const float4 x = rr ? make_float4(-u.y, u.x, -v.y, v.x) : make_float4(u.x, u.y, v.x, v.y);
+      const float4 hi = make_float4(tf32_hi(x.x), tf32_hi(x.y), tf32_hi(x.z), tf32_hi(x.w));
+      uint8_t* dst = img + (warp >> 2) * gjs::TU_CH + n * 128 + ((gq ^ (n & 7)) << 4);
+      *reinterpret_cast<float4*>(dst) = hi;
+      *reinterpret_cast<float4*>(dst + gjs::TU_HALF) = make_float4(x.x - hi.x, x.y - hi.y, x.z - hi.z, x.w - hi.w);
+    }
   }
 }
 
@@ -618,29 +634,6 @@ __device__ __forceinline__ void inv32_block(const float2* Mb, float2* Ts, float2
 // J' = [j1, j1 + jn1) and, at the last step of a slice, the next slice's
 // stencil, permittivity and right-lead block (its first pivot block is then
 // A_{n+1}(J', J') - g_n(J', J') [- G0_R(J', J')])
-// The pivot-block inverse T as the right operand of the step's U product
-// (U = T W'(J, :), computed on the tensor core as conj(U)^T in realified
-// form): image rows 2t = T(t, :) and 2t + 1 = i T(t, :), K = (re, im) of
-// column m, K-major with the 128-byte swizzle, 2 K-chunks of 64 rows; the tf32
-// hi image, then the lo image.  Ts: T in shared memory, row pitch ldt.
-__device__ __forceinline__ void publish_tu(const float2* Ts, int ldt, uint8_t* img, int tid) {
-  const int r = tid >> 3, cq = tid & 7;
-#pragma unroll
-  for (int q = 0; q < 4; q++) {
-    const int m = cq + 8 * q, kf = 2 * m, kc = kf >> 5, gq = (kf & 31) >> 2, ofs = (kf & 3) * 4;
-    const float2 t = Ts[r * ldt + m];
-#pragma unroll
-    for (int rr = 0; rr < 2; rr++) {
-      const int n = 2 * r + rr;
-      const float x0 = rr ? -t.y : t.x, x1 = rr ? t.x : t.y;
-      const uint32_t off = kc * gjs::TU_CH + n * 128 + ((gq ^ (n & 7)) << 4) + ofs;
-      const float h0 = tf32_hi(x0), h1 = tf32_hi(x1);
-      *reinterpret_cast<float2*>(img + off) = make_float2(h0, h1);
-      *reinterpret_cast<float2*>(img + gjs::TU_HALF + off) = make_float2(x0 - h0, x1 - h1);
-    }
-  }
-}
-
 struct GjNext {
   const float2* Tin;
   float2* Tout;
@@ -679,15 +672,14 @@ struct GjNext {
 __device__ void t_server(const float* __restrict__ Wsrc, int64_t lda, int j0, int jn, const GjNext& ns,
                          uint8_t* gb, int* bad) {
   constexpr int LD = NB + 1;
-  const int tid = threadIdx.x, r = tid >> 3, cq = tid & 7;
+  const int tid = threadIdx.x, r = tid >> 3, cq = tid & 7, warp = tid >> 5, lane = tid & 31;
   float2* Tj = reinterpret_cast<float2*>(gb);
   float2* B1 = Tj + NB * LD;  // W(J, J')
   float2* B2 = B1 + NB * LD;  // W(J', J)
   float2* B3 = B2 + NB * LD;  // W(J', J')
   float2* U1 = B3 + NB * LD;
   float2* Mn = U1 + NB * LD;
-  float2* To = Mn + NB * LD;
-  float2* tmp = To + NB * LD;
+  Inv32Sm* ism = reinterpret_cast<Inv32Sm*>(gb + 8 * NB * LD * sizeof(float2));
   const int j1 = ns.j1, jn1 = ns.jn1;
 #pragma unroll
   for (int q = 0; q < 4; q++) {
@@ -710,14 +702,15 @@ __device__ void t_server(const float* __restrict__ Wsrc, int64_t lda, int j0, in
     for (int q = 0; q < 4; q++) Mn[r * LD + cq + 8 * q] = Tj[r * LD + cq + 8 * q];
   }
   __syncthreads();
+  float2 m[4];  // lane = row, warp = four columns
 #pragma unroll
   for (int q = 0; q < 4; q++) {
-    const int c = cq + 8 * q;
-    float2 v = Mn[r * LD + c];
-    if (r < jn1 && c < jn1) {
+    const int c = 4 * warp + q;
+    float2 v = Mn[lane * LD + c];
+    if (lane < jn1 && c < jn1) {
       if (ns.next_slice) {  // A_{n+1}(J', J') - g_n(J', J') [- G0_R(J', J')]
         double2 a = cmk(-(double)v.x, -(double)v.y);
-        const int gi = j1 + r, gc = j1 + c;
+        const int gi = j1 + lane, gc = j1 + c;
 #pragma unroll
         for (int qq = 0; qq < kMaxStencil; qq++)
           if (ns.st_col[gi * kMaxStencil + qq] == gc) a = cadd(a, ns.st_val[gi * kMaxStencil + qq]);
@@ -726,17 +719,14 @@ __device__ void t_server(const float* __restrict__ Wsrc, int64_t lda, int j0, in
         v = make_float2((float)a.x, (float)a.y);
       }
     } else {
-      v = make_float2(r == c ? 1.f : 0.f, 0.f);
+      v = make_float2(lane == c ? 1.f : 0.f, 0.f);
     }
-    Mn[r * LD + c] = v;
+    m[q] = v;
   }
-  __syncthreads();
   MX_PSTAMP(4);
-  inv32_block(Mn, To, tmp, jn1, tid, bad);
+  inv32_cols(m, ism, warp, lane, bad);
   MX_PSTAMP(5);
-#pragma unroll
-  for (int q = 0; q < 4; q++) ns.Tout[r * NB + cq + 8 * q] = To[r * LD + cq + 8 * q];
-  publish_tu(To, LD, ns.tu_out, tid);
+  publish_tu(m, jn1, ns.Tout, ns.tu_out, warp, lane);
 }
 
 __global__ void __launch_bounds__(256, 1)
@@ -989,24 +979,21 @@ __global__ void __launch_bounds__(256) k_mx_t0(const float* __restrict__ W, int6
                                                uint8_t* tu_out, int* status) {
   pdl_open();
   pdl_wait();
-  constexpr int LD = NB + 1;
-  __shared__ float2 Mb[NB * LD];
-  __shared__ float2 To[NB * LD];
-  __shared__ float2 tmp[5 * 16 * 17];
+  __shared__ Inv32Sm ism;
   __shared__ int bad;
-  const int tid = threadIdx.x, r = tid >> 3, cq = tid & 7;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  float2 m[4];
 #pragma unroll
   for (int q = 0; q < 4; q++) {
-    const int c = cq + 8 * q;
-    Mb[r * LD + c] = (r < jn && c < jn) ? *reinterpret_cast<const float2*>(W + (int64_t)r * lda + 2 * c)
-                                        : make_float2(r == c ? 1.f : 0.f, 0.f);
+    const int c = 4 * warp + q;
+    m[q] = (lane < jn && c < jn) ? *reinterpret_cast<const float2*>(W + (int64_t)lane * lda + 2 * c)
+                                 : make_float2(lane == c ? 1.f : 0.f, 0.f);
   }
   if (tid == 0) bad = 0;
   __syncthreads();
-  inv32_block(Mb, To, tmp, jn, tid, &bad);
-#pragma unroll
-  for (int q = 0; q < 4; q++) Tout[r * NB + cq + 8 * q] = To[r * LD + cq + 8 * q];
-  publish_tu(To, LD, tu_out, tid);
+  inv32_cols(m, &ism, warp, lane, &bad);
+  publish_tu(m, jn, Tout, tu_out, warp, lane);
+  __syncthreads();
   if (bad && tid == 0) atomicOr(status, kStatusSingular);
 }
 
