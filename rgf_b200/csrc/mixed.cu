@@ -470,43 +470,27 @@ __device__ unsigned int g_mx_tl_n[2];
   } while (0)
 #endif
 
-// C (32 x 32) = sign * A B (+ D) in shared memory (leading dimension 33) by
-// 256 threads: thread t computes rows i, i + 16 and columns c, c + 16
-// (i = t / 16, c = t % 16)
-__device__ __forceinline__ void mm32(const float2* A, const float2* B, const float2* D, float sign, float2* C,
-                                     int t) {
-  constexpr int LD = NB + 1;
-  const int i = t >> 4, c = t & 15;
-  float2 acc[2][2];
-#pragma unroll
-  for (int u = 0; u < 2; u++)
-#pragma unroll
-    for (int v = 0; v < 2; v++) acc[u][v] = make_float2(0.f, 0.f);
+// c (+)= sign * A B for one warp's part of a 32 x 32 product: lane = row of A
+// (shared memory, row pitch NB + 1), four columns of B (row pitch ldb, 16-byte
+// rows of four read by all lanes at once).  A warp needs only its own columns
+// of B, so a chain of such products passes no block barrier.
+__device__ __forceinline__ void mm_cols(const float2* A, const float2* B, int ldb, float sign, float2 (&c)[4],
+                                        int lane) {
 #pragma unroll 8
   for (int s = 0; s < NB; s++) {
-    const float2 a0 = A[i * LD + s], a1 = A[(i + 16) * LD + s];
-    const float2 b0 = B[s * LD + c], b1 = B[s * LD + c + 16];
+    float2 a = A[lane * (NB + 1) + s];
+    a.x *= sign;
+    a.y *= sign;
+    const float4 b01 = *reinterpret_cast<const float4*>(B + s * ldb);
+    const float4 b23 = *reinterpret_cast<const float4*>(B + s * ldb + 2);
+    const float2 b[4] = {make_float2(b01.x, b01.y), make_float2(b01.z, b01.w), make_float2(b23.x, b23.y),
+                         make_float2(b23.z, b23.w)};
 #pragma unroll
-    for (int u = 0; u < 2; u++)
-#pragma unroll
-      for (int v = 0; v < 2; v++) {
-        const float2 av = u ? a1 : a0, bv = v ? b1 : b0;
-        acc[u][v].x = fmaf(av.x, bv.x, fmaf(-av.y, bv.y, acc[u][v].x));
-        acc[u][v].y = fmaf(av.x, bv.y, fmaf(av.y, bv.x, acc[u][v].y));
-      }
-  }
-#pragma unroll
-  for (int u = 0; u < 2; u++)
-#pragma unroll
-    for (int v = 0; v < 2; v++) {
-      const int o = (i + 16 * u) * LD + c + 16 * v;
-      float2 w = make_float2(sign * acc[u][v].x, sign * acc[u][v].y);
-      if (D) {
-        w.x += D[o].x;
-        w.y += D[o].y;
-      }
-      C[o] = w;
+    for (int q = 0; q < 4; q++) {
+      c[q].x = fmaf(a.x, b[q].x, fmaf(-a.y, b[q].y, c[q].x));
+      c[q].y = fmaf(a.x, b[q].y, fmaf(a.y, b[q].x, c[q].y));
     }
+  }
 }
 
 // T = M^-1 for the identity-padded 32 x 32 pivot block, in registers: lane =
@@ -607,25 +591,40 @@ __device__ __forceinline__ void inv32_cols(float2 (&a)[4], Inv32Sm* sm, int warp
 // form): image rows 2t = T(t, :) and 2t + 1 = i T(t, :), K = (re, im) of
 // column m, K-major with the 128-byte swizzle, 2 K-chunks of 64 rows; the tf32
 // hi image, then the lo image.  A thread's columns 2h, 2h + 1 fill one 16-byte
-// granule of an image row.
-__device__ __forceinline__ void publish_tu(float2 (&a)[4], int jn, float2* Tout, uint8_t* img, int warp, int lane) {
+// granule of an image row; the lanes' granules lie in 32 different lines, so
+// both go through shared memory (stage: TU_BYTES + 8 KB) and leave in whole
+// lines (1.25 us in the step, 1.7 us with scattered stores).
+__device__ __forceinline__ void publish_tu(float2 (&a)[4], int jn, float2* Tout, uint8_t* img, uint8_t* stage,
+                                           int warp, int lane) {
 #pragma unroll
   for (int c = 0; c < 4; c++)
     if (lane >= jn || 4 * warp + c >= jn) a[c] = make_float2(0.f, 0.f);
-  float4* to = reinterpret_cast<float4*>(Tout + lane * NB + 4 * warp);
 #pragma unroll
   for (int h = 0; h < 2; h++) {
     const float2 u = a[2 * h], v = a[2 * h + 1];
-    to[h] = make_float4(u.x, u.y, v.x, v.y);
+    const int g = 2 * warp + h;  // granule of the row, swizzled like the image's
+    *reinterpret_cast<float4*>(stage + gjs::TU_BYTES + lane * 256 + ((g ^ (lane & 7)) << 4)) =
+        make_float4(u.x, u.y, v.x, v.y);
 #pragma unroll
     for (int rr = 0; rr < 2; rr++) {
-      const int n = 2 * lane + rr, gq = 2 * (warp & 3) + h;
+      const int n = 2 * lane + rr;
       const float4 x = rr ? make_float4(-u.y, u.x, -v.y, v.x) : make_float4(u.x, u.y, v.x, v.y);
       const float4 hi = make_float4(tf32_hi(x.x), tf32_hi(x.y), tf32_hi(x.z), tf32_hi(x.w));
-      uint8_t* dst = img + (warp >> 2) * gjs::TU_CH + n * 128 + ((gq ^ (n & 7)) << 4);
+      uint8_t* dst = stage + (warp >> 2) * gjs::TU_CH + n * 128 + (((g & 7) ^ (n & 7)) << 4);
       *reinterpret_cast<float4*>(dst) = hi;
       *reinterpret_cast<float4*>(dst + gjs::TU_HALF) = make_float4(x.x - hi.x, x.y - hi.y, x.z - hi.z, x.w - hi.w);
     }
+  }
+  __syncthreads();
+  const int tid = 32 * warp + lane;
+  const float4* s4 = reinterpret_cast<const float4*>(stage);
+#pragma unroll
+  for (int q = 0; q < (int)(gjs::TU_BYTES / 16 / 256); q++)
+    reinterpret_cast<float4*>(img)[tid + 256 * q] = s4[tid + 256 * q];
+#pragma unroll
+  for (int q = 0; q < NB * NB / 2 / 256; q++) {
+    const int o = tid + 256 * q;
+    reinterpret_cast<float4*>(Tout)[o] = s4[gjs::TU_BYTES / 16 + (o & ~15) + ((o & 15) ^ ((o >> 4) & 7))];
   }
 }
 
@@ -671,42 +670,47 @@ struct GjNext {
 #endif
 __device__ void t_server(const float* __restrict__ Wsrc, int64_t lda, int j0, int jn, const GjNext& ns,
                          uint8_t* gb, int* bad) {
-  constexpr int LD = NB + 1;
+  constexpr int LD = NB + 1, LDB = 40;  // LDB: rows of 16-byte granules
   const int tid = threadIdx.x, r = tid >> 3, cq = tid & 7, warp = tid >> 5, lane = tid & 31;
-  float2* Tj = reinterpret_cast<float2*>(gb);
-  float2* B1 = Tj + NB * LD;  // W(J, J')
-  float2* B2 = B1 + NB * LD;  // W(J', J)
-  float2* B3 = B2 + NB * LD;  // W(J', J')
-  float2* U1 = B3 + NB * LD;
-  float2* Mn = U1 + NB * LD;
-  Inv32Sm* ism = reinterpret_cast<Inv32Sm*>(gb + 8 * NB * LD * sizeof(float2));
+  float2* B1 = reinterpret_cast<float2*>(gb);  // W(J, J')
+  float2* Us = B1 + NB * LDB;                  // T W(J, J'): [warp][row][4 columns]
+  Inv32Sm* ism = reinterpret_cast<Inv32Sm*>(Us + NB * NB);
+  uint8_t* stage = reinterpret_cast<uint8_t*>(ism + 1);
+  float2* Tj = reinterpret_cast<float2*>(stage + gjs::TU_BYTES + NB * NB * sizeof(float2));
+  float2* B2 = Tj + NB * LD;                   // W(J', J)
+  float2* B3 = B2 + NB * LD;                   // W(J', J')
   const int j1 = ns.j1, jn1 = ns.jn1;
 #pragma unroll
   for (int q = 0; q < 4; q++) {
     const int c = cq + 8 * q;
     Tj[r * LD + c] = ns.Tin[r * NB + c];
     const float2 z = make_float2(0.f, 0.f);
-    B1[r * LD + c] = (r < jn && c < jn1) ? *reinterpret_cast<const float2*>(Wsrc + (int64_t)(j0 + r) * lda + 2 * (j1 + c)) : z;
+    B1[r * LDB + c] = (r < jn && c < jn1) ? *reinterpret_cast<const float2*>(Wsrc + (int64_t)(j0 + r) * lda + 2 * (j1 + c)) : z;
     B2[r * LD + c] = (r < jn1 && c < jn) ? *reinterpret_cast<const float2*>(Wsrc + (int64_t)(j1 + r) * lda + 2 * (j0 + c)) : z;
     B3[r * LD + c] = (r < jn1 && c < jn1) ? *reinterpret_cast<const float2*>(Wsrc + (int64_t)(j1 + r) * lda + 2 * (j1 + c)) : z;
   }
   __syncthreads();
   MX_PSTAMP(2);
+  float2 m[4];  // lane = row, warp = four columns
   if (!ns.same_block) {
-    mm32(Tj, B1, nullptr, 1.f, U1, tid);  // U1 = T W(J, J')
-    __syncthreads();
+    float2 u[4] = {};
+    mm_cols(Tj, B1 + 4 * warp, LDB, 1.f, u, lane);  // U1 = T W(J, J')
+    float2* Uw = Us + warp * (4 * NB);
+    *reinterpret_cast<float4*>(Uw + 4 * lane) = make_float4(u[0].x, u[0].y, u[1].x, u[1].y);
+    *reinterpret_cast<float4*>(Uw + 4 * lane + 2) = make_float4(u[2].x, u[2].y, u[3].x, u[3].y);
+#pragma unroll
+    for (int q = 0; q < 4; q++) m[q] = B3[lane * LD + 4 * warp + q];
+    __syncwarp();
     MX_PSTAMP(3);
-    mm32(B2, U1, B3, -1.f, Mn, tid);      // W(J', J') - W(J', J) U1
+    mm_cols(B2, Uw, 4, -1.f, m, lane);  // W(J', J') - W(J', J) U1
   } else {
 #pragma unroll
-    for (int q = 0; q < 4; q++) Mn[r * LD + cq + 8 * q] = Tj[r * LD + cq + 8 * q];
+    for (int q = 0; q < 4; q++) m[q] = Tj[lane * LD + 4 * warp + q];
   }
-  __syncthreads();
-  float2 m[4];  // lane = row, warp = four columns
 #pragma unroll
   for (int q = 0; q < 4; q++) {
     const int c = 4 * warp + q;
-    float2 v = Mn[lane * LD + c];
+    float2 v = m[q];
     if (lane < jn1 && c < jn1) {
       if (ns.next_slice) {  // A_{n+1}(J', J') - g_n(J', J') [- G0_R(J', J')]
         double2 a = cmk(-(double)v.x, -(double)v.y);
@@ -726,7 +730,7 @@ __device__ void t_server(const float* __restrict__ Wsrc, int64_t lda, int j0, in
   MX_PSTAMP(4);
   inv32_cols(m, ism, warp, lane, bad);
   MX_PSTAMP(5);
-  publish_tu(m, jn1, ns.Tout, ns.tu_out, warp, lane);
+  publish_tu(m, jn1, ns.Tout, ns.tu_out, stage, warp, lane);
 }
 
 __global__ void __launch_bounds__(256, 1)
@@ -980,6 +984,7 @@ __global__ void __launch_bounds__(256) k_mx_t0(const float* __restrict__ W, int6
   pdl_open();
   pdl_wait();
   __shared__ Inv32Sm ism;
+  __shared__ __align__(16) uint8_t stage[gjs::TU_BYTES + NB * NB * sizeof(float2)];
   __shared__ int bad;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   float2 m[4];
@@ -992,7 +997,7 @@ __global__ void __launch_bounds__(256) k_mx_t0(const float* __restrict__ W, int6
   if (tid == 0) bad = 0;
   __syncthreads();
   inv32_cols(m, &ism, warp, lane, &bad);
-  publish_tu(m, jn, Tout, tu_out, warp, lane);
+  publish_tu(m, jn, Tout, tu_out, stage, warp, lane);
   __syncthreads();
   if (bad && tid == 0) atomicOr(status, kStatusSingular);
 }
