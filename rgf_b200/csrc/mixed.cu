@@ -79,22 +79,42 @@ __device__ __forceinline__ float2 fcmul(float2 a, float2 b) {
 __device__ __forceinline__ void pdl_open() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+__device__ __forceinline__ bool wait_bar(uint32_t bar, uint32_t parity, int* status, long long timeout) {
+  if (tc32::mbar_try(bar, parity)) return true;
+  const long long t0 = clock64();
+  while (!tc32::mbar_try(bar, parity)) {
+    if (clock64() - t0 > timeout) {
+      atomicOr(status, kStatusTimeout);
+      return false;
+    }
+  }
+  return true;
+}
+
 // launch with programmatic stream serialization (every kernel launched this
 // way waits for its predecessor with pdl_wait before it reads or writes)
 template <typename... KArgs, typename... Args>
-cudaError_t launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
-                       Args&&... args) {
+cudaError_t launch_pdl_cluster(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, int cluster_z,
+                               cudaStream_t s, Args&&... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[0].val.programmaticStreamSerializationAllowed = 1;
+  at[1].id = cudaLaunchAttributeClusterDimension;
+  at[1].val.clusterDim.x = at[1].val.clusterDim.y = 1;
+  at[1].val.clusterDim.z = (unsigned)cluster_z;
   cfg.attrs = at;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = cluster_z > 0 ? 2 : 1;
   return cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...);
+}
+template <typename... KArgs, typename... Args>
+cudaError_t launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
+                       Args&&... args) {
+  return launch_pdl_cluster(kern, grid, block, smem, 0, s, std::forward<Args>(args)...);
 }
 
 // ---------------------------------------------------------------------------
@@ -139,20 +159,9 @@ __global__ void k_mx_assemble(float2* W, int64_t ldw, int64_t N, float* st_hi, f
 
 // ---------------------------------------------------------------------------
 // refinement kernels.  Vectors are N x P row-major per slice (site, column):
-// x (FP64, L slices), y (FP32, L slices), the GEMM partials (ksplit x N x P
-// FP32 complex), and the GEMM's right operand Bt (2P rows x lda, K = 2i, 2i+1).
-// One block = 32 columns x 32 sites, threads (32, 8).
+// x (FP64, L slices), y (FP32, L slices), and the solve's right operand Bt (2P
+// rows x lda, K = 2i, 2i+1; two buffers per side).
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ float2 sum_parts(const float2* part, int ksplit, int64_t stride, int64_t ip) {
-  float2 s = make_float2(0.f, 0.f);
-  for (int z = 0; z < ksplit; z++) {
-    const float2 v = part[z * stride + ip];
-    s.x += v.x;
-    s.y += v.y;
-  }
-  return s;
-}
-
 // write the transposed tile (tile[p][i]) as rows 2p, 2p+1 of Bt
 __device__ __forceinline__ void store_bt(float2 (&tile)[32][33], int64_t p0, int64_t i0, int64_t N, int64_t P,
                                          float* bt_hi, float* bt_lo, int64_t lda) {
@@ -207,41 +216,29 @@ __global__ void __launch_bounds__(256) k_mx_residual(int64_t L, int64_t N, int64
   }
 }
 
-// forward pass, slice k: y_kprev = (GEMM partials) -> ystore[kprev] (over its
-// r; kprev = k -+ 1 by the sweep's direction, < 0 at the sweep's first slice);
-// v_k = r_k + y_kprev (+ y_kprev2 from part2 at the junction slice) -> Bt.
-__global__ void __launch_bounds__(256) k_mx_fwd_prep(int64_t k, int64_t kprev, int64_t N, int64_t P, int64_t ldp,
-                                                     int64_t poff, float2* ystore, const float2* part, int ksplit,
-                                                     const float2* part2, int64_t kprev2, int ksplit2, float* bt_hi,
-                                                     float* bt_lo, int64_t lda, const int* kdev) {
+// right operand of a sweep's first solve and of the junction's: v = r (+ ya)
+// (+ yb) -> Bt.  One block = 32 columns x 32 sites, threads (32, 8).
+__global__ void __launch_bounds__(256) k_mx_rhs(int64_t N, int64_t P, const float2* r, const float2* ya,
+                                                const float2* yb, float* bt_hi, float* bt_lo, int64_t lda) {
   pdl_open();
   pdl_wait();
-  if (kdev) {  // slice index kept on the device (graph-captured sweeps)
-    k += *kdev;
-    kprev += *kdev;
-  }
   __shared__ float2 tile[32][33];
-  const int64_t p0 = blockIdx.x * 32, i0 = blockIdx.y * 32, NP = N * ldp;
+  const int64_t p0 = blockIdx.x * 32, i0 = blockIdx.y * 32;
   const int64_t p = p0 + threadIdx.x;
 #pragma unroll
   for (int u = 0; u < 4; u++) {
     const int q = threadIdx.y + 8 * u;
-    const int64_t i = i0 + q;
+    const int64_t i = i0 + q, ip = i * P + p;
     float2 v = make_float2(0.f, 0.f);
     if (i < N && p < P) {
-      const int64_t ip = i * ldp + poff + p;
-      v = ystore[k * NP + ip];  // r_k
-      if (kprev >= 0) {  // y of the neighbour slice swept before (over its r)
-        const float2 yp = sum_parts(part, ksplit, N * P, i * P + p);
-        ystore[kprev * NP + ip] = yp;
-        v.x += yp.x;
-        v.y += yp.y;
+      v = r[ip];
+      if (ya) {
+        v.x += ya[ip].x;
+        v.y += ya[ip].y;
       }
-      if (part2) {  // junction slice: the other side's neighbour too
-        const float2 yq = sum_parts(part2, ksplit2, N * P, i * P + p);
-        ystore[kprev2 * NP + ip] = yq;
-        v.x += yq.x;
-        v.y += yq.y;
+      if (yb) {
+        v.x += yb[ip].x;
+        v.y += yb[ip].y;
       }
     }
     tile[threadIdx.x][q] = v;
@@ -250,75 +247,263 @@ __global__ void __launch_bounds__(256) k_mx_fwd_prep(int64_t k, int64_t kprev, i
   store_bt(tile, p0, i0, N, P, bt_hi, bt_lo, lda);
 }
 
-// backward pass, slice k: d_k = (GEMM partials) + y_k (add_y; without it the
-// partials are d_k itself: the sweep's first slice); x_k += d_k in FP64; norms
-// of d and x (whole; slice 0; slice L-1); d_k -> Bt (write_bt) and -> Bt2 (the
-// junction slice feeds both sides).  add_y, write_bt < 0: the one-sided rule.
-__global__ void __launch_bounds__(256) k_mx_bwd_prep(int64_t k, int64_t L, int64_t N, int64_t P, int64_t ldp,
-                                                     int64_t poff, double2* x,
-                                                     const float2* ystore, const float2* part, int ksplit,
-                                                     float* bt_hi, float* bt_lo, int64_t lda, double* norms,
-                                                     const int* kdev, int add_y, int write_bt, float* bt2_hi,
-                                                     float* bt2_lo) {
+// One step of the substitution sweeps on both sides at once: D = g_k Bt by
+// 3xTF32 on tcgen05 and everything that follows from it,
+//   forward   y_k = D (over r_k), v = r_next + y_k -> Bt of the next step;
+//   backward  d_k = D (+ y_k), x_k += d_k in FP64, norms of d and x (whole;
+//             slice 0; slice L-1), d_k -> Bt (and Bt2: the junction slice
+//             feeds both sides).
+// A sweep is a chain of these, so its time is the latency of one.  The CTAs
+// of a tile's K-split form a cluster (1, 1, Z): each leaves its accumulator in
+// its shared memory and all of them add up and finish equal shares of the
+// tile over distributed shared memory.  A step is then one launch for both
+// sides; with the partial sums in global memory it was a GEMM and a second
+// kernel per side.
+// Bt is double-buffered: tiles of this step still read the buffer of the step
+// before.  A (the factor store) does not depend on the step before, so its
+// first stages, and y and x into L2, are fetched ahead of griddepcontrol.wait;
+// y and x themselves while the products run.
+// Measured, a step of a sweep (64 / 300 / 512 / 576 / 1024 wide, with 12 / 60 /
+// 102 / 18 / 204 columns): 6.7 / 12.1 / 14.7 / 10.3 / 32 us, against 8.8 / 22 /
+// 21 / 19 / 38 us for the two kernels.  Wide requests are bound by the operands'
+// way into and out of shared memory (0.8 us per 128 x 128 x 32 chunk).
+struct SolveSide {
+  int active;           // 0: this side has no step in this launch
+  int k;                // slice
+  const float2* rnext;  // forward: r of the side's next slice (null: last)
+  float2* y;            // forward: y_k (out); backward: y_k to add (null: none)
+  double2* x;           // backward: x_k
+  float *bt_hi, *bt_lo, *bt2_hi, *bt2_lo;  // right operands to write (null: none)
+  int ends;             // backward: bit 0: slice 0, bit 1: slice L-1
+};
+struct SolveArgs {
+  SolveSide sd[2];
+  int64_t N, P, lda;
+  int k_chunks;         // BK-chunks of K, shared out over the cluster
+  int tiles;            // column tiles per side
+  int fwd;
+  double* norms;
+  int* status;
+  long long timeout;
+};
+struct SolveMaps {
+  CUtensorMap a_hi, a_lo, b_hi[2], b_lo[2];
+};
+
+// lanes: 8 sites x 4 columns, so that the 8 sites of a row of Bt fill 64 bytes
+// and the 4 columns of a row of y 32 bytes
+constexpr int kSolveWarps = 16;
+template <int BN>
+__global__ void __launch_bounds__(kSolveWarps * 32, 1)
+    k_mx_solve(const __grid_constant__ SolveMaps maps, const __grid_constant__ SolveArgs g) {
+  using C = tc32::Cfg<BN>;
+  constexpr int S = C::STAGES;
+  constexpr int TP = BN + 8;   // pitch of the accumulator tile: 8 sites x 4 columns conflict-free
+  constexpr int PQ = BN / 8;   // groups of four columns per tile row
+  constexpr int ITEMS = 16 * PQ, U = 8, W = kSolveWarps;
+  static_assert(tc32::BM * TP * 4 <= S * (int)C::STAGE_BYTES, "accumulator tile");
+  extern __shared__ uint8_t smem_raw[];
+  __shared__ __align__(8) uint64_t full_bar[S];
+  __shared__ __align__(8) uint64_t empty_bar[S];
+  __shared__ __align__(8) uint64_t done_bar;
+  __shared__ uint32_t tmem_sh;
+  __shared__ double red[2][kSolveWarps];
   pdl_open();
-  pdl_wait();
-  if (kdev) k += *kdev;  // slice index kept on the device (graph-captured sweeps)
-  if (add_y < 0) add_y = k < L - 1;   // one-sided sweep: y_k enters except at the first slice
-  if (write_bt < 0) write_bt = k > 0;  // ... and the next GEMM needs d_k except after slice 0
-  __shared__ float2 tile[32][33];
-  __shared__ double red[2][8];
-  const int64_t p0 = blockIdx.x * 32, i0 = blockIdx.y * 32, NP = N * ldp;
-  const int64_t p = p0 + threadIdx.x;
-  double dd = 0.0, xx = 0.0;
-#pragma unroll
-  for (int u = 0; u < 4; u++) {
-    const int q = threadIdx.y + 8 * u;
-    const int64_t i = i0 + q;
-    float2 d = make_float2(0.f, 0.f);
-    if (i < N && p < P) {
-      const int64_t ip = i * ldp + poff + p;
-      d = sum_parts(part, ksplit, N * P, i * P + p);
-      if (add_y) {
-        const float2 y = ystore[k * NP + ip];
-        d.x += y.x;
-        d.y += y.y;
-      }
-      double2* xp = x + k * NP + ip;
-      const double2 xn = cmk(xp->x + (double)d.x, xp->y + (double)d.y);
-      *xp = xn;
-      dd += (double)d.x * d.x + (double)d.y * d.y;
-      xx += xn.x * xn.x + xn.y * xn.y;
+  const int side = blockIdx.x / g.tiles;
+  const SolveSide& sd = g.sd[side];
+  if (!sd.active) return;  // the whole cluster
+  const uint32_t base = (tc32::su32(smem_raw) + 1023u) & ~1023u;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int m0 = blockIdx.y * tc32::BM, n0 = (blockIdx.x - side * g.tiles) * BN;
+  const int z = blockIdx.z, Z = gridDim.z;
+  const int kc0 = z * g.k_chunks / Z, nk = (z + 1) * g.k_chunks / Z - kc0;
+  auto sA = [&](int st) { return base + (uint32_t)st * C::STAGE_BYTES; };
+  auto load_a = [&](int kt) {
+    const int st = kt % S;
+    const uint32_t fb = tc32::su32(&full_bar[st]);
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(fb), "r"(C::STAGE_BYTES) : "memory");
+    tc32::tma_load_3d(sA(st), &maps.a_hi, (kc0 + kt) * tc32::BK, m0, sd.k, fb);
+    tc32::tma_load_3d(sA(st) + C::A_BYTES, &maps.a_lo, (kc0 + kt) * tc32::BK, m0, sd.k, fb);
+  };
+  auto load_b = [&](int kt) {
+    const int st = kt % S;
+    const uint32_t fb = tc32::su32(&full_bar[st]);
+    tc32::tma_load_3d(sA(st) + 2 * C::A_BYTES, &maps.b_hi[side], (kc0 + kt) * tc32::BK, n0, 0, fb);
+    tc32::tma_load_3d(sA(st) + 2 * C::A_BYTES + C::B_BYTES, &maps.b_lo[side], (kc0 + kt) * tc32::BK, n0, 0, fb);
+  };
+  if (tid == 0) {
+    for (int st = 0; st < S; st++) {
+      tc32::mbar_init(tc32::su32(&full_bar[st]), 1);
+      tc32::mbar_init(tc32::su32(&empty_bar[st]), 1);
     }
-    tile[threadIdx.x][q] = d;
+    tc32::mbar_init(tc32::su32(&done_bar), 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    for (int kt = 0; kt < nk && kt < S; kt++) load_a(kt);
   }
-  for (int o = 16; o > 0; o >>= 1) {
-    dd += __shfl_xor_sync(0xffffffffu, dd, o);
-    xx += __shfl_xor_sync(0xffffffffu, xx, o);
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tc32::su32(&tmem_sh)),
+                 "r"(2 * C::TMEM_COLS)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
-  if (threadIdx.x == 0) {
-    red[0][threadIdx.y] = dd;
-    red[1][threadIdx.y] = xx;
+  // this thread's element of item t of the tile (a group of 8 sites x 4 columns)
+  auto site = [&](int t) { return (t / PQ) * 8 + (lane & 7); };
+  auto col = [&](int t) { return (t % PQ) * 4 + (lane >> 3); };
+  for (int t = z * W + warp; t < ITEMS; t += W * Z) {
+    const int64_t i = m0 + site(t), p = (n0 >> 1) + col(t);
+    if (i < g.N && p < g.P) {
+      const float2* ys = g.fwd ? sd.rnext : sd.y;
+      if (ys) asm volatile("prefetch.global.L2 [%0];" ::"l"(ys + i * g.P + p));
+      if (!g.fwd) asm volatile("prefetch.global.L2 [%0];" ::"l"(sd.x + i * g.P + p));
+    }
   }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  if (threadIdx.x == 0 && threadIdx.y == 0) {
-    double a = 0.0, b = 0.0;
-    for (int w = 0; w < 8; w++) {
-      a += red[0][w];
-      b += red[1][w];
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = tmem_sh;
+  pdl_wait();
+
+  if (tid == 0) {
+    for (int kt = 0; kt < nk; kt++) {
+      if (kt >= S) {
+        if (!wait_bar(tc32::su32(&empty_bar[kt % S]), ((kt / S) - 1) & 1, g.status, g.timeout)) break;
+        load_a(kt);
+      }
+      load_b(kt);
     }
-    atomicAdd(norms + 0, a);
-    atomicAdd(norms + 1, b);
-    if (k == 0) {
-      atomicAdd(norms + 2, a);
-      atomicAdd(norms + 3, b);
+  } else if (tid == 32) {
+    // 4 K-steps of 8 per stage: A_hi [B_hi; B_lo] as one MMA of 2 BN columns (A
+    // is read once for both; the operands' reads from shared memory and the
+    // copies into it bound the loop), A_lo B_hi on top of its first half
+    for (int kt = 0; kt < nk; kt++) {
+      const int st = kt % S;
+      if (!wait_bar(tc32::su32(&full_bar[st]), (kt / S) & 1, g.status, g.timeout)) break;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const uint64_t ah = tc32::sw128_desc(sA(st)), al = tc32::sw128_desc(sA(st) + C::A_BYTES);
+      const uint64_t bh = tc32::sw128_desc(sA(st) + 2 * C::A_BYTES);  // B_hi's rows, then B_lo's
+#pragma unroll
+      for (int kk = 0; kk < tc32::BK / 8; kk++) {
+        const uint64_t o = (uint64_t)(kk * 32 / 16);  // 8 fp32 = 32 bytes along the swizzled row
+        tc32::mma_tf32(tmem, ah + o, bh + o, tc32::Cfg<2 * BN>::IDESC, (kt | kk) != 0);
+        tc32::mma_tf32(tmem, al + o, bh + o, C::IDESC, 1);
+      }
+      tc32::mma_commit(tc32::su32(&empty_bar[st]));
     }
-    if (k == L - 1) {
-      atomicAdd(norms + 4, a);
-      atomicAdd(norms + 5, b);
+    tc32::mma_commit(tc32::su32(&done_bar));
+  }
+  __syncwarp();
+  // y and x of this thread's first U elements, while the products run
+  float2 d[U], yv[U];
+  double2 xv[U];
+  auto element = [&](int t, int64_t* ip) {
+    const int64_t i = m0 + site(t), p = (n0 >> 1) + col(t);
+    *ip = i * g.P + p;
+    return t < ITEMS && i < g.N && p < g.P;
+  };
+  auto load_yx = [&](int t0) {
+    const float2* ys = g.fwd ? sd.rnext : sd.y;
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      int64_t ip;
+      const bool in = element(t0 + u * W * Z, &ip);
+      yv[u] = (in && ys) ? ys[ip] : make_float2(0.f, 0.f);
+      if (in && !g.fwd) xv[u] = sd.x[ip];
+    }
+  };
+  load_yx(z * W + warp);
+  // one warp polls, the rest sleep at the barrier; a wait that ran out has set the status the host checks
+  if (warp == 1) wait_bar(tc32::su32(&done_bar), 0, g.status, g.timeout);
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  {  // accumulator -> this CTA's tile (over the drained stages)
+    float* tile = reinterpret_cast<float*>(smem_raw + (base - tc32::su32(smem_raw)));
+    const int row = 32 * (warp & 3) + lane, c0 = (warp >> 2) * (BN * 4 / W);
+#pragma unroll
+    for (int c = 0; c < BN * 4 / W; c += 16) {
+      float v[16], w[16];
+      tc32::tmem_ld16(tmem + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)(c0 + c), v);
+      tc32::tmem_ld16(tmem + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)(BN + c0 + c), w);
+#pragma unroll
+      for (int j = 0; j < 16; j++) v[j] += w[j];
+      float4* t4 = reinterpret_cast<float4*>(tile + row * TP + c0 + c);
+#pragma unroll
+      for (int j = 0; j < 4; j++) t4[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
     }
   }
-  if (write_bt) store_bt(tile, p0, i0, N, P, bt_hi, bt_lo, lda);
-  if (bt2_hi) store_bt(tile, p0, i0, N, P, bt2_hi, bt2_lo, lda);
+  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+
+  double dd = 0.0, xx = 0.0;
+  for (int t0 = z * W + warp; t0 < ITEMS; t0 += U * W * Z) {
+    if (t0 >= U * W * Z) load_yx(t0);
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const int t = t0 + u * W * Z;
+      d[u] = make_float2(0.f, 0.f);
+      if (t < ITEMS) {
+        const uint32_t off = base + (uint32_t)(site(t) * TP + 2 * col(t)) * 4u;
+#pragma unroll
+        for (int q = 0; q < 8; q++) {
+          if (q >= Z) break;
+          uint32_t ra;
+          float2 v;
+          asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(off), "r"(q));
+          asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(ra) : "memory");
+          d[u].x += v.x;
+          d[u].y += v.y;
+        }
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const int t = t0 + u * W * Z;
+      int64_t ip;
+      if (!element(t, &ip)) continue;
+      const int64_t i = m0 + site(t), p = (n0 >> 1) + col(t);
+      float2 v = make_float2(d[u].x + yv[u].x, d[u].y + yv[u].y);
+      if (g.fwd) {
+        sd.y[ip] = d[u];
+      } else {
+        const double2 xn = cmk(xv[u].x + (double)v.x, xv[u].y + (double)v.y);
+        sd.x[ip] = xn;
+        dd += (double)v.x * v.x + (double)v.y * v.y;
+        xx += xn.x * xn.x + xn.y * xn.y;
+      }
+      const int64_t o = (2 * p) * g.lda + 2 * i;
+      if (sd.bt_hi) {
+        split2(v.x, -v.y, sd.bt_hi + o, sd.bt_lo + o);
+        split2(v.y, v.x, sd.bt_hi + o + g.lda, sd.bt_lo + o + g.lda);
+      }
+      if (sd.bt2_hi) {
+        split2(v.x, -v.y, sd.bt2_hi + o, sd.bt2_lo + o);
+        split2(v.y, v.x, sd.bt2_hi + o + g.lda, sd.bt2_lo + o + g.lda);
+      }
+    }
+  }
+  if (!g.fwd) {
+    for (int o = 16; o > 0; o >>= 1) {
+      dd += __shfl_xor_sync(0xffffffffu, dd, o);
+      xx += __shfl_xor_sync(0xffffffffu, xx, o);
+    }
+    if (lane == 0) {
+      red[0][warp] = dd;
+      red[1][warp] = xx;
+    }
+    __syncthreads();
+    if (tid < 2) {
+      double a = 0.0;
+      for (int w = 0; w < W; w++) a += red[tid][w];
+      atomicAdd(g.norms + tid, a);
+      if (sd.ends & 1) atomicAdd(g.norms + 2 + tid, a);
+      if (sd.ends & 2) atomicAdd(g.norms + 4 + tid, a);
+    }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == 1)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * C::TMEM_COLS) : "memory");
+  // no CTA leaves while another reads its tile
+  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
 }
 
 // B columns in S order: left inputs into Bl, right inputs into Br (N x P row-major)
@@ -404,18 +589,6 @@ constexpr int TP = BN + 4;              // pitch of the epilogue staging tile (o
 static_assert(128 * TP * 4 <= OFF_WP, "staging tile");
 static_assert(SMEM <= 227 * 1024, "shared memory of one CTA");
 }  // namespace gjs
-
-__device__ __forceinline__ bool wait_bar(uint32_t bar, uint32_t parity, int* status, long long timeout) {
-  if (tc32::mbar_try(bar, parity)) return true;
-  const long long t0 = clock64();
-  while (!tc32::mbar_try(bar, parity)) {
-    if (clock64() - t0 > timeout) {
-      atomicOr(status, kStatusTimeout);
-      return false;
-    }
-  }
-  return true;
-}
 
 // Development builds only (-DRGF_MX_STAMPS, never in the shipped library):
 // %globaltimer at the phase boundaries of one CTA of the step kernel.
@@ -1004,27 +1177,39 @@ __global__ void __launch_bounds__(256) k_mx_t0(const float* __restrict__ W, int6
 
 inline int64_t lda_of(int64_t N) { return (2 * N + 31) / 32 * 32; }
 
+// K-split of the solve: the largest, up to the 8 CTAs of a portable cluster
+// and the K-chunk count, whose clusters all run at once (a cluster needs its
+// SMs in one GPC, so that fewer fit than SMs / split)
 template <int BN>
-rgf_status gemm_attr() {
-  static thread_local int done_dev = -1;
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (done_dev == dev) return RGF_OK;
-  if (cudaFuncSetAttribute(tc32::k_tc32_gemm<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           tc32::Cfg<BN>::SMEM) != cudaSuccess) {
-    set_error("cannot configure the tcgen05 GEMM's shared memory");
+rgf_status solve_split(int64_t clusters, int64_t kchunks, int* split) {
+  if (cudaFuncSetAttribute(k_mx_solve<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, tc32::Cfg<BN>::SMEM) !=
+      cudaSuccess) {
+    set_error("cannot configure the tcgen05 solve's shared memory");
     return RGF_ERR_CUDA;
   }
-  done_dev = dev;
+  *split = 1;
+  for (int z = (int)std::min<int64_t>(8, kchunks); z > 1; z--) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(1, 1, (unsigned)z);
+    cfg.blockDim = dim3(kSolveWarps * 32);
+    cfg.dynamicSmemBytes = tc32::Cfg<BN>::SMEM;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = (unsigned)z;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    int fit = 0;
+    if (cudaOccupancyMaxActiveClusters(&fit, k_mx_solve<BN>, &cfg) != cudaSuccess) {
+      cudaGetLastError();
+      continue;
+    }
+    if (fit >= clusters) {
+      *split = z;
+      break;
+    }
+  }
   return RGF_OK;
-}
-
-// ksplit: the largest divisor of the K-chunk count that keeps tiles*ksplit <= SMs
-int choose_ksplit(int64_t tiles, int64_t kchunks, int sms) {
-  int best = 1;
-  for (int64_t z = 1; z <= kchunks; z++)
-    if (kchunks % z == 0 && tiles * z <= sms) best = (int)z;
-  return best;
 }
 
 }  // namespace
@@ -1048,8 +1233,7 @@ size_t mixed_workspace_bytes(int64_t N, int64_t L, int64_t P) {
   b += 2 * sizeof(float) * N * lda * L;       // factor store hi/lo
   b += sizeof(double2) * N * P * L;           // x
   b += sizeof(float2) * N * P * L;            // y
-  b += sizeof(float2) * N * P * 148;          // partials (at most one per SM)
-  b += 2 * sizeof(float) * 2 * P * lda;       // Bt hi/lo
+  b += 8 * sizeof(float) * 2 * P * lda;       // Bt hi/lo, two buffers per side
   b += sizeof(double2) * N * P * 6;           // Bl, Br, b0, bL, e0/e1 (also G0 (B + x) at the end)
   b += 4 * (sizeof(float2) * NB * NB + gjs::TU_BYTES);  // pivot-block inverses and their images
   return b;
@@ -1067,7 +1251,7 @@ rgf_status smatrix_mixed(const MixedProblem& mp, const MixedAlloc& alloc, cudaSt
     set_error("cannot configure the Gauss-Jordan step kernel's shared memory");
     return RGF_ERR_CUDA;
   }
-  void *pW, *pT, *pSh, *pSl, *pX, *pY, *pPart, *pBt, *pVec, *pNorm, *pStat;
+  void *pW, *pT, *pSh, *pSl, *pX, *pY, *pBt, *pVec, *pNorm, *pStat;
   const int ntile_m = (int)((N + tc32::BM - 1) / tc32::BM);
   const int kchunks = (int)(lda / tc32::BK);
   // Two-sided form (L >= 8): the slices [0, c-1) are factored from the left
@@ -1080,20 +1264,21 @@ rgf_status smatrix_mixed(const MixedProblem& mp, const MixedAlloc& alloc, cudaSt
   const int64_t cj = two ? (L + 1) / 2 : L;  // junction slice + 1 (two-sided)
   const int nside = two ? 2 : 1;
   // solve GEMM tile width: 64 real columns for narrow requests, else 128 (a
-  // three-deep TMA pipeline).  Measured slower at config 2 (2P = 408): 256-wide
+  // three-deep TMA pipeline).  Measured slower for 2P = 408 columns: 256-wide
   // tiles (two stages only, stalled on the loads) and 3 tiles of 144 with a
-  // ragged 3-way K-split (780 ms of solves against 715 ms for 4 x 128, 2-way).
+  // ragged 3-way K-split.
   const int sbn = (2 * P <= 64) ? 64 : 128;
-  if ((st = gemm_attr<64>()) || (st = gemm_attr<128>())) return st;
   int sTiles = (int)((2 * P + sbn - 1) / sbn);
-  int sSplit = choose_ksplit((int64_t)ntile_m * sTiles, kchunks, sms / nside);
+  int sSplit = 1;
+  if ((st = sbn == 64 ? solve_split<64>((int64_t)ntile_m * sTiles * nside, kchunks, &sSplit)
+                      : solve_split<128>((int64_t)ntile_m * sTiles * nside, kchunks, &sSplit)))
+    return st;
   if ((st = alloc(kMxW, 2 * nside * sizeof(float) * N * lda, &pW)) ||
       (st = alloc(kMxT, (sizeof(float2) * NB * NB + gjs::TU_BYTES) * 2 * nside, &pT)) ||
       (st = alloc(kMxStoreHi, sizeof(float) * N * lda * L, &pSh)) ||
       (st = alloc(kMxStoreLo, sizeof(float) * N * lda * L, &pSl)) ||
       (st = alloc(kMxX, sizeof(double2) * NP * L, &pX)) || (st = alloc(kMxY, sizeof(float2) * NP * L, &pY)) ||
-      (st = alloc(kMxPart, sizeof(float2) * NP * sSplit * nside, &pPart)) ||
-      (st = alloc(kMxBt, 2 * nside * sizeof(float) * 2 * P * lda, &pBt)) ||
+      (st = alloc(kMxBt, 4 * nside * sizeof(float) * 2 * P * lda, &pBt)) ||
       (st = alloc(kMxVec, sizeof(double2) * NP * 6, &pVec)) || (st = alloc(kMxNorm, sizeof(double) * 8, &pNorm)) ||
       (st = alloc(kMxStatus, 4 * sizeof(int), &pStat)))
     return st;
@@ -1113,17 +1298,15 @@ rgf_status smatrix_mixed(const MixedProblem& mp, const MixedAlloc& alloc, cudaSt
 
   // per side: two W buffers with their tensor maps (swizzled 32-column boxes
   // for the update's left operand, unswizzled ones for the W' tile), two
-  // pivot-block inverses, the solve's right operand Bt (2P rows x lda, hi/lo)
-  // and its GEMM partials; the factor store (N rows x lda, L slices) is shared
+  // pivot-block inverses and two buffers of the solve's right operand Bt (2P
+  // rows x lda, hi/lo); the factor store (N rows x lda, L slices) is shared
   struct Side {
     float* W[2];
-    CUtensorMap mA[2], mWp[2], mBh, mBl;
+    CUtensorMap mA[2], mWp[2], mBh[2], mBl[2];
     float2* Tb;
     uint8_t* Tu;  // images of the two inverses (publish_tu)
-    float* bh;
-    float* bl;
-    float2* part;
-    int cur = 0;
+    float *bh[2], *bl[2];
+    int cur = 0, bcur = 0;
     int64_t gstep = 0;
     cudaStream_t q = nullptr;
     int64_t first = 0, count = 0, dir = 1;  // the side's slices: first, first + dir, ... (count of them)
@@ -1137,14 +1320,14 @@ rgf_status smatrix_mixed(const MixedProblem& mp, const MixedAlloc& alloc, cudaSt
     d.W[1] = d.W[0] + N * lda;
     d.Tb = static_cast<float2*>(pT) + 2 * q * NB * NB;
     d.Tu = static_cast<uint8_t*>(pT) + sizeof(float2) * NB * NB * 2 * nside + 2 * q * gjs::TU_BYTES;
-    d.bh = bt_hi + q * 4 * P * lda;
-    d.bl = d.bh + 2 * P * lda;
-    d.part = static_cast<float2*>(pPart) + q * NP * sSplit;
-    for (int w = 0; w < 2; w++)
+    for (int w = 0; w < 2; w++) {
+      d.bh[w] = bt_hi + (q * 4 + 2 * w) * 2 * P * lda;
+      d.bl[w] = d.bh[w] + 2 * P * lda;
       maps_ok = maps_ok && tc32::make_map(&d.mA[w], d.W[w], lda, N, 1, lda, 0, tc32::BM) &&
-                tc32::make_map(&d.mWp[w], d.W[w], lda, N, 1, lda, 0, tc32::BM, CU_TENSOR_MAP_SWIZZLE_NONE);
-    maps_ok = maps_ok && tc32::make_map(&d.mBh, d.bh, lda, 2 * P, 1, lda, 0, sbn) &&
-              tc32::make_map(&d.mBl, d.bl, lda, 2 * P, 1, lda, 0, sbn);
+                tc32::make_map(&d.mWp[w], d.W[w], lda, N, 1, lda, 0, tc32::BM, CU_TENSOR_MAP_SWIZZLE_NONE) &&
+                tc32::make_map(&d.mBh[w], d.bh[w], lda, 2 * P, 1, lda, 0, sbn) &&
+                tc32::make_map(&d.mBl[w], d.bl[w], lda, 2 * P, 1, lda, 0, sbn);
+    }
   }
   if (!maps_ok) {
     set_error("tensor-map encoding for the tcgen05 GEMM failed");
@@ -1189,7 +1372,7 @@ rgf_status smatrix_mixed(const MixedProblem& mp, const MixedAlloc& alloc, cudaSt
   };
   RGF_CUDA_TRY_MX(cudaMemsetAsync(mstat, 0, sizeof(int), s));
   RGF_CUDA_TRY_MX(cudaMemsetAsync(pW, 0, 2 * nside * sizeof(float) * N * lda, s));
-  RGF_CUDA_TRY_MX(cudaMemsetAsync(bt_hi, 0, 2 * nside * sizeof(float) * 2 * P * lda, s));  // zero K padding
+  RGF_CUDA_TRY_MX(cudaMemsetAsync(bt_hi, 0, 4 * nside * sizeof(float) * 2 * P * lda, s));  // zero K padding
   RGF_CUDA_TRY_MX(cudaMemsetAsync(x, 0, sizeof(double2) * NP * L, s));
   cudaEvent_t ev[3];
   for (int q = 0; q < 3; q++) RGF_CUDA_TRY_MX(cudaEventCreate(&ev[q]));
@@ -1309,45 +1492,69 @@ rgf_status smatrix_mixed(const MixedProblem& mp, const MixedAlloc& alloc, cudaSt
   nl += 3;
 
   // (3) refinement
-  tc32::GemmArgs gs[2];
-  for (int q = 0; q < nside; q++) {
-    gs[q] = tc32::GemmArgs{};
-    gs[q].M = (int)N;
-    gs[q].Nr = (int)(2 * P);
-    gs[q].k_chunks = kchunks / sSplit;
-    gs[q].mode = tc32::kPartial;
-    gs[q].out = reinterpret_cast<float*>(sd[q].part);
-    gs[q].ldo = 2 * P;
-    gs[q].split_stride = 2 * NP;
-    gs[q].err = mstat;
-    gs[q].timeout = kGemmTimeout;
-  }
-  const dim3 gsg((unsigned)sTiles, (unsigned)ntile_m, (unsigned)sSplit);
+  const dim3 gsg((unsigned)(sTiles * nside), (unsigned)ntile_m, (unsigned)sSplit);
   const dim3 gp((unsigned)((P + 31) / 32), (unsigned)((N + 31) / 32));
   const dim3 tp(32, 8);
-  // side q's GEMM: partials = g_k Bt (Bt of side qb, default q)
-  auto gemm = [&](int q, int64_t k, cudaStream_t qs) {
-    gs[q].a_z = (int)k;
+  SolveMaps maps;
+  maps.a_hi = mSh;
+  maps.a_lo = mSl;
+  SolveArgs sa{};
+  sa.N = N;
+  sa.P = P;
+  sa.lda = lda;
+  sa.k_chunks = kchunks;
+  sa.tiles = sTiles;
+  sa.norms = norms;
+  sa.status = mstat;
+  sa.timeout = kGemmTimeout;
+  // right operand of side q's first step, or of the junction (slice k, y of its neighbours)
+  auto rhs = [&](int q, int64_t k, const float2* ya, const float2* yb) {
+    launch_pdl(k_mx_rhs, gp, tp, 0, s, N, P, (const float2*)(y + k * NP), ya, yb, sd[q].bh[sd[q].bcur],
+               sd[q].bl[sd[q].bcur], lda);
+    nl++;
+  };
+  // side q's part of the next launch: slice k, reading the side's current right
+  // operand and (next) writing its other buffer, which then is the current one
+  auto step = [&](int q, int64_t k, bool next) -> SolveSide& {
+    Side& d = sd[q];
+    SolveSide& v = sa.sd[q];
+    v = SolveSide{};
+    v.active = 1;
+    v.k = (int)k;
+    maps.b_hi[q] = d.mBh[d.bcur];
+    maps.b_lo[q] = d.mBl[d.bcur];
+    if (next) {
+      d.bcur ^= 1;
+      v.bt_hi = d.bh[d.bcur];
+      v.bt_lo = d.bl[d.bcur];
+    }
+    return v;
+  };
+  auto step_fwd = [&](int q, int64_t k, int64_t knext) {
+    SolveSide& v = step(q, k, knext >= 0);
+    v.y = y + k * NP;
+    v.rnext = knext >= 0 ? y + knext * NP : nullptr;
+  };
+  auto step_bwd = [&](int q, int64_t k, bool add_y, bool next) -> SolveSide& {
+    SolveSide& v = step(q, k, next);
+    v.y = add_y ? y + k * NP : nullptr;
+    v.x = x + k * NP;
+    v.ends = (k == 0 ? 1 : 0) | (k == L - 1 ? 2 : 0);
+    return v;
+  };
+  auto solve = [&](bool fwd) {
+    sa.fwd = fwd;
     if (sbn == 64)
-      launch_pdl(tc32::k_tc32_gemm<64>, gsg, dim3(tc32::kThreads), tc32::Cfg<64>::SMEM, qs, mSh, mSl, sd[q].mBh,
-                 sd[q].mBl, gs[q]);
+      launch_pdl_cluster(k_mx_solve<64>, gsg, dim3(kSolveWarps * 32), tc32::Cfg<64>::SMEM, sSplit, s, maps, sa);
     else
-      launch_pdl(tc32::k_tc32_gemm<128>, gsg, dim3(tc32::kThreads), tc32::Cfg<128>::SMEM, qs, mSh, mSl, sd[q].mBh,
-                 sd[q].mBl, gs[q]);
+      launch_pdl_cluster(k_mx_solve<128>, gsg, dim3(kSolveWarps * 32), tc32::Cfg<128>::SMEM, sSplit, s, maps, sa);
     nl++;
+    sa.sd[0].active = sa.sd[1].active = 0;
   };
-  auto fwd_prep = [&](int q, int64_t k, int64_t kprev, cudaStream_t qs, int q2 = -1, int64_t kprev2 = -1) {
-    launch_pdl(k_mx_fwd_prep, gp, tp, 0, qs, k, kprev, N, P, P, (int64_t)0, y, (const float2*)sd[q].part, sSplit,
-               (const float2*)(q2 >= 0 ? sd[q2].part : nullptr), kprev2, sSplit, sd[q].bh, sd[q].bl, lda,
-               (const int*)nullptr);
-    nl++;
-  };
-  auto bwd_prep = [&](int q, int64_t k, int add_y, int write_bt, cudaStream_t qs, int q2 = -1) {
-    launch_pdl(k_mx_bwd_prep, gp, tp, 0, qs, k, L, N, P, P, (int64_t)0, x, (const float2*)y,
-               (const float2*)sd[q].part, sSplit, sd[q].bh, sd[q].bl, lda, norms, (const int*)nullptr, add_y,
-               write_bt, q2 >= 0 ? sd[q2].bh : nullptr, q2 >= 0 ? sd[q2].bl : nullptr);
-    nl++;
-  };
+  for (int q = 0; q < 2; q++) {  // a side without a step still needs valid maps
+    maps.b_hi[q] = sd[0].mBh[0];
+    maps.b_lo[q] = sd[0].mBl[0];
+  }
   double prev = 1.0, change = 1.0;
   bool conv = false;
   int it = 0;
@@ -1364,42 +1571,33 @@ rgf_status smatrix_mixed(const MixedProblem& mp, const MixedAlloc& alloc, cudaSt
                (const double2*)b0, (const double2*)bL, (const double2*)(have_x ? e0 : nullptr),
                (const double2*)(have_x ? e1 : nullptr));
     nl++;
-    if (!two) {
-      // forward y_k = g_k (r_k + y_{k-1}), backward d_k = y_k + g_k d_{k+1}
-      for (int64_t k = 0; k < L; k++) {
-        fwd_prep(0, k, k - 1, s);
-        gemm(0, k, s);
+    // forward y_k = g_k (r_k + y of the slice before) from the leads to the
+    // slice kj in front of which the sides meet (one side: the last slice),
+    // d_kj = g_kj v_kj there, backward d_k = y_k + g_k d of the slice before
+    const int64_t kj = two ? cj - 1 : L - 1;
+    const int64_t nf = two ? std::max(sd[0].count, sd[1].count) : L - 1;
+    for (int q = 0; q < nside; q++) rhs(q, sd[q].first, nullptr, nullptr);
+    for (int64_t i = 0; i < nf; i++) {
+      for (int q = 0; q < nside; q++) {
+        if (two && i >= sd[q].count) continue;
+        const int64_t k = sd[q].first + sd[q].dir * i;
+        step_fwd(q, k, two && i + 1 == sd[q].count ? -1 : k + sd[q].dir);
       }
-      for (int64_t k = L - 1; k >= 0; k--) {
-        bwd_prep(0, k, k < L - 1, k > 0, s);
-        if (k > 0) gemm(0, k - 1, s);
+      solve(true);
+    }
+    if (two) rhs(0, kj, y + (cj - 2) * NP, y + cj * NP);
+    SolveSide& vj = step_bwd(0, kj, false, true);
+    if (two) {
+      vj.bt2_hi = sd[1].bh[sd[1].bcur];
+      vj.bt2_lo = sd[1].bl[sd[1].bcur];
+    }
+    solve(false);
+    for (int64_t i = nf - 1; i >= 0; i--) {
+      for (int q = 0; q < nside; q++) {
+        if (two && i >= sd[q].count) continue;
+        step_bwd(q, sd[q].first + sd[q].dir * i, true, i > 0);
       }
-    } else {
-      // forward from both leads towards the junction slice cj - 1
-      if ((st = fork_sides())) return st;
-      const int64_t nmx = std::max(sd[0].count, sd[1].count);
-      for (int64_t i = 0; i < nmx; i++)
-        for (int q = 0; q < 2; q++) {
-          if (i >= sd[q].count) continue;
-          const int64_t k = sd[q].first + sd[q].dir * i;
-          fwd_prep(q, k, i > 0 ? k - sd[q].dir : -1, sd[q].q);
-          gemm(q, k, sd[q].q);
-        }
-      if ((st = join_sides())) return st;
-      // junction: d_{cj-1} = G_{cj-1} (r + y_{cj-2} + y_{cj}), into both sides' Bt
-      fwd_prep(0, cj - 1, cj - 2, s, 1, cj);
-      gemm(0, cj - 1, s);
-      bwd_prep(0, cj - 1, 0, 1, s, 1);
-      // backward outwards: d_k = y_k + g_k d_{k +- 1}
-      if ((st = fork_sides())) return st;
-      for (int64_t i = nmx - 1; i >= 0; i--)
-        for (int q = 0; q < 2; q++) {
-          if (i >= sd[q].count) continue;
-          const int64_t k = sd[q].first + sd[q].dir * i;
-          gemm(q, k, sd[q].q);
-          bwd_prep(q, k, 1, i > 0, sd[q].q);
-        }
-      if ((st = join_sides())) return st;
+      solve(false);
     }
     RGF_CUDA_TRY_MX(cudaGetLastError());
     double hn[8];
