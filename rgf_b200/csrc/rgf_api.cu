@@ -100,6 +100,7 @@ struct rgf_handle_s {
   DevBuf sp_ck[2], sp_m0, sp_seg, sp_g[2];  // gradient and fields of a split structure
   cudaStream_t aux_stream = nullptr;  // the right chain's joins
   cudaEvent_t aux_ev[2] = {nullptr, nullptr};
+  GjAhead ahead{};  // panels of the per-step engine beside the updates
   // tuned tile table of the persistent engine: rows Rp <= tile_rmax[i] use
   // tile tile_bm[i] (first match) when its grid fits the GPU
   std::vector<int64_t> tile_rmax;
@@ -760,6 +761,23 @@ rgf_status second_stream(rgf_handle h) {
   return RGF_OK;
 }
 
+// widths from which the per-step engine runs its panels beside the updates:
+// below, a step is all panel and the launches and events between two streams
+// cost more than they hide (us a step, in turn / side by side: 58.9 / 60.2 at
+// N = 256, 58.4 / 57.0 at 400, 70 / 63 at 512, 85 / 69 at 1000, 106 / 78 at
+// 1500, 146 / 102 at 1900)
+constexpr int64_t kAheadMin = 400;
+rgf_status ensure_ahead(rgf_handle h) {
+  GjAhead& a = h->ahead;
+  if (a.stream) return RGF_OK;
+  if (!a.panel) RGF_CUDA_TRY(cudaEventCreateWithFlags(&a.panel, cudaEventDisableTiming));
+  if (!a.update) RGF_CUDA_TRY(cudaEventCreateWithFlags(&a.update, cudaEventDisableTiming));
+  int least = 0, greatest = 0;
+  RGF_CUDA_TRY(cudaDeviceGetStreamPriorityRange(&least, &greatest));
+  RGF_CUDA_TRY(cudaStreamCreateWithPriority(&a.stream, cudaStreamNonBlocking, greatest));
+  return RGF_OK;
+}
+
 // sweep of a join matrix Q (R x C, leading dimension C): N pivots over the
 // whole column with the buffers of chain c; only the corner is kept up to date
 // unless `whole`
@@ -768,8 +786,8 @@ rgf_status join_sweep(rgf_handle h, const SplitProblem& p, double2* Q, int64_t R
   const int kSwW = sweep_block_width();
   for (int64_t j0 = 0; j0 < p.N; j0 += kSwW) {
     const int jn = (int)std::min<int64_t>(kSwW, p.N - j0);
-    RGF_CUDA_TRY(launch_gj_panel(Q, C, R, p.N, j0, jn, !whole, as<double2>(h->sp_p[c]), h->sp_s[c].p, p.status, s));
-    launch_gj_update(Q, C, R, p.N, C, j0, jn, !whole, as<double2>(h->sp_p[c]), as<double2>(h->sp_w[c]), h->sp_s[c].p, s);
+    RGF_CUDA_TRY(launch_gj_step(Q, C, R, p.N, C, j0, jn, !whole, as<double2>(h->sp_p[c]), as<double2>(h->sp_w[c]),
+                                h->sp_s[c].p, p.status, s));
     h->launches += 3;
   }
   if (whole) {
@@ -1573,12 +1591,19 @@ rgf_status smatrix_run(rgf_handle h, const Problem& p, const rgf_request* req, c
   // the swept matrix.
   auto sweep = [&](int64_t Ract, int64_t Cact, bool timed, bool corner_only) -> rgf_status {
     const bool in_cluster = gj_step_fits(Ract);
-    for (int64_t j0 = 0; j0 < N; j0 += kSwW) {
+    const bool ahead = in_cluster && !timed && !h->arena && !h->sm_budget && N >= kAheadMin;
+    if (ahead) {
+      if ((st = ensure_ahead(h)) || (st = ensure(h, h->pc, 2 * sizeof(double2) * std::max(R, Cp) * kSwW))) return st;
+      const cudaError_t e = launch_gj_sweep(M, ldm, Ract, N, Cact, corner_only, as<double2>(h->pc), as<double2>(h->u),
+                                            h->gepp.p, status, h->stream, h->ahead);
+      if (e != cudaSuccess) cudaStreamSynchronize(h->ahead.stream);
+      RGF_CUDA_TRY(e);
+      h->launches += 5 * ((N + kSwW - 1) / kSwW) - 2;
+    }
+    for (int64_t j0 = 0; j0 < N && !ahead; j0 += kSwW) {
       int jn = (int)std::min<int64_t>(kSwW, N - j0);
-      if (in_cluster) {
-        RGF_CUDA_TRY(launch_gj_panel(M, ldm, Ract, N, j0, jn, corner_only, as<double2>(h->pc), h->gepp.p, status,
-                                     h->stream));
-      } else {
+      cudaEvent_t before = nullptr, after = nullptr;
+      if (!in_cluster) {
         launch_gepp_step(M, ldm, N, Cact, j0, jn, h->gepp.p, status, h->stream);
         launch_sweep_panel(M, ldm, Ract, Cact, j0, jn, as<double2>(h->pc), as<double2>(h->u), ldm, status,
                            h->stream);
@@ -1590,19 +1615,19 @@ rgf_status smatrix_run(rgf_handle h, const Problem& p, const rgf_request* req, c
           RGF_CUDA_TRY(cudaEventCreate(&ev));
           h->ev.push_back(ev);
         }
-        RGF_CUDA_TRY(cudaEventRecord(h->ev[ev_used], h->stream));
-      }
-      if (in_cluster) {
-        launch_gj_update(M, ldm, Ract, N, Cact, j0, jn, corner_only, as<double2>(h->pc), as<double2>(h->u),
-                         h->gepp.p, h->stream);
-        h->launches++;
-      } else {
-        launch_sweep_update(M, ldm, Ract, Cact, j0, jn, as<double2>(h->pc), as<double2>(h->u), ldm, h->stream);
-      }
-      if (timed) {
-        RGF_CUDA_TRY(cudaEventRecord(h->ev[ev_used + 1], h->stream));
+        before = h->ev[ev_used];
+        after = h->ev[ev_used + 1];
         ev_used += 2;
         prof_flops += 8.0 * (double)Ract * (double)Cact * (double)jn;
+      }
+      if (in_cluster) {
+        RGF_CUDA_TRY(launch_gj_step(M, ldm, Ract, N, Cact, j0, jn, corner_only, as<double2>(h->pc), as<double2>(h->u),
+                                    h->gepp.p, status, h->stream, before, after));
+        h->launches++;
+      } else {
+        if (timed) RGF_CUDA_TRY(cudaEventRecord(before, h->stream));
+        launch_sweep_update(M, ldm, Ract, Cact, j0, jn, as<double2>(h->pc), as<double2>(h->u), ldm, h->stream);
+        if (timed) RGF_CUDA_TRY(cudaEventRecord(after, h->stream));
       }
       h->launches += 2;
     }
@@ -2089,8 +2114,8 @@ rgf_status segment_merge(rgf_handle h, const Problem& p, const rgf_request* req,
   for (int64_t j0 = 0; j0 < N; j0 += kSwW) {
     const int jn = (int)std::min<int64_t>(kSwW, N - j0);
     if (in_cluster) {
-      RGF_CUDA_TRY(launch_gj_panel(M, ldm, R, N, j0, jn, true, as<double2>(h->pc), h->gepp.p, status, h->stream));
-      launch_gj_update(M, ldm, R, N, C, j0, jn, true, as<double2>(h->pc), as<double2>(h->u), h->gepp.p, h->stream);
+      RGF_CUDA_TRY(launch_gj_step(M, ldm, R, N, C, j0, jn, true, as<double2>(h->pc), as<double2>(h->u), h->gepp.p,
+                                  status, h->stream));
       h->launches += 3;
       continue;
     }
@@ -2250,6 +2275,9 @@ rgf_status rgf_destroy(rgf_handle h) {
   for (cudaEvent_t ev : h->aux_ev)
     if (ev) cudaEventDestroy(ev);
   if (h->aux_stream) cudaStreamDestroy(h->aux_stream);
+  if (h->ahead.panel) cudaEventDestroy(h->ahead.panel);
+  if (h->ahead.update) cudaEventDestroy(h->ahead.update);
+  if (h->ahead.stream) cudaStreamDestroy(h->ahead.stream);
   for (cudaEvent_t ev : h->ev) cudaEventDestroy(ev);
   if (h->own_stream) cudaStreamDestroy(h->own_stream);
   for (rgf_handle_s* w : h->workers) rgf_destroy(w);

@@ -570,7 +570,8 @@ __global__ void k_colperm(double2* M, int64_t ldm, int64_t R, int64_t N, const i
 // step's 2900 when it was done that way).  Lane = column with a row per register
 // needs no rotation but three times the instructions per pivot: 84 us against
 // 72 us for 1700 rows.  The one-CTA panel above (its rows in L2) takes 770 us
-// there; a whole step went from 787 to 104 us at N = 1500.
+// there; a whole step went from 787 to 106 us at N = 1500, and to 78 us with the
+// panels beside the updates (launch_gj_sweep).
 // ---------------------------------------------------------------------------
 constexpr int kGjRows = 256;     // most rows of a CTA
 constexpr int kGjCluster = 16;   // most CTAs of a cluster
@@ -777,11 +778,12 @@ constexpr int kColpermCtas = 64;
 // Wr(q, c) = W(src[q], c) on columns [c0, Cc) (unit columns in J, zero rows
 // from jn on), and the displaced rows of J to their places outside it.  32
 // columns a CTA; every thread reads its rows before the CTA writes any.
-__global__ void __launch_bounds__(256) k_pivot_rows(double2* W, int64_t ldm, int64_t c0, int64_t Cc, int64_t j0, int jn,
-                                                    const int* __restrict__ src, const int* __restrict__ dst,
-                                                    double2* __restrict__ Wr) {
+__global__ void __launch_bounds__(256) k_pivot_rows(double2* W, int64_t ldm, int64_t c0, int64_t Cc, int64_t x0,
+                                                    int64_t x1, int64_t j0, int jn, const int* __restrict__ src,
+                                                    const int* __restrict__ dst, double2* __restrict__ Wr) {
   const int64_t c = c0 + blockIdx.x * (int64_t)32 + (threadIdx.x & 31);
   const int g = threadIdx.x >> 5;
+  const bool in = c < Cc && !(c >= x0 && c < x1);
   double2 v[4], u[4];
   int to[4];
 #pragma unroll
@@ -789,7 +791,7 @@ __global__ void __launch_bounds__(256) k_pivot_rows(double2* W, int64_t ldm, int
     const int q = g * 4 + k;
     to[k] = -1;
     v[k] = u[k] = cmk(0.0, 0.0);
-    if (q < jn && c < Cc) {
+    if (q < jn && in) {
       if (c >= j0 && c < j0 + jn) {
         v[k] = cmk(c - j0 == q ? 1.0 : 0.0, 0.0);
       } else {
@@ -803,7 +805,7 @@ __global__ void __launch_bounds__(256) k_pivot_rows(double2* W, int64_t ldm, int
     }
   }
   __syncthreads();
-  if (c >= Cc) return;
+  if (!in) return;
 #pragma unroll
   for (int k = 0; k < 4; k++) {
     Wr[(int64_t)(g * 4 + k) * ldm + c] = v[k];
@@ -818,8 +820,8 @@ __global__ void __launch_bounds__(256) k_pivot_rows(double2* W, int64_t ldm, int
 // 64 x 64 tiles take 32 x 32 ones.
 template <int kT>
 __global__ void __launch_bounds__(128, kT == 4 ? 3 : 4)
-    k_gj_update(double2* W, int64_t ldm, int64_t r0, int64_t R, int64_t c0, int64_t Cc, int64_t j0, int jn,
-                const double2* __restrict__ P, const double2* __restrict__ Wr) {
+    k_gj_update(double2* W, int64_t ldm, int64_t r0, int64_t R, int64_t c0, int64_t Cc, int64_t x0, int64_t x1,
+                int64_t j0, int jn, const double2* __restrict__ P, const double2* __restrict__ Wr) {
   constexpr int kTile = 16 * kT, kBst = kTile + 2;
   extern __shared__ double2 gj_sm[];
   double2* As = gj_sm;               // [kTile][kAS]
@@ -889,7 +891,7 @@ __global__ void __launch_bounds__(128, kT == 4 ? 3 : 4)
 #pragma unroll
       for (int h = 0; h < 2; h++) {
         const int64_t c = n0 + wc * 8 * kT + ni * 8 + (lane & 3) * 2 + h;
-        if (c < Cc) __stcg(W + r * ldm + c, cmk(acc[mi][ni][h], acc[mi][ni][2 + h]));
+        if (c < Cc && !(c >= x0 && c < x1)) __stcg(W + r * ldm + c, cmk(acc[mi][ni][h], acc[mi][ni][2 + h]));
       }
   }
 }
@@ -954,10 +956,9 @@ bool gj_step_fits(int64_t active_rows) {
   return active_rows <= (int64_t)kGjRows * gj_max_cluster<4 * kGjRows>();
 }
 
-cudaError_t launch_gj_panel(const double2* W, int64_t ldm, int64_t R, int64_t N, int64_t j0, int jn, bool trailing,
-                            double2* P, void* scratch, int* status, cudaStream_t s) {
+static cudaError_t launch_gj_panel(const double2* W, int64_t ldm, int64_t R, int64_t N, int64_t j0, int jn,
+                                   bool trailing, double2* P, void* scratch, int* src, int* status, cudaStream_t s) {
   int* swaps = reinterpret_cast<int*>(reinterpret_cast<double2*>(scratch) + (size_t)N * (kSw + kColpermCtas));
-  int* src = reinterpret_cast<int*>(scratch);
   const int64_t row0 = trailing ? j0 : 0, n = R - row0;
   const int most = std::min(gj_max_cluster<512>(), gj_max_cluster<4 * kGjRows>());
   int K = 1;
@@ -969,15 +970,16 @@ cudaError_t launch_gj_panel(const double2* W, int64_t ldm, int64_t R, int64_t N,
                                s);
 }
 
-void launch_gj_update(double2* W, int64_t ldm, int64_t R, int64_t N, int64_t Cc, int64_t j0, int jn, bool trailing,
-                      const double2* P, double2* Wr, void* scratch, cudaStream_t s) {
-  const int* src = reinterpret_cast<const int*>(scratch);
-  const int64_t lo = trailing ? j0 + jn : 0;
-  if (lo >= Cc || lo >= R) return;
-  k_pivot_rows<<<(unsigned)((Cc - lo + 31) / 32), 256, 0, s>>>(W, ldm, lo, Cc, j0, jn, src, src + kSw, Wr);
-  if (((Cc - lo + kBN - 1) / kBN) * ((R - lo + kBM - 1) / kBM) < kSmallTiles) {
-    const dim3 grid((unsigned)((Cc - lo + 31) / 32), (unsigned)((R - lo + 31) / 32));
-    k_gj_update<2><<<grid, 128, sizeof(double2) * (32 * kAS + kBK * 34), s>>>(W, ldm, lo, R, lo, Cc, j0, jn, P, Wr);
+// pivot rows and rank-32 update of the columns [c0, Cc) without [x0, x1)
+static void launch_gj_update(double2* W, int64_t ldm, int64_t lo, int64_t R, int64_t c0, int64_t Cc, int64_t x0,
+                             int64_t x1, int64_t j0, int jn, const double2* P, double2* Wr, const int* src,
+                             cudaStream_t s) {
+  if (c0 >= Cc || lo >= R) return;
+  k_pivot_rows<<<(unsigned)((Cc - c0 + 31) / 32), 256, 0, s>>>(W, ldm, c0, Cc, x0, x1, j0, jn, src, src + kSw, Wr);
+  if (((Cc - c0 + kBN - 1) / kBN) * ((R - lo + kBM - 1) / kBM) < kSmallTiles) {
+    const dim3 grid((unsigned)((Cc - c0 + 31) / 32), (unsigned)((R - lo + 31) / 32));
+    k_gj_update<2><<<grid, 128, sizeof(double2) * (32 * kAS + kBK * 34), s>>>(W, ldm, lo, R, c0, Cc, x0, x1, j0, jn, P,
+                                                                             Wr);
     return;
   }
   static std::atomic<bool> attr[kMaxDevices];
@@ -987,8 +989,59 @@ void launch_gj_update(double2* W, int64_t ldm, int64_t R, int64_t N, int64_t Cc,
     cudaFuncSetAttribute(k_gj_update<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGemmSmem);
     attr[dev & (kMaxDevices - 1)].store(true);
   }
-  const dim3 grid((unsigned)((Cc - lo + kBN - 1) / kBN), (unsigned)((R - lo + kBM - 1) / kBM));
-  k_gj_update<4><<<grid, 128, kGemmSmem, s>>>(W, ldm, lo, R, lo, Cc, j0, jn, P, Wr);
+  const dim3 grid((unsigned)((Cc - c0 + kBN - 1) / kBN), (unsigned)((R - lo + kBM - 1) / kBM));
+  k_gj_update<4><<<grid, 128, kGemmSmem, s>>>(W, ldm, lo, R, c0, Cc, x0, x1, j0, jn, P, Wr);
+}
+
+cudaError_t launch_gj_step(double2* W, int64_t ldm, int64_t R, int64_t N, int64_t Cc, int64_t j0, int jn, bool trailing,
+                           double2* P, double2* Wr, void* scratch, int* status, cudaStream_t s, cudaEvent_t before,
+                           cudaEvent_t after) {
+  int* src = reinterpret_cast<int*>(scratch);
+  const int64_t lo = trailing ? j0 + jn : 0;
+  cudaError_t e = launch_gj_panel(W, ldm, R, N, j0, jn, trailing, P, scratch, src, status, s);
+  if (e == cudaSuccess && before) e = cudaEventRecord(before, s);
+  if (e != cudaSuccess) return e;
+  launch_gj_update(W, ldm, lo, R, lo, Cc, 0, 0, j0, jn, P, Wr, src, s);
+  return after ? cudaEventRecord(after, s) : cudaSuccess;
+}
+
+// Look-ahead: of a step's update the next panel's 32 columns go first, on the
+// panel stream, then the next panel runs there (16 SMs) beside the rest of the
+// update on s.  The panel is launched first and its stream has priority, or
+// the update would leave its cluster no SMs until its last wave.  P and the
+// row lists alternate between two buffers; the pivot rows Wr do not: a step's
+// are written after the update before has finished.  A step is then the panel
+// (60 to 75 us) and ~10 us for its columns: 106 -> 78 us at N = 1500.
+cudaError_t launch_gj_sweep(double2* W, int64_t ldm, int64_t R, int64_t N, int64_t Cc, bool trailing, double2* P,
+                            double2* Wr, void* scratch, int* status, cudaStream_t s, const GjAhead& ah) {
+  auto width = [&](int64_t j0) { return (int)std::min<int64_t>(kSw, N - j0); };
+  cudaError_t e = cudaSuccess;
+  auto ok = [&](cudaError_t v) { return (e = v) == cudaSuccess; };
+  const int64_t ldp = R * kSw;
+  int* src = reinterpret_cast<int*>(scratch);
+  if (!ok(cudaEventRecord(ah.update, s)) || !ok(cudaStreamWaitEvent(ah.stream, ah.update, 0)) ||
+      !ok(launch_gj_panel(W, ldm, R, N, 0, width(0), trailing, P, scratch, src, status, ah.stream)))
+    return e;
+  int b = 0;
+  for (int64_t j0 = 0; j0 < N; j0 += kSw, b ^= 1) {
+    const int jn = width(j0);
+    const int64_t lo = trailing ? j0 + jn : 0, j1 = j0 + kSw;
+    const int64_t x1 = j1 < N ? j1 + width(j1) : j1;
+    double2* Pb = P + b * ldp;
+    int* srcb = src + b * 2 * kSw;
+    if (j1 < N) {
+      if (!ok(cudaStreamWaitEvent(ah.stream, ah.update, 0))) return e;
+      launch_gj_update(W, ldm, lo, R, j1, x1, 0, 0, j0, jn, Pb, Wr, srcb, ah.stream);
+    }
+    if (!ok(cudaEventRecord(ah.panel, ah.stream))) return e;
+    if (j1 < N && !ok(launch_gj_panel(W, ldm, R, N, j1, width(j1), trailing, P + (b ^ 1) * ldp, scratch,
+                                      src + (b ^ 1) * 2 * kSw, status, ah.stream)))
+      return e;
+    if (!ok(cudaStreamWaitEvent(s, ah.panel, 0))) return e;
+    launch_gj_update(W, ldm, lo, R, lo, Cc, j1, j1 < N ? x1 : j1, j0, jn, Pb, Wr, srcb, s);
+    if (!ok(cudaEventRecord(ah.update, s))) return e;
+  }
+  return cudaGetLastError();
 }
 
 size_t gepp_scratch_bytes(int64_t N) {
