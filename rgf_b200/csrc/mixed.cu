@@ -565,7 +565,7 @@ __global__ void k_mx_delta(double2* S, int64_t ldS, const int* pairs, int npairs
 // One Gauss-Jordan step of the slice inverse in a single launch:
 //   W_dst = W' - V U,  V = W(:, J) - E_J,  U = T W'(J, :),  T = W(J, J)^-1,
 //   W' = W_src with the columns J replaced by those of the identity (E_J).
-// Every CTA owns a 128 x 128 real tile of W (64 complex columns) and forms
+// Every CTA owns 128 rows x H x 128 real columns of W and forms
 // T itself (redundantly: the 32-pivot chain sets the step time anyway, and
 // no CTA waits for another), U for its columns straight into the swizzled
 // shared-memory operand, the 3xTF32 product on tcgen05 (TMEM accumulator)
@@ -573,21 +573,22 @@ __global__ void k_mx_delta(double2* S, int64_t ldS, const int* pairs, int npairs
 // finishes early never overwrites what another still reads.  256 threads.
 // ---------------------------------------------------------------------------
 namespace gjs {
-constexpr int BN = 128;                 // real columns per tile
+constexpr int BN = 128;                 // real columns of a half
 constexpr uint32_t CH = 16384;          // one operand K-chunk: 128 rows x 32 fp32 (128-byte rows)
-// A = V (hi, lo); B = U (hi, lo), which first holds the U product's left
-// operand realify_right(W'(J, tile columns)) in the same geometry
-constexpr uint32_t OFF_AH = 0, OFF_AL = 2 * CH, OFF_BH = 4 * CH, OFF_BL = 6 * CH;  // 32 KB each
-constexpr uint32_t OFF_WP = 8 * CH;     // W' tile: 4 chunks [chunk][row][32 fp32], unswizzled
+// A = V (hi, lo); per half B = U (hi, lo), which first holds the U product's
+// left operand realify_right(W'(J, columns of the half)) in the same geometry
+// and last the half's 128 x 128 result on its way to memory
+constexpr uint32_t OFF_AH = 0, OFF_AL = 2 * CH, OFF_B = 4 * CH, B_BYTES = 4 * CH, B_LO = 2 * CH;
 constexpr uint32_t TU_CH = 8192;        // one K-chunk of the T image: 64 rows x 128 bytes
 constexpr uint32_t TU_HALF = 2 * TU_CH; // hi image, then lo image
 constexpr uint32_t TU_BYTES = 2 * TU_HALF;
-constexpr uint32_t OFF_TU = 12 * CH;    // the realified T image (right operand of the U product)
-constexpr uint32_t SMEM = OFF_TU + TU_BYTES + 1024;
-constexpr uint32_t TMEM_COLS = 256;     // update accumulator: columns [0, 128); U product: [128, 192)
-constexpr int TP = BN + 4;              // pitch of the epilogue staging tile (over the operands)
-static_assert(128 * TP * 4 <= OFF_WP, "staging tile");
-static_assert(SMEM <= 227 * 1024, "shared memory of one CTA");
+template <int H>
+struct Lay {  // H halves per CTA
+  static constexpr uint32_t OFF_TU = OFF_B + H * B_BYTES;  // the realified T image (right operand of the U product)
+  static constexpr uint32_t SMEM = OFF_TU + TU_BYTES + 1024;
+  static constexpr uint32_t TMEM_COLS = 256 * H;  // per half: update accumulator [0, 128), U product [128, 192)
+};
+static_assert(Lay<2>::SMEM <= 227 * 1024, "shared memory of one CTA");
 }  // namespace gjs
 
 // Development builds only (-DRGF_MX_STAMPS, never in the shipped library):
@@ -681,6 +682,8 @@ __device__ __forceinline__ void mm_cols(const float2* A, const float2* B, int ld
 // panels stays rolled: every launch runs this once on an SM whose instruction
 // cache the tile CTAs have filled, so code is paid by the line.
 // A zero or non-finite pivot sets *bad.
+// the server's 256 threads (the first eight warps of a step's CTA)
+__device__ __forceinline__ void server_sync() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
 struct Inv32Sm {
   float4 F[2][2][32];
   float4 R[8][4][2];
@@ -733,7 +736,7 @@ __device__ __forceinline__ void inv32_cols(float2 (&a)[4], Inv32Sm* sm, int warp
         R[k][1] = sm->R[warp][k][1];
       }
     }
-    __syncthreads();
+    server_sync();
     if (warp != p) {
       const float4 f01 = F[0][lane], f23 = F[1][lane];
       const float2 f[4] = {make_float2(f01.x, f01.y), make_float2(f01.z, f01.w), make_float2(f23.x, f23.y),
@@ -788,7 +791,7 @@ __device__ __forceinline__ void publish_tu(float2 (&a)[4], int jn, float2* Tout,
       *reinterpret_cast<float4*>(dst + gjs::TU_HALF) = make_float4(x.x - hi.x, x.y - hi.y, x.z - hi.z, x.w - hi.w);
     }
   }
-  __syncthreads();
+  server_sync();
   const int tid = 32 * warp + lane;
   const float4* s4 = reinterpret_cast<const float4*>(stage);
 #pragma unroll
@@ -856,13 +859,13 @@ __device__ void t_server(const float* __restrict__ Wsrc, int64_t lda, int j0, in
 #pragma unroll
   for (int q = 0; q < 4; q++) {
     const int c = cq + 8 * q;
-    Tj[r * LD + c] = ns.Tin[r * NB + c];
+    Tj[r * LD + c] = __ldcg(ns.Tin + r * NB + c);
     const float2 z = make_float2(0.f, 0.f);
-    B1[r * LDB + c] = (r < jn && c < jn1) ? *reinterpret_cast<const float2*>(Wsrc + (int64_t)(j0 + r) * lda + 2 * (j1 + c)) : z;
-    B2[r * LD + c] = (r < jn1 && c < jn) ? *reinterpret_cast<const float2*>(Wsrc + (int64_t)(j1 + r) * lda + 2 * (j0 + c)) : z;
-    B3[r * LD + c] = (r < jn1 && c < jn1) ? *reinterpret_cast<const float2*>(Wsrc + (int64_t)(j1 + r) * lda + 2 * (j1 + c)) : z;
+    B1[r * LDB + c] = (r < jn && c < jn1) ? __ldcg(reinterpret_cast<const float2*>(Wsrc + (int64_t)(j0 + r) * lda + 2 * (j1 + c))) : z;
+    B2[r * LD + c] = (r < jn1 && c < jn) ? __ldcg(reinterpret_cast<const float2*>(Wsrc + (int64_t)(j1 + r) * lda + 2 * (j0 + c))) : z;
+    B3[r * LD + c] = (r < jn1 && c < jn1) ? __ldcg(reinterpret_cast<const float2*>(Wsrc + (int64_t)(j1 + r) * lda + 2 * (j1 + c))) : z;
   }
-  __syncthreads();
+  server_sync();
   MX_PSTAMP(2);
   float2 m[4];  // lane = row, warp = four columns
   if (!ns.same_block) {
@@ -906,16 +909,16 @@ __device__ void t_server(const float* __restrict__ Wsrc, int64_t lda, int j0, in
   publish_tu(m, jn1, ns.Tout, ns.tu_out, stage, warp, lane);
 }
 
-__global__ void __launch_bounds__(256, 1)
-    k_mx_gj_step(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapW,
-                 const float* __restrict__ Wsrc, float* __restrict__ Wdst, int64_t lda, int N, int j0, int jn,
-                 const GjNext ns, int* status, long long timeout) {
+template <int H>
+__global__ void __launch_bounds__(256 * H, 1)
+    k_mx_gj_step(const __grid_constant__ CUtensorMap mapA, const float* __restrict__ Wsrc, float* __restrict__ Wdst, int64_t lda, int N, int j0,
+                 int jn, const GjNext ns, int* status, long long timeout) {
   using namespace gjs;
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t bar_ld;
   __shared__ __align__(8) uint64_t bar_tu;
-  __shared__ __align__(8) uint64_t bar_mu;
-  __shared__ __align__(8) uint64_t bar_mma;
+  __shared__ __align__(8) uint64_t bar_mu[H];
+  __shared__ __align__(8) uint64_t bar_mma[H];
   __shared__ uint32_t tmem_sh;
   __shared__ int bad;
   pdl_open();
@@ -933,18 +936,24 @@ __global__ void __launch_bounds__(256, 1)
     pdl_wait();
     MX_SSTAMP(0);
     __syncthreads();
-    if (ns.Tout) t_server(Wsrc, lda, j0, jn, ns, gb, &bad);
+    if (ns.Tout && tid < 256) t_server(Wsrc, lda, j0, jn, ns, gb, &bad);
     __syncthreads();
     MX_SSTAMP(1);
     if (bad && tid == 0) atomicOr(status, kStatusSingular);
     return;
   }
-  const int m0 = blockIdx.y * 128, n0 = (blockIdx.x - 1) * BN;
+  // eight warps (w8) per half of the CTA's columns; V and T are shared
+  constexpr uint32_t OFF_TU = Lay<H>::OFF_TU, TMEM_COLS = Lay<H>::TMEM_COLS;
+  const int half = warp >> 3, w8 = warp & 7;
+  const int m0 = blockIdx.y * 128, n0 = ((blockIdx.x - 1) * H + half) * BN;
+  const uint32_t OFF_BH = OFF_B + half * B_BYTES, OFF_BL = OFF_BH + B_LO;
   if (tid == 0) {
     tc32::mbar_init(tc32::su32(&bar_ld), 1);
     tc32::mbar_init(tc32::su32(&bar_tu), 1);
-    tc32::mbar_init(tc32::su32(&bar_mu), 1);
-    tc32::mbar_init(tc32::su32(&bar_mma), 1);
+    for (int h = 0; h < H; h++) {
+      tc32::mbar_init(tc32::su32(&bar_mu[h]), 1);
+      tc32::mbar_init(tc32::su32(&bar_mma[h]), 1);
+    }
     bad = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -958,14 +967,14 @@ __global__ void __launch_bounds__(256, 1)
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const uint32_t tmem = tmem_sh;
+  const uint32_t tmem0 = tmem_sh, tmem = tmem0 + 256 * half;
   pdl_wait();
   MX_STAMP(1);
   MX_TSTAMP(0);
 
   // (1) the image of this step's pivot-block inverse (published by the server
   //     of the step before); TMA: V's rows W_src(m0.., 2 j0 .. 2 j0 + 63)
-  //     swizzled for the MMA, and the W' tile
+  //     swizzled for the MMA
   const uint32_t bl = tc32::su32(&bar_ld), btu = tc32::su32(&bar_tu);
   if (tid == 0) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(btu), "r"(TU_BYTES) : "memory");
@@ -973,21 +982,20 @@ __global__ void __launch_bounds__(256, 1)
                      sb + OFF_TU),
                  "l"(ns.tu_in), "r"(TU_BYTES), "r"(btu)
                  : "memory");
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bl), "r"(6 * CH) : "memory");
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bl), "r"(2 * CH) : "memory");
     for (int kc = 0; kc < 2; kc++) tc32::tma_load_3d(sb + OFF_AH + kc * CH, &mapA, 2 * j0 + 32 * kc, m0, 0, bl);
-    for (int kc = 0; kc < 4; kc++) tc32::tma_load_3d(sb + OFF_WP + kc * CH, &mapW, n0 + 32 * kc, m0, 0, bl);
   }
   // (2) the U product's left operand realify_right(W'(J, tile columns)), W' =
   //     W with the pivot columns replaced by the identity's: lane = pivot row m
-  //     (K = 2m, 2m + 1), warp = 8 complex columns j (rows 2j: conj W'(m, j),
+  //     (K = 2m, 2m + 1), w8 = 8 complex columns j (rows 2j: conj W'(m, j),
   //     2j + 1: i conj W'(m, j)), split hi/lo into the B area
   {
     const int m = lane, kf = 2 * m, kc = kf >> 5, gq = (kf & 31) >> 2, ofs = (kf & 3) * 4;
     float4 wv[4];
 #pragma unroll
     for (int q = 0; q < 4; q++) {
-      const int n = n0 + 16 * warp + 4 * q;
-      wv[q] = (m < jn && n < lda) ? *reinterpret_cast<const float4*>(Wsrc + (int64_t)(j0 + m) * lda + n)
+      const int n = n0 + 16 * w8 + 4 * q;
+      wv[q] = (m < jn && n < lda) ? __ldcg(reinterpret_cast<const float4*>(Wsrc + (int64_t)(j0 + m) * lda + n))
                                   : make_float4(0.f, 0.f, 0.f, 0.f);
     }
     MX_STAMP(2);
@@ -995,7 +1003,7 @@ __global__ void __launch_bounds__(256, 1)
     for (int q = 0; q < 4; q++) {
 #pragma unroll
       for (int h = 0; h < 2; h++) {
-        const int j = 8 * warp + 2 * q + h, c = (n0 >> 1) + j;
+        const int j = 8 * w8 + 2 * q + h, c = (n0 >> 1) + j;
         float re = h ? wv[q].z : wv[q].x, im = h ? wv[q].w : wv[q].y;
         if (c >= j0 && c < j0 + jn) {
           re = (j0 + m == c && m < jn) ? 1.f : 0.f;
@@ -1018,8 +1026,8 @@ __global__ void __launch_bounds__(256, 1)
   MX_STAMP(3);
   // (3) the U product on tcgen05 (3xTF32, M = 128, N = 64, K = 64) into TMEM
   //     columns [128, 192): row n of the result is row n of U's operand
-  const uint32_t bmu = tc32::su32(&bar_mu);
-  if (tid == 0) {
+  const uint32_t bmu = tc32::su32(&bar_mu[half]);
+  if (w8 == 0 && lane == 0) {
     wait_bar(btu, 0, status, timeout);
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
@@ -1042,8 +1050,8 @@ __global__ void __launch_bounds__(256, 1)
   const bool ok_ld = wait_bar(bl, 0, status, timeout);
   MX_STAMP(4);
 #pragma unroll
-  for (int u = 0; u < 8; u++) {
-    const int g = tid + 256 * u, kc = g >> 10, gi = g & 1023, row = gi >> 3, gp = gi & 7;
+  for (int u = 0; u < 8 / H; u++) {
+    const int g = tid + 256 * H * u, kc = g >> 10, gi = g & 1023, row = gi >> 3, gp = gi & 7;
     const int kf = kc * 32 + ((gp ^ (row & 7)) << 2);  // logical fp32 column of the granule
     const uint32_t off = OFF_AH + kc * CH + row * 128 + gp * 16;
     float4 x = *reinterpret_cast<const float4*>(gb + off);
@@ -1064,7 +1072,7 @@ __global__ void __launch_bounds__(256, 1)
   __syncwarp();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   {
-    const int n = 32 * (warp & 3) + lane, kc = warp >> 2;
+    const int n = 32 * (w8 & 3) + lane, kc = w8 >> 2;
 #pragma unroll
     for (int hf = 0; hf < 2; hf++) {
       float v[16];
@@ -1085,8 +1093,8 @@ __global__ void __launch_bounds__(256, 1)
   __syncthreads();
   MX_STAMP(6);
   // (6) 2 K-chunks x 4 K-steps x 3 products on tcgen05
-  const uint32_t bm = tc32::su32(&bar_mma);
-  if (tid == 0) {
+  const uint32_t bm = tc32::su32(&bar_mma[half]);
+  if (w8 == 0 && lane == 0) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
     for (int kc = 0; kc < 2; kc++) {
@@ -1103,43 +1111,51 @@ __global__ void __launch_bounds__(256, 1)
     tc32::mma_commit(bm);
   }
   __syncwarp();
+  // W' of this warp's rows (every eighth of the half), while the products run
+  const int n = n0 + 4 * lane;
+  float4 w[16];
+#pragma unroll
+  for (int u = 0; u < 16; u++) {
+    const int m = m0 + w8 + 8 * u;
+    if (m < N && n < lda) w[u] = __ldcg(reinterpret_cast<const float4*>(Wsrc + (int64_t)m * lda + n));
+  }
   const bool ok = wait_bar(bm, 0, status, timeout) && ok_ld && ok_u;
   MX_STAMP(7);
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  // (7) epilogue: D (TMEM) -> staging over the operands -> W_dst = W' - D, one warp per row
-  float* stg = reinterpret_cast<float*>(gb + OFF_AH);
-  if (warp < 4) {
-    const int row = warp * 32 + lane;
-#pragma unroll 1
-    for (int c = 0; c < BN; c += 16) {
-      float v[16];
-      tc32::tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c, v);
-      float4* t4 = reinterpret_cast<float4*>(stg + row * TP + c);
+  // (7) epilogue: D (TMEM) -> the half's B area (granules of 16 bytes, column
+  //     granule g of row r at g ^ (r mod 32)) -> W_dst = W' - D, one warp per row
+  float4* stg = reinterpret_cast<float4*>(gb + OFF_BH);
+  {
+    const int row = 32 * (w8 & 3) + lane, c0 = 64 * (w8 >> 2);
 #pragma unroll
-      for (int j = 0; j < 4; j++) t4[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+    for (int c = 0; c < 64; c += 16) {
+      float v[16];
+      tc32::tmem_ld16(tmem + ((uint32_t)(32 * (w8 & 3)) << 16) + (uint32_t)(c0 + c), v);
+#pragma unroll
+      for (int j = 0; j < 4; j++)
+        stg[row * 32 + (((c0 + c) / 4 + j) ^ lane)] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
     }
   }
-  __syncthreads();
+  asm volatile("bar.sync %0, 256;" ::"r"(2 + half) : "memory");
   MX_STAMP(8);
-  if (ok) {
-    const int cc = lane * 4, n = n0 + cc;
-    const float* wp = reinterpret_cast<const float*>(gb + OFF_WP) + (cc >> 5) * (CH / 4) + (cc & 31);
-#pragma unroll 4
-    for (int rr = warp; rr < 128; rr += 8) {
-      const int m = m0 + rr;
-      if (m >= N || n >= lda) continue;
-      const float4 d = *reinterpret_cast<const float4*>(stg + rr * TP + cc);
-      float4 w = *reinterpret_cast<const float4*>(wp + rr * 32);
-      const int c0 = n >> 1;  // complex columns c0, c0 + 1
-      if (c0 >= j0 && c0 < j0 + jn) {
-        w.x = (c0 == m) ? 1.f : 0.f;
-        w.y = 0.f;
+  if (ok && n < lda) {
+    const int c0 = n >> 1;  // complex columns c0, c0 + 1
+    const bool u0 = c0 >= j0 && c0 < j0 + jn, u1 = c0 + 1 >= j0 && c0 + 1 < j0 + jn;
+#pragma unroll
+    for (int u = 0; u < 16; u++) {
+      const int rr = w8 + 8 * u, m = m0 + rr;
+      if (m >= N) continue;
+      const float4 d = stg[rr * 32 + (lane ^ (rr & 31))];
+      if (u0) {
+        w[u].x = (c0 == m) ? 1.f : 0.f;
+        w[u].y = 0.f;
       }
-      if (c0 + 1 >= j0 && c0 + 1 < j0 + jn) {
-        w.z = (c0 + 1 == m) ? 1.f : 0.f;
-        w.w = 0.f;
+      if (u1) {
+        w[u].z = (c0 + 1 == m) ? 1.f : 0.f;
+        w[u].w = 0.f;
       }
-      *reinterpret_cast<float4*>(Wdst + (int64_t)m * lda + n) = make_float4(w.x - d.x, w.y - d.y, w.z - d.z, w.w - d.w);
+      *reinterpret_cast<float4*>(Wdst + (int64_t)m * lda + n) =
+          make_float4(w[u].x - d.x, w[u].y - d.y, w[u].z - d.z, w[u].w - d.w);
     }
   }
   MX_STAMP(9);
@@ -1147,7 +1163,7 @@ __global__ void __launch_bounds__(256, 1)
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   if (warp == 0)
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem0), "r"(TMEM_COLS) : "memory");
 }
 
 // the first pivot-block inverse of the first slice (later ones come from the
@@ -1247,7 +1263,10 @@ rgf_status smatrix_mixed(const MixedProblem& mp, const MixedAlloc& alloc, cudaSt
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  if (cudaFuncSetAttribute(k_mx_gj_step, cudaFuncAttributeMaxDynamicSharedMemorySize, gjs::SMEM) != cudaSuccess) {
+  if (cudaFuncSetAttribute(k_mx_gj_step<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, gjs::Lay<1>::SMEM) !=
+          cudaSuccess ||
+      cudaFuncSetAttribute(k_mx_gj_step<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, gjs::Lay<2>::SMEM) !=
+          cudaSuccess) {
     set_error("cannot configure the Gauss-Jordan step kernel's shared memory");
     return RGF_ERR_CUDA;
   }
@@ -1297,12 +1316,11 @@ rgf_status smatrix_mixed(const MixedProblem& mp, const MixedAlloc& alloc, cudaSt
   int* mstat = static_cast<int*>(pStat);
 
   // per side: two W buffers with their tensor maps (swizzled 32-column boxes
-  // for the update's left operand, unswizzled ones for the W' tile), two
-  // pivot-block inverses and two buffers of the solve's right operand Bt (2P
+  // for the update's left operand), two pivot-block inverses and two buffers of the solve's right operand Bt (2P
   // rows x lda, hi/lo); the factor store (N rows x lda, L slices) is shared
   struct Side {
     float* W[2];
-    CUtensorMap mA[2], mWp[2], mBh[2], mBl[2];
+    CUtensorMap mA[2], mBh[2], mBl[2];
     float2* Tb;
     uint8_t* Tu;  // images of the two inverses (publish_tu)
     float *bh[2], *bl[2];
@@ -1324,7 +1342,6 @@ rgf_status smatrix_mixed(const MixedProblem& mp, const MixedAlloc& alloc, cudaSt
       d.bh[w] = bt_hi + (q * 4 + 2 * w) * 2 * P * lda;
       d.bl[w] = d.bh[w] + 2 * P * lda;
       maps_ok = maps_ok && tc32::make_map(&d.mA[w], d.W[w], lda, N, 1, lda, 0, tc32::BM) &&
-                tc32::make_map(&d.mWp[w], d.W[w], lda, N, 1, lda, 0, tc32::BM, CU_TENSOR_MAP_SWIZZLE_NONE) &&
                 tc32::make_map(&d.mBh[w], d.bh[w], lda, 2 * P, 1, lda, 0, sbn) &&
                 tc32::make_map(&d.mBl[w], d.bl[w], lda, 2 * P, 1, lda, 0, sbn);
     }
@@ -1388,7 +1405,13 @@ rgf_status smatrix_mixed(const MixedProblem& mp, const MixedAlloc& alloc, cudaSt
   RGF_CUDA_TRY_MX(cudaEventRecord(ev[0], s));
   const dim3 ga((unsigned)((ldw + 255) / 256), (unsigned)std::min<int64_t>(N, 8192));
   // one grid column more than the tiles (column 0): its first CTA serves the next pivot block
-  const dim3 ggj((unsigned)((lda + gjs::BN - 1) / gjs::BN + 1), (unsigned)ntile_m);
+  const int64_t halves = (lda + gjs::BN - 1) / gjs::BN;
+  // 128 x 256 tiles where 128 x 128 ones would need close to two waves or more
+  // (a CTA has its SM to itself, and one of two halves takes 10.4 us instead of
+  // 6): a slice of N = 850 / 900 / 1024 / 1400 / 2048 takes 289 / 348 / 420 /
+  // 1072 / 3258 us with 128 columns and 353 / 379 / 410 / 918 / 2869 us with 256
+  const bool wide_cta = 10 * nside * (halves * ntile_m + 1) > 17 * sms;
+  const dim3 ggj((unsigned)((wide_cta ? (halves + 1) / 2 : halves) + 1), (unsigned)ntile_m);
   auto lead = [&](int64_t k, int side) -> const double2* {  // lead block in slice k's matrix
     if (side == 0) return (k == 0) ? mp.G0[0] : nullptr;
     return (k == L - 1) ? mp.G0[1] : nullptr;
@@ -1440,7 +1463,8 @@ rgf_status smatrix_mixed(const MixedProblem& mp, const MixedAlloc& alloc, cudaSt
     } else {
       ns.Tout = nullptr;  // nothing follows this step within the side
     }
-    launch_pdl(k_mx_gj_step, ggj, dim3(256), gjs::SMEM, d.q, d.mA[d.cur], d.mWp[d.cur], (const float*)d.W[d.cur],
+    launch_pdl(wide_cta ? k_mx_gj_step<2> : k_mx_gj_step<1>, ggj, dim3(wide_cta ? 512 : 256),
+               wide_cta ? gjs::Lay<2>::SMEM : gjs::Lay<1>::SMEM, d.q, d.mA[d.cur], (const float*)d.W[d.cur],
                d.W[d.cur ^ 1], lda, (int)N, (int)j0, jn, ns, mstat, kGemmTimeout);
     d.cur ^= 1;
     d.gstep++;
