@@ -124,14 +124,18 @@ typedef struct {
   int32_t precision;  /* rgf_precision (0 = RGF_FP64)                                  */
   int32_t engine;     /* 0 (default): persistent register-resident sweep kernel when
                          the matrix fits on the GPU, pivoting inside each 32 x 32
-                         pivot block; every slice inverse is checked a posteriori
-                         and the call is recomputed with engine 1 if one fails.
+                         pivot block; a structure whose slices leave SMs idle is cut
+                         along its length into parts that are swept side by side and
+                         joined; every slice inverse is checked a posteriori and the
+                         call is recomputed, as one sweep, then with engine 1, if one
+                         fails.
                          1: one launch sequence per pivot step with partial
                          pivoting over the whole column (LAPACK zgetrf's choice,
                          as MATLAB's inv)                                            */
   int32_t S_on_device;/* 1: S is a device pointer (no D2H copy)                        */
   int32_t profile;    /* > 0: time the dominant kernel with CUDA events on every
-                         profile-th slice (read back with rgf_last_profile)           */
+                         profile-th slice (read back with rgf_last_profile); such a
+                         call is never cut into parts                                 */
 } rgf_options;
 
 /* channels struct (setup_channels.m:30-82).  All pointers are caller-owned
@@ -171,8 +175,9 @@ RGF_API rgf_status rgf_smatrix_3d(rgf_handle h, const rgf_syst3d* syst, const rg
  * set-up runs on a host thread and stream of its own, and all their slice
  * sweeps run in ONE persistent cooperative launch in which gangs of CTAs,
  * sized to each structure, take the structures from a work queue in device
- * memory, largest first (at most 160 structures per launch; a structure that
- * needs tiles smaller than 96 x 96 sweeps on its own first).  workers > 0:
+ * memory, largest first (at most 160 sweeps per launch; up to 80 structures are
+ * swept as two halves each; a structure that needs tiles smaller than 96 x 96
+ * sweeps on its own first).  workers > 0:
  * that many concurrent pipelines (host threads, each with its own stream and
  * workspace), whose persistent sweeps share the GPU's SMs through one budget.
  * With opt->precision = RGF_TF32X3 every structure takes the split-precision
@@ -192,8 +197,8 @@ RGF_API rgf_status rgf_smatrix_batch_2d(rgf_handle h, int64_t count, const rgf_s
  * For a real objective F of S with dF = 2 Re sum_ab D_ab dS_ab (e.g. D = conj(S)
  * for F = sum |S_ab|^2), dF/d Re(eps) = 2 Re g and dF/d Im(eps) = -2 Im g.
  * Method: the forward sweep keeps a checkpoint every `checkpoint` slices
- * (<= 0: ceil(sqrt(L))); the backward pass recomputes one segment at a time
- * and runs the recursions Psi_k = [X_k, 0] + g_k Psi_{k+1},
+ * (<= 0: ceil(sqrt(L))); the backward pass recomputes the segments, as many
+ * side by side as fit the GPU and 1 GiB of snapshots, and runs the recursions Psi_k = [X_k, 0] + g_k Psi_{k+1},
  * Phi_k = [Z_k; 0] + Phi_{k+1} g_k over the start-connected slice inverses g_k.
  * D, S and g are device pointers when opt->S_on_device, host otherwise. */
 RGF_API rgf_status rgf_smatrix_grad_2d(rgf_handle h, const rgf_syst2d* syst, const rgf_request* req,
@@ -300,7 +305,9 @@ RGF_API rgf_status rgf_last_profile(rgf_handle h, int64_t* timed_launches, doubl
  * tile[i] (32, 64 or 96) of the first entry with Rp <= rows_max[i] (rows_max
  * non-decreasing) whenever its grid fits the GPU, else the built-in choice
  * (the largest tile that keeps >= 60% of the SMs busy).  n = 0 clears the
- * table.  Batched calls pass it to their pipelines.  rgf_b200.autotune writes
+ * table.  It governs sweeps in one piece: parts of a structure cut along its
+ * length choose their tile with their number.  Batched calls pass it to their
+ * pipelines.  rgf_b200.autotune writes
  * such a table from timed sweeps and caches it as JSON. */
 RGF_API rgf_status rgf_set_tile_table(rgf_handle h, int32_t n, const int64_t* rows_max, const int32_t* tile);
 /* Issue all work of this handle on the caller's stream (a cudaStream_t);

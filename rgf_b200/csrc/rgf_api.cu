@@ -1591,9 +1591,14 @@ rgf_status smatrix_run(rgf_handle h, const Problem& p, const rgf_request* req, c
   // the swept matrix.
   auto sweep = [&](int64_t Ract, int64_t Cact, bool timed, bool corner_only) -> rgf_status {
     const bool in_cluster = gj_step_fits(Ract);
-    const bool ahead = in_cluster && !timed && !h->arena && !h->sm_budget && N >= kAheadMin;
+    const size_t pc_bytes = sizeof(double2) * std::max(R, Cp) * kSwW;
+    bool ahead = in_cluster && !timed && !h->arena && !h->sm_budget && N >= kAheadMin;
+    if (ahead && (ensure_ahead(h) || ensure(h, h->pc, 2 * pc_bytes))) {  // no room: the steps in turn
+      cudaGetLastError();
+      ahead = false;
+      if ((st = ensure(h, h->pc, pc_bytes))) return st;
+    }
     if (ahead) {
-      if ((st = ensure_ahead(h)) || (st = ensure(h, h->pc, 2 * sizeof(double2) * std::max(R, Cp) * kSwW))) return st;
       const cudaError_t e = launch_gj_sweep(M, ldm, Ract, N, Cact, corner_only, as<double2>(h->pc), as<double2>(h->u),
                                             h->gepp.p, status, h->stream, h->ahead);
       if (e != cudaSuccess) cudaStreamSynchronize(h->ahead.stream);
