@@ -764,8 +764,8 @@ rgf_status second_stream(rgf_handle h) {
 // widths from which the per-step engine runs its panels beside the updates:
 // below, a step is all panel and the launches and events between two streams
 // cost more than they hide (us a step, in turn / side by side: 58.9 / 60.2 at
-// N = 256, 58.4 / 57.0 at 400, 70 / 63 at 512, 85 / 69 at 1000, 106 / 78 at
-// 1500, 146 / 102 at 1900)
+// N = 256, with the kernels not yet placed early; 53.3 / 52.9 at 400, 66 / 60 at
+// 512, 82 / 64 at 1000, 103 / 75 at 1500, 150 / 102 at 1900)
 constexpr int64_t kAheadMin = 400;
 rgf_status ensure_ahead(rgf_handle h) {
   GjAhead& a = h->ahead;

@@ -570,7 +570,7 @@ __global__ void k_colperm(double2* M, int64_t ldm, int64_t R, int64_t N, const i
 // step's 2900 when it was done that way).  Lane = column with a row per register
 // needs no rotation but three times the instructions per pivot: 84 us against
 // 72 us for 1700 rows.  The one-CTA panel above (its rows in L2) takes 770 us
-// there; a whole step went from 787 to 106 us at N = 1500, and to 78 us with the
+// there; a whole step went from 787 to 106 us at N = 1500, and to 75 us with the
 // panels beside the updates (launch_gj_sweep).
 // ---------------------------------------------------------------------------
 constexpr int kGjRows = 256;     // most rows of a CTA
@@ -643,6 +643,8 @@ __global__ void __launch_bounds__(kThreads, 1)
     k_gj_panel(const double2* __restrict__ W, int64_t ldm, int R, int N, int row0, int j0, int jn, int rows,
                double2* __restrict__ P, int* __restrict__ swaps, int* __restrict__ src, int* __restrict__ dst,
                int* status) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   extern __shared__ __align__(16) unsigned char gj_raw[];
   GjShared& sh = *reinterpret_cast<GjShared*>(gj_raw);
   const unsigned full = 0xffffffffu;
@@ -778,9 +780,19 @@ constexpr int kColpermCtas = 64;
 // Wr(q, c) = W(src[q], c) on columns [c0, Cc) (unit columns in J, zero rows
 // from jn on), and the displaced rows of J to their places outside it.  32
 // columns a CTA; every thread reads its rows before the CTA writes any.
+// the three kernels of a step follow one another by programmatic dependent
+// launch: a kernel's CTAs are placed while the one before still runs and wait
+// here for its results (3 us of a step: 59 -> 55 us at N = 100 to 256, 78 -> 75
+// at 1500)
+__device__ __forceinline__ void gj_after_previous() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 __global__ void __launch_bounds__(256) k_pivot_rows(double2* W, int64_t ldm, int64_t c0, int64_t Cc, int64_t x0,
                                                     int64_t x1, int64_t j0, int jn, const int* __restrict__ src,
                                                     const int* __restrict__ dst, double2* __restrict__ Wr) {
+  gj_after_previous();
   const int64_t c = c0 + blockIdx.x * (int64_t)32 + (threadIdx.x & 31);
   const int g = threadIdx.x >> 5;
   const bool in = c < Cc && !(c >= x0 && c < x1);
@@ -795,10 +807,10 @@ __global__ void __launch_bounds__(256) k_pivot_rows(double2* W, int64_t ldm, int
       if (c >= j0 && c < j0 + jn) {
         v[k] = cmk(c - j0 == q ? 1.0 : 0.0, 0.0);
       } else {
-        v[k] = W[(int64_t)src[q] * ldm + c];
-        const int d = dst[q];
+        v[k] = __ldcg(W + (int64_t)__ldcg(src + q) * ldm + c);
+        const int d = __ldcg(dst + q);
         if (d < j0 || d >= j0 + jn) {
-          u[k] = W[(j0 + q) * ldm + c];
+          u[k] = __ldcg(W + (j0 + q) * ldm + c);
           to[k] = d;
         }
       }
@@ -823,6 +835,7 @@ __global__ void __launch_bounds__(128, kT == 4 ? 3 : 4)
     k_gj_update(double2* W, int64_t ldm, int64_t r0, int64_t R, int64_t c0, int64_t Cc, int64_t x0, int64_t x1,
                 int64_t j0, int jn, const double2* __restrict__ P, const double2* __restrict__ Wr) {
   constexpr int kTile = 16 * kT, kBst = kTile + 2;
+  gj_after_previous();
   extern __shared__ double2 gj_sm[];
   double2* As = gj_sm;               // [kTile][kAS]
   double2* Bs = gj_sm + kTile * kAS; // [kBK][kBst]
@@ -933,16 +946,21 @@ template <int kThreads>
 static cudaError_t gj_panel(const double2* W, int64_t ldm, int R, int N, int row0, int j0, int jn, int K, int rows,
                             double2* P, int* swaps, int* src, int* dst, int* status, cudaStream_t s) {
   cudaLaunchConfig_t cfg{};
-  cudaLaunchAttribute at{};
-  at.id = cudaLaunchAttributeClusterDimension;
-  at.val.clusterDim.x = K;
-  at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  cudaLaunchAttribute at[2]{};
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = K;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  // a CTA of the larger kind needs a whole SM: placed early it finds none beside
+  // the columns' update, and then loses them to the rest (104 -> 117 us a step at
+  // N = 1900)
+  at[1].val.programmaticStreamSerializationAllowed = kThreads == 512;
   cfg.gridDim = dim3(K);
   cfg.blockDim = dim3(4 * rows);
   cfg.dynamicSmemBytes = sizeof(GjShared);
   cfg.stream = s;
-  cfg.attrs = &at;
-  cfg.numAttrs = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 2;
   return cudaLaunchKernelEx(&cfg, k_gj_panel<kThreads>, W, ldm, R, N, row0, j0, jn, rows, P, swaps, src, dst, status);
 }
 
@@ -970,16 +988,33 @@ static cudaError_t launch_gj_panel(const double2* W, int64_t ldm, int64_t R, int
                                s);
 }
 
+template <typename... KArgs, typename... Args>
+static void launch_after(bool early, void (*kern)(KArgs...), dim3 grid, int threads, size_t smem, cudaStream_t s,
+                         Args... args) {
+  cudaLaunchConfig_t cfg{};
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = early ? 1 : 0;
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
+}
+
 // pivot rows and rank-32 update of the columns [c0, Cc) without [x0, x1)
 static void launch_gj_update(double2* W, int64_t ldm, int64_t lo, int64_t R, int64_t c0, int64_t Cc, int64_t x0,
                              int64_t x1, int64_t j0, int jn, const double2* P, double2* Wr, const int* src,
-                             cudaStream_t s) {
+                             cudaStream_t s, bool early) {
   if (c0 >= Cc || lo >= R) return;
-  k_pivot_rows<<<(unsigned)((Cc - c0 + 31) / 32), 256, 0, s>>>(W, ldm, c0, Cc, x0, x1, j0, jn, src, src + kSw, Wr);
+  launch_after(early, k_pivot_rows, dim3((unsigned)((Cc - c0 + 31) / 32)), 256, 0, s, W, ldm, c0, Cc, x0, x1, j0, jn, src,
+               src + kSw, Wr);
   if (((Cc - c0 + kBN - 1) / kBN) * ((R - lo + kBM - 1) / kBM) < kSmallTiles) {
     const dim3 grid((unsigned)((Cc - c0 + 31) / 32), (unsigned)((R - lo + 31) / 32));
-    k_gj_update<2><<<grid, 128, sizeof(double2) * (32 * kAS + kBK * 34), s>>>(W, ldm, lo, R, c0, Cc, x0, x1, j0, jn, P,
-                                                                             Wr);
+    launch_after(early, k_gj_update<2>, grid, 128, sizeof(double2) * (32 * kAS + kBK * 34), s, W, ldm, lo, R, c0, Cc, x0, x1,
+                 j0, jn, P, Wr);
     return;
   }
   static std::atomic<bool> attr[kMaxDevices];
@@ -990,7 +1025,7 @@ static void launch_gj_update(double2* W, int64_t ldm, int64_t lo, int64_t R, int
     attr[dev & (kMaxDevices - 1)].store(true);
   }
   const dim3 grid((unsigned)((Cc - c0 + kBN - 1) / kBN), (unsigned)((R - lo + kBM - 1) / kBM));
-  k_gj_update<4><<<grid, 128, kGemmSmem, s>>>(W, ldm, lo, R, c0, Cc, x0, x1, j0, jn, P, Wr);
+  launch_after(early, k_gj_update<4>, grid, 128, kGemmSmem, s, W, ldm, lo, R, c0, Cc, x0, x1, j0, jn, P, Wr);
 }
 
 cudaError_t launch_gj_step(double2* W, int64_t ldm, int64_t R, int64_t N, int64_t Cc, int64_t j0, int jn, bool trailing,
@@ -1001,17 +1036,18 @@ cudaError_t launch_gj_step(double2* W, int64_t ldm, int64_t R, int64_t N, int64_
   cudaError_t e = launch_gj_panel(W, ldm, R, N, j0, jn, trailing, P, scratch, src, status, s);
   if (e == cudaSuccess && before) e = cudaEventRecord(before, s);
   if (e != cudaSuccess) return e;
-  launch_gj_update(W, ldm, lo, R, lo, Cc, 0, 0, j0, jn, P, Wr, src, s);
+  launch_gj_update(W, ldm, lo, R, lo, Cc, 0, 0, j0, jn, P, Wr, src, s, true);
   return after ? cudaEventRecord(after, s) : cudaSuccess;
 }
 
 // Look-ahead: of a step's update the next panel's 32 columns go first, on the
 // panel stream, then the next panel runs there (16 SMs) beside the rest of the
 // update on s.  The panel is launched first and its stream has priority, or
-// the update would leave its cluster no SMs until its last wave.  P and the
+// the update would leave its cluster no SMs until its last wave (which is also
+// why that update is not placed early).  P and the
 // row lists alternate between two buffers; the pivot rows Wr do not: a step's
 // are written after the update before has finished.  A step is then the panel
-// (60 to 75 us) and ~10 us for its columns: 106 -> 78 us at N = 1500.
+// (60 to 75 us) and ~8 us for its columns: 106 -> 75 us at N = 1500.
 cudaError_t launch_gj_sweep(double2* W, int64_t ldm, int64_t R, int64_t N, int64_t Cc, bool trailing, double2* P,
                             double2* Wr, void* scratch, int* status, cudaStream_t s, const GjAhead& ah) {
   auto width = [&](int64_t j0) { return (int)std::min<int64_t>(kSw, N - j0); };
@@ -1031,14 +1067,14 @@ cudaError_t launch_gj_sweep(double2* W, int64_t ldm, int64_t R, int64_t N, int64
     int* srcb = src + b * 2 * kSw;
     if (j1 < N) {
       if (!ok(cudaStreamWaitEvent(ah.stream, ah.update, 0))) return e;
-      launch_gj_update(W, ldm, lo, R, j1, x1, 0, 0, j0, jn, Pb, Wr, srcb, ah.stream);
+      launch_gj_update(W, ldm, lo, R, j1, x1, 0, 0, j0, jn, Pb, Wr, srcb, ah.stream, true);
     }
     if (!ok(cudaEventRecord(ah.panel, ah.stream))) return e;
     if (j1 < N && !ok(launch_gj_panel(W, ldm, R, N, j1, width(j1), trailing, P + (b ^ 1) * ldp, scratch,
                                       src + (b ^ 1) * 2 * kSw, status, ah.stream)))
       return e;
     if (!ok(cudaStreamWaitEvent(s, ah.panel, 0))) return e;
-    launch_gj_update(W, ldm, lo, R, lo, Cc, j1, j1 < N ? x1 : j1, j0, jn, Pb, Wr, srcb, s);
+    launch_gj_update(W, ldm, lo, R, lo, Cc, j1, j1 < N ? x1 : j1, j0, jn, Pb, Wr, srcb, s, false);
     if (!ok(cudaEventRecord(ah.update, s))) return e;
   }
   return cudaGetLastError();
